@@ -123,3 +123,34 @@ def test_resolve_and_pfm_output(native, ctx, tmp_path):
     lin = (a[:, :3] / a[:, 3:4]).reshape(30, 40, 3)
     assert np.array_equal(img, lin)
     fb.close()
+
+
+@pytest.mark.parametrize("spp", [1.0, 3.0])
+def test_tonemap_bytes_at_every_step(native, ctx, spp):
+    """Values on both sides of each of the 255 rounding steps of the sRGB byte,
+    and the ends of the range (negative, above 1, infinite, NaN), against the
+    double-precision power: the bytes are equal."""
+    n = np.arange(255) + 0.5
+    s = n / 255.0
+    lin = np.where(s < 12.92 * 0.0031308, s / 12.92, ((s + 0.055) / 1.055) ** 2.4).astype(np.float32)
+    near = lin.view(np.uint32)[:, None] + np.arange(-40, 41, dtype=np.int64)[None, :]
+    r = np.concatenate([near.astype(np.uint32).view(np.float32).ravel(), np.linspace(0.0, 1.0, 4096, dtype=np.float32),
+                        np.array([-1.0, -0.0, 1.0, 1.5, np.inf, -np.inf, np.nan, 1e-30, 0.0031308], np.float32)])
+    acc = np.zeros((len(r), 4), np.float32)
+    with np.errstate(invalid="ignore"):
+        acc[:, :3] = (r * np.float32(spp))[:, None]
+        q = (acc[:, 0] / np.float32(spp)).astype(np.float32)
+    acc[:, 3] = spp
+    dev = torch.from_numpy(acc).cuda()
+    out = torch.zeros(len(r), dtype=torch.int32, device="cuda")
+    native.tonemap(dev, len(r), 1, out)
+    torch.cuda.synchronize()
+    q = np.where(np.isnan(q), np.float32(0), np.clip(q, 0, 1)).astype(np.float32)
+    p = np.power(q.astype(np.float64), np.float64(np.float32(1) / np.float32(2.4))).astype(np.float32)
+    enc = np.where(q < 0.0031308, (q.astype(np.float64) * 12.92).astype(np.float32),
+                   (p.astype(np.float64) * 1.055 - np.float64(np.float32(0.055))).astype(np.float32))
+    byte = np.floor((enc * np.float32(255)).astype(np.float64) + 0.5).astype(np.uint32)
+    want = byte * np.uint32(0x010101) + np.uint32(0xFF000000)
+    got = out.cpu().numpy().view(np.uint32)
+    bad = np.flatnonzero(got != want)
+    assert bad.size == 0, f"{bad.size} of {len(r)} differ, e.g. {r[bad[:4]]}: {got[bad[:4]]} vs {want[bad[:4]]}"
