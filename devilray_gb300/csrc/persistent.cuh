@@ -45,28 +45,21 @@ constexpr int kP8MinBlocks = DR_P8_MIN_BLOCKS;
 #ifndef DR_POSTPONE_MIN
 #define DR_POSTPONE_MIN 0
 #endif
-// Which traversals send their leaf triangles through the warp's staged
-// triangle batch (tri_batch.cuh) instead of each lane's own loop: the public
-// closest-hit and any-hit kernels, the renderer's path rays and shadow rays.
-// Measured (incoherent workload: 2^20 triangles, 16.8 M rays, 23 % hits;
-// many-light 1080p and box-room renders, 16 spp): closest hit 3.81 -> 4.37
-// Grays/s and any hit 3.43 -> 3.35 ms with the batch; the renders 51.9 ->
-// 53.4 ms and 2.50 -> 2.90 ms with the path rays batched, 53.0 and 2.87 ms
-// with the shadow rays batched. Path and shadow rays of a closed scene nearly
-// all hit, and the batch delays the early exits and the shrinking closest-hit
-// bound that then prune the traversal; the public rays mostly miss, so the
-// batch only saves issue slots.
+// Which public traversals send their leaf triangles through the warp's staged
+// triangle batch (tri_batch.cuh) instead of each lane's own loop. Measured
+// (incoherent workload: 2^20 triangles, 16.8 M rays, 23 % hits): closest hit
+// 3.81 -> 4.37 Grays/s and any hit 3.43 -> 3.35 ms with the batch. The
+// renderer's rays keep the lane loop (many-light 1080p render 51.9 -> 53.4 ms,
+// box room 2.50 -> 2.90 ms with the path rays batched; 53.0 and 2.87 ms with
+// the shadow rays batched): path and shadow rays of a closed scene nearly all
+// hit, and the batch delays the early exits and the shrinking closest-hit bound
+// that then prune the traversal; the public rays mostly miss, so the batch only
+// saves issue slots.
 #ifndef DR_TRI_BATCH_CLOSEST
 #define DR_TRI_BATCH_CLOSEST 1
 #endif
 #ifndef DR_TRI_BATCH_ANY
 #define DR_TRI_BATCH_ANY 1
-#endif
-#ifndef DR_TRI_BATCH_PATHS
-#define DR_TRI_BATCH_PATHS 0
-#endif
-#ifndef DR_TRI_BATCH_SHADOW
-#define DR_TRI_BATCH_SHADOW 0
 #endif
 // The batch is tested once it holds this many pairs, or once this many lanes
 // wait for its results (their rays have no node left). Measured: 16 -> 4.38,
@@ -130,12 +123,14 @@ __device__ __forceinline__ uint32_t persistent_chunk(uint64_t n, uint32_t fixed 
 
 // Ray source of the public entry points: ray i of a contiguous array, all rays
 // in one hierarchy. A source's load() gives the ray and the root node of the
-// hierarchy it is traced in (kNoRoot: nothing to traverse, the ray misses).
+// hierarchy it is traced in (kNoRoot: nothing to traverse, the ray misses),
+// is_any() whether a ray of a mixed queue asks for any hit.
 struct DirectSource {
     const dr_ray *rays;
     dr_hit *hits;
     uint8_t *occluded;
     uint32_t root;
+    __device__ __forceinline__ bool is_any(uint64_t) const { return occluded != nullptr; }
     __device__ __forceinline__ bool load(uint64_t i, DevRay &r, uint32_t &node) const
     {
         node = root;
@@ -150,14 +145,16 @@ struct DirectSource {
     __device__ __forceinline__ void any(uint64_t i, bool hit) const { occluded[i] = hit ? 1 : 0; }
 };
 
-template <int MODE, bool ANY, bool COUNT, bool BATCH, int STACK = DR_SMEM_STACK, class Source>
+template <int MODE, Query Q, bool COUNT, bool BATCH, int STACK = DR_SMEM_STACK, class Source>
 __device__ __forceinline__ void persistent_wide(const Wide8Args &a, const Source &src, uint64_t n,
                                                 unsigned long long *counter, unsigned long long &nn,
                                                 unsigned long long &nb, unsigned long long &nt,
                                                 unsigned long long &nhits, uint32_t fixed_chunk = 0)
 {
     constexpr unsigned FULL = 0xffffffffu;
-    constexpr bool HALF = !ANY && DR_HALF_CVT;  // node tests with FP16 grid planes (closest hit)
+    constexpr bool ANY = Q == Query::kAny;
+    static_assert(Q != Query::kMixed || !BATCH, "triangle batches serve one kind of query");
+    constexpr bool HALF = !ANY && DR_HALF_CVT;  // node tests with FP16 grid planes (all but any hit)
     constexpr bool LUT = !DR_NO_OCT_ORDER && (DR_OCT_LUT == 1 || (DR_OCT_LUT == 2 && ANY));
     const uint8_t *oct_lut = nullptr;
     if constexpr (LUT) {
@@ -223,8 +220,9 @@ __device__ __forceinline__ void persistent_wide(const Wide8Args &a, const Source
                 uint32_t root;
                 if (src.load(idx, r, root) && root != kNoRoot) {
                     wide_init<MODE>(s, r, root);
+                    if constexpr (Q == Query::kMixed) s.any = src.is_any(idx);
                     active = true;
-                } else if (ANY) {
+                } else if (ANY || (Q == Query::kMixed && src.is_any(idx))) {
                     src.any(idx, false);
                 } else {
                     src.closest(idx, 0.0f, INT_MAX);
@@ -248,7 +246,7 @@ __device__ __forceinline__ void persistent_wide(const Wide8Args &a, const Source
                 const bool go = active && !waiting && !fin && s.tmask == 0;
                 if (__popc(__ballot_sync(FULL, go)) < DR_INNER_MIN_LANES_BATCH) break;
                 if (go) {
-                    fin = wide_advance<ANY>(a, s, stack);
+                    fin = wide_advance(a, s, stack);
                     if (!fin && s.have_node) wide_visit<MODE, HALF, LUT>(a, s, cn, cb, oct_lut);
                 }
             }
@@ -272,7 +270,7 @@ __device__ __forceinline__ void persistent_wide(const Wide8Args &a, const Source
             nbatch += __reduce_max_sync(FULL, fits ? incl : 0u);
             // 3. next node; a ray with no node left waits for its pairs' results
             if (active && !waiting && s.tmask == 0) {
-                done = fin || wide_advance<ANY>(a, s, stack);
+                done = fin || wide_advance(a, s, stack);
                 if (done && pend != 0) {
                     waiting = true;
                     done = false;
@@ -306,7 +304,7 @@ __device__ __forceinline__ void persistent_wide(const Wide8Args &a, const Source
                 const bool go = active && !fin && s.tmask == 0;
                 if (__popc(__ballot_sync(FULL, go)) < DR_INNER_MIN_LANES_LANE) break;
                 if (go) {
-                    fin = wide_advance<ANY>(a, s, stack);
+                    fin = wide_advance(a, s, stack);
                     if (!fin && s.have_node) wide_visit<MODE, HALF, LUT>(a, s, cn, cb, oct_lut);
                 }
             }
@@ -323,15 +321,15 @@ __device__ __forceinline__ void persistent_wide(const Wide8Args &a, const Source
                 if (postpone) {
                     stack.put(s.sp++, make_uint2(s.tbase, s.tmask | kTriGroupFlag));
                     s.tmask = 0;
-                } else if (wide_triangles<MODE, ANY>(a, s, ct)) {
+                } else if (wide_triangles<MODE, Q>(a, s, ct)) {
                     done = found = true;
                 }
             }
             // 3. next node
-            if (active && !done && s.tmask == 0) done = fin || wide_advance<ANY>(a, s, stack);
+            if (active && !done && s.tmask == 0) done = fin || wide_advance(a, s, stack);
         }
         if (active && done) {
-            if (ANY) {
+            if (ANY || (Q == Query::kMixed && s.any)) {
                 src.any(idx, found);
             } else {
                 src.closest(idx, s.best_t, s.best_prim);

@@ -60,6 +60,7 @@ struct RenderParams {
     uint32_t wave;             // slots of this wave
     uint32_t wave_pix;         // accumulation threads of this wave
     uint32_t chunk;            // persistent fetch size, 0 = adaptive
+    int max_depth;             // bounces of this render
     // per-slot buffers
     float4 *rays;              // dr_ray, 2 x float4
     float2 *hits;
@@ -70,7 +71,7 @@ struct RenderParams {
     uint32_t *list[2];
     uint32_t *shadow_list;
     uint32_t *counts;          // [0, 64): active paths per bounce, [64, 128): shadow rays per bounce
-    unsigned long long *work;  // persistent-kernel counters: [b] closest hit, [64 + b] shadow rays
+    unsigned long long *work;  // persistent-kernel counters: [b] the traversals before the shading of bounce b
     unsigned long long *ray_totals;  // rays of the render: [0] path rays, [1] shadow rays
     // path guiding (guided kernels only)
     float *guide_y;            // [slot][40] network output at the slot's current vertex
@@ -417,94 +418,73 @@ __global__ void __launch_bounds__(kRenderBlock) k_debug(SceneArrays p, RenderJob
     if (J.pix_casts) J.pix_casts[pixel] += casts;
 }
 
-// Ray sources of the persistent wide kernels: list entry i names a path slot,
-// whose job names the hierarchy root.
-struct PathSource {
-    const uint32_t *list;
-    const float4 *rays;
+// Ray source of the persistent wide kernel: the path rays of a bounce, then
+// the shadow rays of the bounce before it. An entry of either list names a path
+// slot, whose job names the hierarchy root.
+struct BounceSource {
+    const uint32_t *paths, *shadows;
+    uint32_t npaths;
+    const float4 *rays, *shadow_rays;
     float2 *hits;
-    const uint32_t *slot_job;
-    const RenderJob *jobs;
-    __device__ __forceinline__ bool load(uint64_t i, DevRay &r, uint32_t &root) const
-    {
-        const uint32_t slot = list[i];
-        root = jobs[slot_job[slot]].root;
-        return load_ray(reinterpret_cast<const dr_ray *>(rays), slot, r);
-    }
-    __device__ __forceinline__ void closest(uint64_t i, float t, int32_t prim) const
-    {
-        hits[list[i]] = prim != INT_MAX ? make_float2(t, __int_as_float(prim))
-                                        : make_float2(__int_as_float(0x7f800000), __int_as_float(-1));
-    }
-    __device__ __forceinline__ void any(uint64_t, bool) const {}
-};
-
-struct ShadowSource {
-    const uint32_t *list;
-    const float4 *rays;
     float4 *color;
     const float4 *pending;
     const uint32_t *slot_job;
     const RenderJob *jobs;
+    __device__ __forceinline__ bool is_any(uint64_t i) const { return i >= npaths; }
+    __device__ __forceinline__ uint32_t slot(uint64_t i) const { return is_any(i) ? shadows[i - npaths] : paths[i]; }
     __device__ __forceinline__ bool load(uint64_t i, DevRay &r, uint32_t &root) const
     {
-        const uint32_t slot = list[i];
-        root = jobs[slot_job[slot]].root;
-        return load_ray(reinterpret_cast<const dr_ray *>(rays), slot, r);
+        const uint32_t s = slot(i);
+        root = jobs[slot_job[s]].root;
+        return load_ray(reinterpret_cast<const dr_ray *>(is_any(i) ? shadow_rays : rays), s, r);
     }
-    __device__ __forceinline__ void closest(uint64_t, float, int32_t) const {}
+    __device__ __forceinline__ void closest(uint64_t i, float t, int32_t prim) const
+    {
+        hits[paths[i]] = prim != INT_MAX ? make_float2(t, __int_as_float(prim))
+                                         : make_float2(__int_as_float(0x7f800000), __int_as_float(-1));
+    }
     __device__ __forceinline__ void any(uint64_t i, bool occluded) const
     {
         if (!occluded) {
-            const uint32_t slot = list[i];
-            const float4 c = color[slot], q = pending[slot];
-            color[slot] = make_float4(c.x + q.x, c.y + q.y, c.z + q.z, c.w + q.w);
+            const uint32_t s = shadows[i - npaths];
+            const float4 c = color[s], q = pending[s];
+            color[s] = make_float4(c.x + q.x, c.y + q.y, c.z + q.z, c.w + q.w);
         }
     }
 };
 
+// The traversals between the shading of bounce b - 1 and that of bounce b: the
+// shadow rays of bounce b - 1 and the path rays of bounce b, independent of one
+// another, as one queue. A launch lasts as long as its slowest rays, whatever
+// their number: one launch per bounce pays that tail once, and the longer queue
+// keeps more warps busy (path rays first: theirs are the longer walks). b = 0
+// has path rays only, b = max_depth shadow rays only. Two launches per bounce ->
+// one: box room 256x256, 1 spp, 992 -> 692 us; 16 spp 2.26 -> 1.88 ms;
+// many-light 1080p, 4 spp, 11.0 -> 9.9 ms.
 // STACK: shared-memory entries of each lane's traversal stack (kStackDepths).
 template <int MODE, int STACK>
-__global__ void __launch_bounds__(kTraceBlock, kP8MinBlocks) k_wave_closest_p8(RenderParams p, int b)
+__global__ void __launch_bounds__(kTraceBlock, kP8MinBlocks) k_wave_trace_p8(RenderParams p, int b)
 {
     const Wide8Args w{p.trace.nodes8, p.trace.tri_ref, p.trace.tri_wt, p.trace.prim, p.trace.num_nodes, p.trace.error,
                       p.trace.stack_limit};
-    const PathSource src{p.list[b & 1], p.rays, p.hits, p.slot_job, p.jobs};
+    const uint32_t npaths = b < p.max_depth ? p.counts[b] : 0u, nshadows = b > 0 ? p.counts[64 + b - 1] : 0u;
+    const BounceSource src{p.list[b & 1], p.shadow_list, npaths, p.rays, p.shadow_rays, p.hits, p.color, p.pending,
+                           p.slot_job, p.jobs};
     unsigned long long nn = 0, nb = 0, nt = 0, nh = 0;
-    persistent_wide<MODE, false, false, DR_TRI_BATCH_PATHS != 0, STACK>(w, src, p.counts[b], p.work + b, nn, nb, nt,
-                                                                         nh, p.chunk);
+    persistent_wide<MODE, Query::kMixed, false, false, STACK>(w, src, (uint64_t)npaths + nshadows, p.work + b, nn, nb,
+                                                              nt, nh, p.chunk);
 }
 
-template <int MODE, int STACK>
-__global__ void __launch_bounds__(kTraceBlock, kP8MinBlocks) k_wave_shadow_p8(RenderParams p, int b)
-{
-    const Wide8Args w{p.trace.nodes8, p.trace.tri_ref, p.trace.tri_wt, p.trace.prim, p.trace.num_nodes, p.trace.error,
-                      p.trace.stack_limit};
-    const ShadowSource src{p.shadow_list, p.shadow_rays, p.color, p.pending, p.slot_job, p.jobs};
-    unsigned long long nn = 0, nb = 0, nt = 0, nh = 0;
-    persistent_wide<MODE, true, false, DR_TRI_BATCH_SHADOW != 0, STACK>(w, src, p.counts[64 + b], p.work + 64 + b, nn,
-                                                                      nb, nt, nh, p.chunk);
-}
+// The persistent traversal kernel of one (triangle test, stack depth).
+using WaveTrace = void (*)(RenderParams, int);
 
-// The persistent traversal kernels of one (triangle test, stack depth).
-struct P8Kernels {
-    void (*closest)(RenderParams, int);
-    void (*shadow)(RenderParams, int);
-};
-
-template <int MODE, int STACK>
-constexpr P8Kernels p8_kernels()
-{
-    return P8Kernels{k_wave_closest_p8<MODE, STACK>, k_wave_shadow_p8<MODE, STACK>};
-}
-
-P8Kernels select_p8(int tri_mode, uint32_t stack)
+WaveTrace select_p8(int tri_mode, uint32_t stack)
 {
     const bool wt = tri_mode == DR_TRI_WATERTIGHT;
     switch (stack) {
-    case 4: return wt ? p8_kernels<1, 4>() : p8_kernels<0, 4>();
-    case 16: return wt ? p8_kernels<1, 16>() : p8_kernels<0, 16>();
-    default: return wt ? p8_kernels<1, 8>() : p8_kernels<0, 8>();
+    case 4: return wt ? k_wave_trace_p8<1, 4> : k_wave_trace_p8<0, 4>;
+    case 16: return wt ? k_wave_trace_p8<1, 16> : k_wave_trace_p8<0, 16>;
+    default: return wt ? k_wave_trace_p8<1, 8> : k_wave_trace_p8<0, 8>;
     }
 }
 
@@ -1067,11 +1047,7 @@ dr_status WaveRunner::prepare(const std::vector<RenderJob> &jobs, const WavePlan
     const size_t need = wave_buffer_bytes(plan.max_slots, gr != nullptr);
     // occupancy of the persistent kernels, queried here so enqueue (which may
     // be under stream capture) only reads the cache
-    for (int mode = 0; mode < 2; ++mode) {
-        const P8Kernels k = select_p8(mode, cfg.stack);
-        resident_blocks((const void *)k.closest, kTraceBlock);
-        resident_blocks((const void *)k.shadow, kTraceBlock);
-    }
+    for (int mode = 0; mode < 2; ++mode) resident_blocks((const void *)select_p8(mode, cfg.stack), kTraceBlock);
     const uint32_t train_need = gr ? std::max<uint32_t>(1, gr->batch) * std::max<uint32_t>(1, gr->steps) : 0;
     bool grow = jobs.size() > jobs_capacity || plan.segs.size() > segs_capacity || train_need > train_cap;
     for (int k = 0; k < K; ++k) grow = grow || wave_bytes[k] < need;
@@ -1147,9 +1123,8 @@ dr_status WaveRunner::enqueue(const SceneArrays &sc, const WavePlan &plan, const
     }
     const int sms = ctx->num_sms;
     const bool wt = tri_mode == DR_TRI_WATERTIGHT, wide = sc.trace.layout == 8;
-    const P8Kernels p8 = select_p8(tri_mode, cfg.stack);
-    const int closest_per_sm = resident_blocks((const void *)p8.closest, kTraceBlock);
-    const int shadow_per_sm = resident_blocks((const void *)p8.shadow, kTraceBlock);
+    const WaveTrace p8 = select_p8(tri_mode, cfg.stack);
+    const int trace_per_sm = resident_blocks((const void *)p8, kTraceBlock);
     DR_CUDA(cudaMemsetAsync(d_totals, 0, 2 * sizeof(unsigned long long), st));
     DR_CUDA(cudaEventRecord(fork, st));
     for (int k = 0; k < K; ++k) DR_CUDA(cudaStreamWaitEvent(stream[k], fork, 0));
@@ -1175,6 +1150,7 @@ dr_status WaveRunner::enqueue(const SceneArrays &sc, const WavePlan &plan, const
             q.guide_alpha = gr->alpha * f;
         }
         q.ray_totals = d_totals;
+        q.max_depth = (int)plan.max_depth;
         q.segs = d_segs + plan.wave_first[w];
         q.nsegs = plan.wave_first[w + 1] - plan.wave_first[w];
         q.wave = plan.wave_slots[w];
@@ -1182,16 +1158,18 @@ dr_status WaveRunner::enqueue(const SceneArrays &sc, const WavePlan &plan, const
         const uint32_t W = q.wave;
         const unsigned trace_grid = (unsigned)std::min<uint64_t>((W + kTraceBlock - 1) / kTraceBlock, (uint64_t)sms * 16);
         const unsigned shade_grid = (unsigned)std::min<uint64_t>((W + kRenderBlock - 1) / kRenderBlock, (uint64_t)sms * 16);
-        const uint64_t trace_blocks = (W + kTraceBlock - 1) / kTraceBlock;
-        const unsigned pgrid = (unsigned)std::min<uint64_t>(trace_blocks, (uint64_t)sms * closest_per_sm);
-        const unsigned sgrid = (unsigned)std::min<uint64_t>(trace_blocks, (uint64_t)sms * shadow_per_sm);
+        // bounce 0 traces the wave's camera rays, later launches up to twice as many rays
+        auto trace_blocks = [&](int b) {
+            const uint64_t rays = (uint64_t)W * (b > 0 && b < (int)plan.max_depth ? 2 : 1);
+            return (unsigned)std::min<uint64_t>((rays + kTraceBlock - 1) / kTraceBlock, (uint64_t)sms * trace_per_sm);
+        };
         DR_CUDA(cudaMemsetAsync(q.counts, 0, 128 * sizeof(uint32_t), ws));
         DR_CUDA(cudaMemsetAsync(q.work, 0, 128 * sizeof(unsigned long long), ws));
         if (gr) DR_CUDA(cudaMemsetAsync(q.guide_counts, 0, 64 * sizeof(uint32_t), ws));
         k_camera<<<(W + kRenderBlock - 1) / kRenderBlock, kRenderBlock, 0, ws>>>(q);
         for (int b = 0; b < (int)plan.max_depth; ++b) {
             if (wide) {
-                p8.closest<<<pgrid, kTraceBlock, 0, ws>>>(q, b);
+                p8<<<trace_blocks(b), kTraceBlock, 0, ws>>>(q, b);
             } else {
                 if (wt) k_wave_closest<1, 2><<<trace_grid, kTraceBlock, 0, ws>>>(q, b);
                 else k_wave_closest<0, 2><<<trace_grid, kTraceBlock, 0, ws>>>(q, b);
@@ -1211,13 +1189,12 @@ dr_status WaveRunner::enqueue(const SceneArrays &sc, const WavePlan &plan, const
             } else {
                 k_shade<false><<<shade_grid, kRenderBlock, 0, ws>>>(q, b);
             }
-            if (wide) {
-                p8.shadow<<<sgrid, kTraceBlock, 0, ws>>>(q, b);
-            } else {
+            if (!wide) {
                 if (wt) k_wave_shadow<1, 2><<<trace_grid, kTraceBlock, 0, ws>>>(q, b);
                 else k_wave_shadow<0, 2><<<trace_grid, kTraceBlock, 0, ws>>>(q, b);
             }
         }
+        if (wide) p8<<<trace_blocks((int)plan.max_depth), kTraceBlock, 0, ws>>>(q, (int)plan.max_depth);
         // images receive the waves in order
         if (w > 0) DR_CUDA(cudaStreamWaitEvent(ws, acc_done[(w - 1) % (uint32_t)K], 0));
         if (learn) {

@@ -514,8 +514,14 @@ struct WideState {
     uint2 group;
     int sp;
     bool have_node;
+    bool any;               // the ray ends at its first hit (Query::kMixed)
     uint32_t tbase, tmask;  // triangles waiting to be tested (persistent kernels)
 };
+
+// What a traversal answers: the closest hit, any hit, or per ray the one its
+// source asks for (WideState::any). An any-hit ray's best_t stays its tmax, so
+// one bound serves both.
+enum class Query { kClosest, kAny, kMixed };
 
 template <int MODE>
 __host__ __device__ __forceinline__ void wide_init(WideState &s, const DevRay &r, uint32_t root)
@@ -555,9 +561,10 @@ __device__ __forceinline__ void wide_visit(const Wide8Args &a, WideState &s, uns
 }
 
 // Tests the pending triangles; true when an any-hit query is answered.
-template <int MODE, bool ANY>
+template <int MODE, Query Q>
 __device__ __forceinline__ bool wide_triangles(const Wide8Args &a, WideState &s, unsigned long long &nt)
 {
+    constexpr bool ANY = Q == Query::kAny;
     uint32_t m = s.tmask;
     s.tmask = 0;
     while (m) {
@@ -569,7 +576,7 @@ __device__ __forceinline__ bool wide_triangles(const Wide8Args &a, WideState &s,
         const bool ok = MODE == 1 ? tri_test_wt(a.tri_wt, k, s.r, s.w, ANY ? s.r.tmax : s.best_t, t)
                                   : tri_test_ref(a.tri_ref, k, s.r, ANY ? s.r.tmax : s.best_t, t);
         if (ok) {
-            if (ANY) return true;
+            if (ANY || (Q == Query::kMixed && s.any)) return true;
             const int32_t prim = DR_LD(a.prim + k);
             if (t < s.best_t || prim < s.best_prim) {
                 s.best_t = t;
@@ -611,7 +618,7 @@ using LaneStack = LaneStackT<DR_SMEM_STACK>;
 
 // Next node: from the current group, else from the stack (a popped triangle
 // group becomes pending and is tested first). True when the ray is finished.
-template <bool ANY, class Stack>
+template <class Stack>
 __device__ __forceinline__ bool wide_advance(const Wide8Args &a, WideState &s, Stack &stack)
 {
     if ((s.group.y >> 8) == 0) {
