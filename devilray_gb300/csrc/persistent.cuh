@@ -10,6 +10,7 @@
 // unchanged, so results stay bit-identical.
 #pragma once
 
+#include "team.cuh"
 #include "trace_kernels.cuh"
 #include "trace_wide.cuh"
 #include "tri_batch.cuh"
@@ -175,8 +176,7 @@ __device__ __forceinline__ void persistent_wide(const Wide8Args &a, const Source
     WideState s;
     LaneStackT<STACK> stack;
     if constexpr (STACK > 0) {
-        __shared__ uint2 s_stack[kTraceBlock / 32][STACK > 0 ? STACK : 1][32];
-        stack.shared = &s_stack[threadIdx.x >> 5][0][threadIdx.x & 31];
+        stack.shared = block_stacks<STACK>() + (threadIdx.x >> 5) * (32 * STACK) + (threadIdx.x & 31);
     } else {
         stack.shared = nullptr;
     }

@@ -104,6 +104,16 @@ __global__ void __launch_bounds__(kTraceBlock, kP8MinBlocks) k_trace_any_p8(Trac
     persistent_wide<MODE, Query::kAny, false, DR_TRI_BATCH_ANY != 0>(w, src, a.n, a.work, nn, nb, nt, nh);
 }
 
+// Few rays: a team of lanes per ray (closest hit, or any hit when `occluded`
+// is set). Bound by the longest ray's chain of node and triangle steps.
+template <int MODE>
+__global__ void __launch_bounds__(kTraceBlock, 8) k_trace_team(TraceArgs a)
+{
+    const Wide8Args w{a.nodes8, a.tri_ref, a.tri_wt, a.prim, a.num_nodes, a.error, a.stack_limit};
+    const DirectSource src{a.rays, a.hits, a.occluded, scene_root(a.num_nodes)};
+    team_wide<MODE, kTeamTrace, 8>(w, src, GridQueue<kTeamTrace>{a.n, a.work});
+}
+
 int resident_blocks(const void *kernel, int block_threads)
 {
     // one entry per kernel: kernels of the same signature differ in registers
@@ -129,6 +139,23 @@ unsigned persistent_grid(K kernel, int num_sms, uint64_t n)
     return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(need, (uint64_t)num_sms * per_sm));
 }
 
+// One ray per warp until the chip is full, then further teams of each warp.
+static cudaError_t launch_team(const TraceArgs &a, int mode, cudaStream_t s)
+{
+    constexpr int kWarps = kTraceBlock / 32, kTeams = kTraceBlock / kTeamTrace;
+    const auto kernel = mode == 1 ? k_trace_team<1> : k_trace_team<0>;
+    const uint64_t resident = (uint64_t)a.num_sms * resident_blocks((const void *)kernel, kTraceBlock);
+    const unsigned grid = (unsigned)std::min<uint64_t>((a.n + kWarps - 1) / kWarps, resident);
+    if (a.n > (uint64_t)grid * kTeams) {  // otherwise no team takes a second ray
+        const cudaError_t e = cudaMemsetAsync(a.work, 0, sizeof(unsigned long long), s);
+        if (e != cudaSuccess) return e;
+    }
+    kernel<<<grid, kTraceBlock, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
+static bool few_rays(const TraceArgs &a) { return a.n <= (uint64_t)a.num_sms * kTeamRaysPerSm; }
+
 cudaError_t launch_trace_closest(const TraceArgs &a, int mode, bool count, cudaStream_t s)
 {
     if (a.n == 0) return cudaSuccess;
@@ -136,6 +163,7 @@ cudaError_t launch_trace_closest(const TraceArgs &a, int mode, bool count, cudaS
     if (blocks > 0x7fffffffull) return cudaErrorInvalidValue;
     const dim3 grid((unsigned)blocks), block(kTraceBlock);
     if (a.layout == 8) {
+        if (!count && few_rays(a)) return launch_team(a, mode, s);
         cudaError_t e = cudaMemsetAsync(a.work, 0, sizeof(unsigned long long), s);
         if (e != cudaSuccess) return e;
         if (mode == 1) {
@@ -164,6 +192,7 @@ cudaError_t launch_trace_any(const TraceArgs &a, int mode, cudaStream_t s)
     if (blocks > 0x7fffffffull) return cudaErrorInvalidValue;
     const dim3 grid((unsigned)blocks), block(kTraceBlock);
     if (a.layout == 8) {
+        if (few_rays(a)) return launch_team(a, mode, s);
         cudaError_t e = cudaMemsetAsync(a.work, 0, sizeof(unsigned long long), s);
         if (e != cudaSuccess) return e;
         if (mode == 1) k_trace_any_p8<1><<<persistent_grid(k_trace_any_p8<1>, a.num_sms, a.n), block, 0, s>>>(a);
