@@ -47,6 +47,20 @@ constexpr int kRenderBlock = 128;
 #endif
 constexpr int kShadeMinBlocks = DR_SHADE_MIN_BLOCKS;
 
+// Where k_wave_paths takes over. Waves of up to kWholePathsPerSm paths per SM
+// (155,648 on 152 SMs) run in it from the camera rays on; paths per wave and
+// time by bounces / in one kernel: 65,536 (box room) 696 / 464 us; 129,600
+// (2^17-triangle many-light) 853 / 490 us; 163,840 (box room) 950 / 872 us;
+// 262,144 (box room) 1,030 / 1,111 us. Larger waves hand over when at most
+// kTailPathsPerSm paths per SM (32,832) are left at bounce 2, 4, 8, 16 or 32: a
+// check that does not take over costs an empty launch (2 us). Limits of 16,384 /
+// 32,768 / 65,536 paths: many-light 2^16 triangles 512x512, 4 spp 1,439 / 1,359 /
+// 1,367 us (1,716 without), eight uneven scenes 967 / 969 / 969 us (1,286); a
+// limit of 131,072 makes the 1080p many-light image slower (10.0 -> 12.7 ms), where
+// the longest walks of a 2^20-triangle scene want more rays in flight.
+constexpr uint32_t kWholePathsPerSm = 1024, kTailPathsPerSm = 216;
+constexpr bool tail_check(int b) { return b >= 2 && (b & (b - 1)) == 0; }
+
 struct RenderParams {
     TraceArgs trace;
     const float4 *shade;
@@ -61,6 +75,7 @@ struct RenderParams {
     uint32_t wave_pix;         // accumulation threads of this wave
     uint32_t chunk;            // persistent fetch size, 0 = adaptive
     int max_depth;             // bounces of this render
+    uint32_t path_rays;        // with at most this many paths left k_wave_paths finishes them, 0 = never
     // per-slot buffers
     float4 *rays;              // dr_ray, 2 x float4
     float2 *hits;
@@ -470,9 +485,9 @@ __global__ void __launch_bounds__(kTraceBlock, kP8MinBlocks) k_wave_trace_p8(Ren
     const uint32_t npaths = b < p.max_depth ? p.counts[b] : 0u, nshadows = b > 0 ? p.counts[64 + b - 1] : 0u;
     const BounceSource src{p.list[b & 1], p.shadow_list, npaths, p.rays, p.shadow_rays, p.hits, p.color, p.pending,
                            p.slot_job, p.jobs};
+    const uint64_t n = (uint64_t)npaths + nshadows;
     unsigned long long nn = 0, nb = 0, nt = 0, nh = 0;
-    persistent_wide<MODE, Query::kMixed, false, false, STACK>(w, src, (uint64_t)npaths + nshadows, p.work + b, nn, nb,
-                                                              nt, nh, p.chunk);
+    persistent_wide<MODE, Query::kMixed, false, false, STACK>(w, src, n, p.work + b, nn, nb, nt, nh, p.chunk);
 }
 
 // The persistent traversal kernel of one (triangle test, stack depth).
@@ -513,10 +528,246 @@ __device__ __forceinline__ float object_ior(const RenderParams &p, int obj)
     return m.kind == DR_MAT_DIELECTRIC ? m.ior : 1.0f;
 }
 
+// The path vertex of `slot` at bounce b, given its closest hit: emission with
+// MIS, a light sample (`shadow`: its shadow ray is set and wants tracing), the
+// BSDF sample (`keep`: the path goes on with the ray it has set).
 template <bool GUIDED>
-__global__ void __launch_bounds__(kRenderBlock, GUIDED ? DR_GUIDE_SHADE_BLOCKS : kShadeMinBlocks) k_shade(RenderParams p, int b)
+__device__ __forceinline__ void shade_vertex(const RenderParams &p, int b, uint32_t slot, float2 h, bool &keep, bool &shadow)
+{
+    bool dead = false;
+    p.casts[slot] += 1;
+    const RenderJob &J = p.jobs[p.slot_job[slot]];
+    float *closed = nullptr;  // guided: the record this vertex closes
+    if (GUIDED && p.rec_n) {
+        // the radiance gathered before this vertex closes the last record
+        const uint32_t rn = p.rec_n[slot];
+        if (rn & kRecOpen) {
+            const uint32_t r = (rn & ~kRecOpen) - 1;
+            closed = p.rec + ((size_t)slot * kGuideRecords + r) * kRecFloats;
+            closed[11] = luminance(p.color[slot]);
+            p.rec_n[slot] = rn & ~kRecOpen;
+        }
+    }
+    const int prim = __float_as_int(h.y);
+    if (prim >= 0) {
+        const float t = h.x;
+        const float4 r0 = p.rays[2 * slot], r1 = p.rays[2 * slot + 1];
+        const F3 ro = f3(r0.x, r0.y, r0.z), rv = f3(r1.x, r1.y, r1.z);
+        const float4 s0 = __ldg(p.shade + 3 * prim), s1 = __ldg(p.shade + 3 * prim + 1),
+                     s2 = __ldg(p.shade + 3 * prim + 2);
+        const F3 A = f3(s0.x, s0.y, s0.z), B = f3(s0.w, s1.x, s1.y), C = f3(s1.z, s1.w, s2.x);
+        const int obj = __float_as_int(s2.y), mat_id = __float_as_int(s2.z);
+        // getIntersectionTris (IntersectionTestsImpl.hpp:36-67), identity transform
+        F3 n = normalized(cross(sub(A, B), sub(A, C)));
+        if (dot(n, rv) > 0) n = mul(n, -1.0f);
+        n = normalized(f3(n.x * 1.0f, n.y * 1.0f, n.z * 1.0f));
+        F3 hp = add(ro, mul(rv, t));
+        hp = f3(hp.x * 1.0f + 0.0f, hp.y * 1.0f + 0.0f, hp.z * 1.0f + 0.0f);
+        const dr_material &M = p.materials[mat_id];
+        float4 thr = p.thr[slot];
+        float4 col = p.color[slot];
+        const float4 pp4 = p.prev_p[slot];
+        const uint32_t pixel = p.slot_pix[slot], sample = p.slot_sample[slot];
+        float u[12];
+        const uint32_t g = 1u + 3u * (uint32_t)b;
+        uniforms4(J, pixel, sample, g, u);
+        F3 normal = n;
+        F3 new_o, new_v;
+        if (M.kind == DR_MAT_DIFFUSE) {
+            const float4 E = make_float4(M.emission[0], M.emission[1], M.emission[2], M.emission[3]);
+            const float4 alb = make_float4(M.albedo[0], M.albedo[1], M.albedo[2], M.albedo[3]);
+            // misWeightedEmission (PathGeneration.hpp:306-318) with the
+            // pdfs of computeNextBounceMisPdfs (:320-334) for (prev, this)
+            if (pp4.w == 0.0f) {
+                col = add4(col, mul4(E, thr));
+            } else {
+                const float4 pn4 = p.prev_n[slot];
+                const F3 pp = f3(pp4.x, pp4.y, pp4.z), pn = f3(pn4.x, pn4.y, pn4.z);
+                // guided: the density of the direction actually sampled there
+                const float pdf_bsdf = GUIDED ? p.prev_pdf[slot] : cosine_pdf(pp, hp, pn);
+                const float L = luminance(mul4s(E, kPi));
+                const float pdf_area = L / J.total_power;
+                const float pdf_nee = pdf_area * area_to_solid_angle(pp, hp, n);
+                if (pdf_bsdf + pdf_nee > 0) {
+                    const float wm = power_heuristic(pdf_bsdf, pdf_nee);
+                    col = add4(col, mul4s(mul4(E, thr), wm));
+#if DR_GUIDE_FULL_EMISSION
+                    // training only: the emission's share left to next-event
+                    // estimation (1 - wm) counts in the closed record's target
+                    if (GUIDED && closed) closed[11] -= luminance(mul4(E, thr)) * (1.0f - wm);
+#endif
+                }
+            }
+            const float alpha = GUIDED && b < p.guide_bounces ? p.guide_alpha : 0.0f;
+#if DR_GUIDE_DECODED
+            const float *lobes = GUIDED ? p.guide_y + (size_t)slot * kGuideOut : nullptr;
+#else
+            GuideMix lobes;
+            if (GUIDED && alpha > 0.0f) lobes = guide_mix(p.guide_y + (size_t)slot * kGuideOut);
+#endif
+            // next-event estimation: samplePointOnLights (:234-272) and
+            // evaluateDirectLighting (:336-361); visibility is the shadow ray
+            if (J.lights) {
+                uniforms4(J, pixel, sample, g + 1, u + 4);
+                uniforms4(J, pixel, sample, g + 2, u + 8);
+                int32_t oi, ti;
+                float opdf, tpdf;
+                alias_sample(p.light_table + J.obj_base, J.num_objects, u[3], u[4], oi, opdf);
+                const dr_object ob = p.objects[J.obj_base + oi];
+                alias_sample(p.tri_tables + ob.tri_begin, ob.tri_count, u[5], u[6], ti, tpdf);
+                const int lt = (int)ob.tri_begin + ti;
+                const float4 l0 = __ldg(p.shade + 3 * lt), l1 = __ldg(p.shade + 3 * lt + 1),
+                             l2 = __ldg(p.shade + 3 * lt + 2);
+                const F3 LA = f3(l0.x, l0.y, l0.z), LB = f3(l0.w, l1.x, l1.y), LC = f3(l1.z, l1.w, l2.x);
+                float uu = u[7], vv = u[8];
+                if (uu + vv > 1) {
+                    uu = 1 - uu;
+                    vv = 1 - vv;
+                }
+                F3 lp = add(add(LA, mul(sub(LB, LA), uu)), mul(sub(LC, LA), vv));
+                const F3 Aw = f3(LA.x * 1.0f, LA.y * 1.0f, LA.z * 1.0f);
+                const F3 Bw = f3(LB.x * 1.0f, LB.y * 1.0f, LB.z * 1.0f);
+                const F3 Cw = f3(LC.x * 1.0f, LC.y * 1.0f, LC.z * 1.0f);
+                const F3 perp = cross(sub(Aw, Bw), sub(Aw, Cw));
+                const float plen = length(perp);
+                const F3 ln = divs(perp, plen);
+                const float area = plen / 2.0f;
+                const float lpdf = opdf * tpdf / area;
+                lp = f3(lp.x * 1.0f + 0.0f, lp.y * 1.0f + 0.0f, lp.z * 1.0f + 0.0f);
+                const dr_material &LM = p.materials[ob.material];
+                float nee_pdf_bsdf = cosine_pdf(hp, lp, n);
+                if (GUIDED && alpha > 0.0f) {
+                    const F3 wl0 = normalized(sub(lp, hp));
+                    nee_pdf_bsdf = alpha * guide_density(lobes, wl0, n) + (1.0f - alpha) * nee_pdf_bsdf;
+                }
+                const float nee_pdf_nee = lpdf * area_to_solid_angle(hp, lp, ln);
+                const float dist = length(sub(lp, hp));
+                const F3 wl = divs(sub(lp, hp), dist);
+                const float cos_s = dot(wl, n);
+                const float cos_l = dot(wl, ln);
+                if (cos_s > 0 && nee_pdf_nee + nee_pdf_bsdf > 0) {
+                    const float4 brdf = mul4s(alb, 1.0f / kPi);
+                    const float G = cos_s * fabsf(cos_l) / (dist * dist);
+                    const float4 LE = make_float4(LM.emission[0], LM.emission[1], LM.emission[2],
+                                                  LM.emission[3]);
+                    const float4 Ld = mul4s(mul4s(mul4(LE, brdf), G), 1.0f / lpdf);
+                    p.pending[slot] = mul4s(mul4(Ld, thr), power_heuristic(nee_pdf_nee, nee_pdf_bsdf));
+                    // visible(): ray from p0 + v 1e-5, occluded when a hit has
+                    // t <= distance - 2e-5 (evaluated in double)
+                    const F3 so = add(hp, mul(wl, 1e-5f));
+                    const float tmax = __double2float_rd((double)dist - 1e-5 * 2);
+                    p.shadow_rays[2 * slot] = make_float4(so.x, so.y, so.z, tmax);
+                    p.shadow_rays[2 * slot + 1] = make_float4(wl.x, wl.y, wl.z, 0.0f);
+                    shadow = true;
+                }
+            }
+            if (GUIDED && !J.lights) uniforms4(J, pixel, sample, g + 2, u + 8);
+            bool cosine = true;
+            if (GUIDED && u[9] < alpha) {
+                cosine = false;
+                new_v = guide_draw(lobes, u[10], u[0], u[1]);
+#if DR_GUIDE_REFLECT
+                // a direction below the surface is mirrored into the upper
+                // hemisphere (guide_pdf_above is the density of the result)
+                const float cb = dot(new_v, n);
+                if (cb < 0.0f) new_v = sub(new_v, mul(n, 2.0f * cb));
+#endif
+            }
+            if (cosine) {
+                // cosineWeightedHemisphereSample (DistributionSamplers.hpp:33-42)
+                const float theta0 = 2 * kPi * u[0];
+                const float theta1 = pt::acos(1 - 2 * u[1]);
+                float sn0, cs0, sn1, cs1;
+                pt::sincos(theta0, sn0, cs0);
+                pt::sincos(theta1, sn1, cs1);
+                const F3 sph = f3(sn1 * sn0, sn1 * cs0, cs1);
+                new_v = normalized(add(sph, normal));
+            }
+            if (GUIDED) {
+                // one-sample MIS over the mixture and the cosine lobe: f cos / pdf_mix
+                const float c = dot(new_v, n);
+                const float pdf_mix = (alpha > 0.0f ? alpha * guide_density(lobes, new_v, n) : 0.0f) +
+                                      (1.0f - alpha) * fmaxf(c, 0.0f) / kPi;
+                const float f = c > 0.0f && pdf_mix > 0.0f ? c / (kPi * pdf_mix) : 0.0f;
+                thr = mul4s(mul4(thr, alb), f);
+                p.prev_pdf[slot] = pdf_mix;
+                if (f == 0.0f) dead = true;
+                const uint32_t rn = p.rec_n ? p.rec_n[slot] : (uint32_t)kGuideRecords;
+                if (!dead && alpha > 0.0f && rn < (uint32_t)kGuideRecords && b + 1 < (int)J.max_depth) {
+                    // 48-byte record as three 16-byte stores: hit point, normal,
+                    // direction, density, throughput (word 11, the radiance at
+                    // the next vertex, is written when that vertex closes it)
+                    float4 *rc = reinterpret_cast<float4 *>(p.rec + ((size_t)slot * kGuideRecords + rn) * kRecFloats);
+                    rc[0] = make_float4(hp.x, hp.y, hp.z, n.x);
+                    rc[1] = make_float4(n.y, n.z, new_v.x, new_v.y);
+                    rc[2] = make_float4(new_v.z, pdf_mix, luminance(thr), 0.0f);
+                    p.rec_n[slot] = (rn + 1) | kRecOpen;
+                }
+            } else {
+                thr = mul4(thr, alb);
+            }
+            new_o = hp;
+            p.prev_p[slot] = make_float4(hp.x, hp.y, hp.z, 1.0f);
+            p.prev_n[slot] = make_float4(n.x, n.y, n.z, 0.0f);
+        } else {
+            // transparent branch of generateNewRay (PathGeneration.hpp:138-208),
+            // including Stack::top() popping (:64-67); capacity 3
+            int4 st = p.stack[slot];
+            int stk[3] = {st.x, st.y, st.z};
+            int ss = st.w;
+            float n1, n2;
+            if (ss > 0 && stk[ss - 1] == obj) {
+                n1 = M.ior;
+                --ss;
+                if (ss == 0) n2 = 1;
+                else n2 = object_ior(p, stk[--ss]);
+                if (ss < 3) stk[ss++] = obj;
+            } else {
+                n2 = M.ior;
+                if (ss == 0) n1 = 1;
+                else n1 = object_ior(p, stk[--ss]);
+            }
+            const float eta = n1 / n2;
+            const float d = dot(rv, normal);
+            const float k = 1 - eta * eta * (1 - d * d);
+            if (n1 > n2 && k < 0) {
+                new_v = sub(rv, mul(mul(normal, 2.0f), d));
+            } else {
+                const float rr = (n1 - n2) / (n1 + n2);
+                const float R0 = rr * rr;
+                const float cosT1 = 1 - (-d);
+                const float c2 = cosT1 * cosT1;
+                const float c4 = c2 * c2;
+                const float c5 = c4 * cosT1;
+                const float F = (float)((double)R0 + (1.0 - (double)R0) * (double)c5);
+                if (u[2] < F) {
+                    new_v = sub(rv, mul(mul(normal, 2.0f), d));
+                } else {
+                    if (ss > 0 && stk[ss - 1] == obj) --ss;
+                    else if (ss < 3) stk[ss++] = obj;
+                    normal = mul(normal, -1.0f);
+                    const float dotp = -d;
+                    new_v = add(mul(normal, __fsqrt_rn(k) - dotp * eta), mul(rv, eta));
+                }
+            }
+            new_o = hp;
+            p.stack[slot] = make_int4(stk[0], stk[1], stk[2], ss);
+            p.prev_p[slot] = make_float4(hp.x, hp.y, hp.z, 0.0f);
+        }
+        new_o = add(new_o, mul(normal, 1e-5f));
+        p.rays[2 * slot] = make_float4(new_o.x, new_o.y, new_o.z, __int_as_float(0x7f800000));
+        p.rays[2 * slot + 1] = make_float4(new_v.x, new_v.y, new_v.z, 0.0f);
+        p.thr[slot] = thr;
+        p.color[slot] = col;
+        keep = b + 1 < (int)J.max_depth && !dead;
+    }
+}
+
+template <bool GUIDED>
+__global__ void __launch_bounds__(kRenderBlock, GUIDED ? DR_GUIDE_SHADE_BLOCKS : kShadeMinBlocks) k_shade(RenderParams p, int b, uint32_t at_least)
 {
     const uint32_t count = p.counts[b];
+    if (count < at_least) return;  // k_wave_paths has taken these paths to their ends
     const uint32_t *list = p.list[b & 1];
     uint32_t *next_list = p.list[(b + 1) & 1];
     // warp-uniform loop so that every lane reaches the ballots
@@ -524,240 +775,156 @@ __global__ void __launch_bounds__(kRenderBlock, GUIDED ? DR_GUIDE_SHADE_BLOCKS :
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t base = warp_first; base < count; base += stride) {
         const uint32_t i = base + (threadIdx.x & 31);
-        bool keep = false, shadow = false, dead = false;
+        bool keep = false, shadow = false;
         uint32_t slot = 0;
         if (i < count) {
             slot = list[i];
-            p.casts[slot] += 1;
-            const RenderJob &J = p.jobs[p.slot_job[slot]];
-            float *closed = nullptr;  // guided: the record this vertex closes
-            if (GUIDED && p.rec_n) {
-                // the radiance gathered before this vertex closes the last record
-                const uint32_t rn = p.rec_n[slot];
-                if (rn & kRecOpen) {
-                    const uint32_t r = (rn & ~kRecOpen) - 1;
-                    closed = p.rec + ((size_t)slot * kGuideRecords + r) * kRecFloats;
-                    closed[11] = luminance(p.color[slot]);
-                    p.rec_n[slot] = rn & ~kRecOpen;
-                }
-            }
-            const float2 h = p.hits[slot];
-            const int prim = __float_as_int(h.y);
-            if (prim >= 0) {
-                const float t = h.x;
-                const float4 r0 = p.rays[2 * slot], r1 = p.rays[2 * slot + 1];
-                const F3 ro = f3(r0.x, r0.y, r0.z), rv = f3(r1.x, r1.y, r1.z);
-                const float4 s0 = __ldg(p.shade + 3 * prim), s1 = __ldg(p.shade + 3 * prim + 1),
-                             s2 = __ldg(p.shade + 3 * prim + 2);
-                const F3 A = f3(s0.x, s0.y, s0.z), B = f3(s0.w, s1.x, s1.y), C = f3(s1.z, s1.w, s2.x);
-                const int obj = __float_as_int(s2.y), mat_id = __float_as_int(s2.z);
-                // getIntersectionTris (IntersectionTestsImpl.hpp:36-67), identity transform
-                F3 n = normalized(cross(sub(A, B), sub(A, C)));
-                if (dot(n, rv) > 0) n = mul(n, -1.0f);
-                n = normalized(f3(n.x * 1.0f, n.y * 1.0f, n.z * 1.0f));
-                F3 hp = add(ro, mul(rv, t));
-                hp = f3(hp.x * 1.0f + 0.0f, hp.y * 1.0f + 0.0f, hp.z * 1.0f + 0.0f);
-                const dr_material &M = p.materials[mat_id];
-                float4 thr = p.thr[slot];
-                float4 col = p.color[slot];
-                const float4 pp4 = p.prev_p[slot];
-                const uint32_t pixel = p.slot_pix[slot], sample = p.slot_sample[slot];
-                float u[12];
-                const uint32_t g = 1u + 3u * (uint32_t)b;
-                uniforms4(J, pixel, sample, g, u);
-                F3 normal = n;
-                F3 new_o, new_v;
-                if (M.kind == DR_MAT_DIFFUSE) {
-                    const float4 E = make_float4(M.emission[0], M.emission[1], M.emission[2], M.emission[3]);
-                    const float4 alb = make_float4(M.albedo[0], M.albedo[1], M.albedo[2], M.albedo[3]);
-                    // misWeightedEmission (PathGeneration.hpp:306-318) with the
-                    // pdfs of computeNextBounceMisPdfs (:320-334) for (prev, this)
-                    if (pp4.w == 0.0f) {
-                        col = add4(col, mul4(E, thr));
-                    } else {
-                        const float4 pn4 = p.prev_n[slot];
-                        const F3 pp = f3(pp4.x, pp4.y, pp4.z), pn = f3(pn4.x, pn4.y, pn4.z);
-                        // guided: the density of the direction actually sampled there
-                        const float pdf_bsdf = GUIDED ? p.prev_pdf[slot] : cosine_pdf(pp, hp, pn);
-                        const float L = luminance(mul4s(E, kPi));
-                        const float pdf_area = L / J.total_power;
-                        const float pdf_nee = pdf_area * area_to_solid_angle(pp, hp, n);
-                        if (pdf_bsdf + pdf_nee > 0) {
-                            const float wm = power_heuristic(pdf_bsdf, pdf_nee);
-                            col = add4(col, mul4s(mul4(E, thr), wm));
-#if DR_GUIDE_FULL_EMISSION
-                            // training only: the emission's share left to next-event
-                            // estimation (1 - wm) counts in the closed record's target
-                            if (GUIDED && closed) closed[11] -= luminance(mul4(E, thr)) * (1.0f - wm);
-#endif
-                        }
-                    }
-                    const float alpha = GUIDED && b < p.guide_bounces ? p.guide_alpha : 0.0f;
-#if DR_GUIDE_DECODED
-                    const float *lobes = GUIDED ? p.guide_y + (size_t)slot * kGuideOut : nullptr;
-#else
-                    GuideMix lobes;
-                    if (GUIDED && alpha > 0.0f) lobes = guide_mix(p.guide_y + (size_t)slot * kGuideOut);
-#endif
-                    // next-event estimation: samplePointOnLights (:234-272) and
-                    // evaluateDirectLighting (:336-361); visibility is the shadow ray
-                    if (J.lights) {
-                        uniforms4(J, pixel, sample, g + 1, u + 4);
-                        uniforms4(J, pixel, sample, g + 2, u + 8);
-                        int32_t oi, ti;
-                        float opdf, tpdf;
-                        alias_sample(p.light_table + J.obj_base, J.num_objects, u[3], u[4], oi, opdf);
-                        const dr_object ob = p.objects[J.obj_base + oi];
-                        alias_sample(p.tri_tables + ob.tri_begin, ob.tri_count, u[5], u[6], ti, tpdf);
-                        const int lt = (int)ob.tri_begin + ti;
-                        const float4 l0 = __ldg(p.shade + 3 * lt), l1 = __ldg(p.shade + 3 * lt + 1),
-                                     l2 = __ldg(p.shade + 3 * lt + 2);
-                        const F3 LA = f3(l0.x, l0.y, l0.z), LB = f3(l0.w, l1.x, l1.y), LC = f3(l1.z, l1.w, l2.x);
-                        float uu = u[7], vv = u[8];
-                        if (uu + vv > 1) {
-                            uu = 1 - uu;
-                            vv = 1 - vv;
-                        }
-                        F3 lp = add(add(LA, mul(sub(LB, LA), uu)), mul(sub(LC, LA), vv));
-                        const F3 Aw = f3(LA.x * 1.0f, LA.y * 1.0f, LA.z * 1.0f);
-                        const F3 Bw = f3(LB.x * 1.0f, LB.y * 1.0f, LB.z * 1.0f);
-                        const F3 Cw = f3(LC.x * 1.0f, LC.y * 1.0f, LC.z * 1.0f);
-                        const F3 perp = cross(sub(Aw, Bw), sub(Aw, Cw));
-                        const float plen = length(perp);
-                        const F3 ln = divs(perp, plen);
-                        const float area = plen / 2.0f;
-                        const float lpdf = opdf * tpdf / area;
-                        lp = f3(lp.x * 1.0f + 0.0f, lp.y * 1.0f + 0.0f, lp.z * 1.0f + 0.0f);
-                        const dr_material &LM = p.materials[ob.material];
-                        float nee_pdf_bsdf = cosine_pdf(hp, lp, n);
-                        if (GUIDED && alpha > 0.0f) {
-                            const F3 wl0 = normalized(sub(lp, hp));
-                            nee_pdf_bsdf = alpha * guide_density(lobes, wl0, n) + (1.0f - alpha) * nee_pdf_bsdf;
-                        }
-                        const float nee_pdf_nee = lpdf * area_to_solid_angle(hp, lp, ln);
-                        const float dist = length(sub(lp, hp));
-                        const F3 wl = divs(sub(lp, hp), dist);
-                        const float cos_s = dot(wl, n);
-                        const float cos_l = dot(wl, ln);
-                        if (cos_s > 0 && nee_pdf_nee + nee_pdf_bsdf > 0) {
-                            const float4 brdf = mul4s(alb, 1.0f / kPi);
-                            const float G = cos_s * fabsf(cos_l) / (dist * dist);
-                            const float4 LE = make_float4(LM.emission[0], LM.emission[1], LM.emission[2],
-                                                          LM.emission[3]);
-                            const float4 Ld = mul4s(mul4s(mul4(LE, brdf), G), 1.0f / lpdf);
-                            p.pending[slot] = mul4s(mul4(Ld, thr), power_heuristic(nee_pdf_nee, nee_pdf_bsdf));
-                            // visible(): ray from p0 + v 1e-5, occluded when a hit has
-                            // t <= distance - 2e-5 (evaluated in double)
-                            const F3 so = add(hp, mul(wl, 1e-5f));
-                            const float tmax = __double2float_rd((double)dist - 1e-5 * 2);
-                            p.shadow_rays[2 * slot] = make_float4(so.x, so.y, so.z, tmax);
-                            p.shadow_rays[2 * slot + 1] = make_float4(wl.x, wl.y, wl.z, 0.0f);
-                            shadow = true;
-                        }
-                    }
-                    if (GUIDED && !J.lights) uniforms4(J, pixel, sample, g + 2, u + 8);
-                    bool cosine = true;
-                    if (GUIDED && u[9] < alpha) {
-                        cosine = false;
-                        new_v = guide_draw(lobes, u[10], u[0], u[1]);
-#if DR_GUIDE_REFLECT
-                        // a direction below the surface is mirrored into the upper
-                        // hemisphere (guide_pdf_above is the density of the result)
-                        const float cb = dot(new_v, n);
-                        if (cb < 0.0f) new_v = sub(new_v, mul(n, 2.0f * cb));
-#endif
-                    }
-                    if (cosine) {
-                        // cosineWeightedHemisphereSample (DistributionSamplers.hpp:33-42)
-                        const float theta0 = 2 * kPi * u[0];
-                        const float theta1 = pt::acos(1 - 2 * u[1]);
-                        float sn0, cs0, sn1, cs1;
-                        pt::sincos(theta0, sn0, cs0);
-                        pt::sincos(theta1, sn1, cs1);
-                        const F3 sph = f3(sn1 * sn0, sn1 * cs0, cs1);
-                        new_v = normalized(add(sph, normal));
-                    }
-                    if (GUIDED) {
-                        // one-sample MIS over the mixture and the cosine lobe: f cos / pdf_mix
-                        const float c = dot(new_v, n);
-                        const float pdf_mix = (alpha > 0.0f ? alpha * guide_density(lobes, new_v, n) : 0.0f) +
-                                              (1.0f - alpha) * fmaxf(c, 0.0f) / kPi;
-                        const float f = c > 0.0f && pdf_mix > 0.0f ? c / (kPi * pdf_mix) : 0.0f;
-                        thr = mul4s(mul4(thr, alb), f);
-                        p.prev_pdf[slot] = pdf_mix;
-                        if (f == 0.0f) dead = true;
-                        const uint32_t rn = p.rec_n ? p.rec_n[slot] : (uint32_t)kGuideRecords;
-                        if (!dead && alpha > 0.0f && rn < (uint32_t)kGuideRecords && b + 1 < (int)J.max_depth) {
-                            // 48-byte record as three 16-byte stores: hit point, normal,
-                            // direction, density, throughput (word 11, the radiance at
-                            // the next vertex, is written when that vertex closes it)
-                            float4 *rc = reinterpret_cast<float4 *>(p.rec + ((size_t)slot * kGuideRecords + rn) * kRecFloats);
-                            rc[0] = make_float4(hp.x, hp.y, hp.z, n.x);
-                            rc[1] = make_float4(n.y, n.z, new_v.x, new_v.y);
-                            rc[2] = make_float4(new_v.z, pdf_mix, luminance(thr), 0.0f);
-                            p.rec_n[slot] = (rn + 1) | kRecOpen;
-                        }
-                    } else {
-                        thr = mul4(thr, alb);
-                    }
-                    new_o = hp;
-                    p.prev_p[slot] = make_float4(hp.x, hp.y, hp.z, 1.0f);
-                    p.prev_n[slot] = make_float4(n.x, n.y, n.z, 0.0f);
-                } else {
-                    // transparent branch of generateNewRay (PathGeneration.hpp:138-208),
-                    // including Stack::top() popping (:64-67); capacity 3
-                    int4 st = p.stack[slot];
-                    int stk[3] = {st.x, st.y, st.z};
-                    int ss = st.w;
-                    float n1, n2;
-                    if (ss > 0 && stk[ss - 1] == obj) {
-                        n1 = M.ior;
-                        --ss;
-                        if (ss == 0) n2 = 1;
-                        else n2 = object_ior(p, stk[--ss]);
-                        if (ss < 3) stk[ss++] = obj;
-                    } else {
-                        n2 = M.ior;
-                        if (ss == 0) n1 = 1;
-                        else n1 = object_ior(p, stk[--ss]);
-                    }
-                    const float eta = n1 / n2;
-                    const float d = dot(rv, normal);
-                    const float k = 1 - eta * eta * (1 - d * d);
-                    if (n1 > n2 && k < 0) {
-                        new_v = sub(rv, mul(mul(normal, 2.0f), d));
-                    } else {
-                        const float rr = (n1 - n2) / (n1 + n2);
-                        const float R0 = rr * rr;
-                        const float cosT1 = 1 - (-d);
-                        const float c2 = cosT1 * cosT1;
-                        const float c4 = c2 * c2;
-                        const float c5 = c4 * cosT1;
-                        const float F = (float)((double)R0 + (1.0 - (double)R0) * (double)c5);
-                        if (u[2] < F) {
-                            new_v = sub(rv, mul(mul(normal, 2.0f), d));
-                        } else {
-                            if (ss > 0 && stk[ss - 1] == obj) --ss;
-                            else if (ss < 3) stk[ss++] = obj;
-                            normal = mul(normal, -1.0f);
-                            const float dotp = -d;
-                            new_v = add(mul(normal, __fsqrt_rn(k) - dotp * eta), mul(rv, eta));
-                        }
-                    }
-                    new_o = hp;
-                    p.stack[slot] = make_int4(stk[0], stk[1], stk[2], ss);
-                    p.prev_p[slot] = make_float4(hp.x, hp.y, hp.z, 0.0f);
-                }
-                new_o = add(new_o, mul(normal, 1e-5f));
-                p.rays[2 * slot] = make_float4(new_o.x, new_o.y, new_o.z, __int_as_float(0x7f800000));
-                p.rays[2 * slot + 1] = make_float4(new_v.x, new_v.y, new_v.z, 0.0f);
-                p.thr[slot] = thr;
-                p.color[slot] = col;
-                keep = b + 1 < (int)J.max_depth && !dead;
-            }
+            shade_vertex<GUIDED>(p, b, slot, p.hits[slot], keep, shadow);
         }
         warp_append(keep, slot, next_list, p.counts + b + 1);
         warp_append(shadow, slot, p.shadow_list, p.counts + 64 + b);
+    }
+}
+
+// The rays of one warp in shared memory, ready to traverse: (o, tmax),
+// (v, root), (1 / v, target); target = the lane whose path the ray belongs to,
+// with kRayAny for its shadow ray.
+struct WarpRays {
+    float4 o[64], v[64], inv[64];
+};
+constexpr uint32_t kRayAny = 32u;
+
+struct WarpSource {
+    const WarpRays *rays;
+    const uint32_t *slots;  // per lane
+    float2 *hits;           // per lane
+    float4 *color;
+    const float4 *pending;
+    __device__ __forceinline__ uint32_t target(uint32_t i) const { return __float_as_uint(rays->inv[i].w); }
+    __device__ __forceinline__ bool is_any(uint32_t i) const { return target(i) & kRayAny; }
+    __device__ __forceinline__ bool load(uint32_t i, DevRay &r, uint32_t &root) const
+    {
+        const float4 o = rays->o[i], v = rays->v[i], inv = rays->inv[i];
+        r.o = make_float3(o.x, o.y, o.z);
+        r.v = make_float3(v.x, v.y, v.z);
+        r.inv = make_float3(inv.x, inv.y, inv.z);
+        r.tmax = o.w;
+        root = __float_as_uint(v.w);
+        return true;
+    }
+    __device__ __forceinline__ void closest(uint32_t i, float t, int32_t prim) const
+    {
+        hits[target(i)] = prim != INT_MAX ? make_float2(t, __int_as_float(prim))
+                                          : make_float2(__int_as_float(0x7f800000), __int_as_float(-1));
+    }
+    __device__ __forceinline__ void any(uint32_t i, bool occluded) const
+    {
+        if (!occluded) {
+            const uint32_t s = slots[target(i) & 31u];
+            color[s] = add4(color[s], pending[s]);
+        }
+    }
+};
+
+// Puts ray `q` (dr_ray, two float4) of this lane's path in place i.
+__device__ __forceinline__ void put_ray(WarpRays &rays, uint32_t i, const float4 *q, uint32_t root, uint32_t target)
+{
+    const float4 o = q[0], d = q[1];
+    DevRay r;
+    // a ray that cannot be traversed misses: it gets no root
+    if (!make_dev_ray(make_float3(o.x, o.y, o.z), make_float3(d.x, d.y, d.z), o.w, r)) root = kNoRoot;
+    rays.o[i] = o;
+    rays.v[i] = make_float4(d.x, d.y, d.z, __uint_as_float(root));
+    rays.inv[i] = make_float4(r.inv.x, r.inv.y, r.inv.z, __uint_as_float(target));
+}
+
+// The rest of every path of a wave, from bounce b0 on: each warp carries up to
+// 32 paths (one per lane) from vertex to vertex until they end, its up to 64 path
+// and shadow rays traced by the warp's teams of lanes (team.cuh), the vertices
+// shaded one per lane. `traced`: the paths' hits of bounce b0 are known, and the
+// kernel only runs when at most path_rays paths are left. The per-bounce kernels
+// cost two launches and the latency of the slowest of all rays and vertices per
+// bounce, some 60 us however few paths are left; here a path waits only for
+// the 31 others of its warp. Bound by instruction latency (0.48 of the issue
+// slots at 10 warps per SM); 5 blocks per SM (96 registers) against 4: box room
+// 256x256, 1 spp 464 against 511 us; 6 blocks 465 us.
+template <int MODE>
+__global__ void __launch_bounds__(kTraceBlock, 5) k_wave_paths(RenderParams p, int b0, bool traced)
+{
+    constexpr unsigned FULL = 0xffffffffu;
+    constexpr int W = kTraceBlock / 32;
+    const uint32_t count = p.counts[b0];
+    if (b0 > 0 && count > p.path_rays) return;
+    __shared__ WarpRays s_rays[W];
+    __shared__ uint32_t s_slot[W][32];
+    __shared__ float2 s_hit[W][32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned lower = (1u << lane) - 1u;
+    const uint32_t *list = p.list[b0 & 1];
+    const Wide8Args w{p.trace.nodes8, p.trace.tri_ref, p.trace.tri_wt, p.trace.prim, p.trace.num_nodes, p.trace.error,
+                      p.trace.stack_limit};
+    const WarpSource src{&s_rays[warp], s_slot[warp], s_hit[warp], p.color, p.pending};
+    // the first paths: an even share of the list; then, where there are more,
+    // new ones for the lanes that ended
+    const uint32_t warps = gridDim.x * W, id = blockIdx.x * W + warp;
+    const uint32_t share = min(32u, (count + warps - 1) / warps);
+    uint32_t at = (uint32_t)lane < share ? id * share + lane : count;
+    uint32_t given = warps * share;  // paths handed out before those of the counter
+    uint32_t slot = 0, root = 0;
+    int b = b0;
+    bool alive = false, shadow = false, known = false;
+    unsigned long long np = 0, ns = 0;
+    while (true) {
+        if (!alive && !shadow && at < count) {
+            slot = list[at];
+            at = count;
+            b = b0;
+            alive = true;
+            known = traced;
+            s_slot[warp][lane] = slot;
+            root = p.jobs[p.slot_job[slot]].root;
+        }
+        const unsigned path_rays = __ballot_sync(FULL, alive && !known), shadow_rays = __ballot_sync(FULL, shadow);
+        if (__ballot_sync(FULL, alive || shadow) == 0) break;
+        const uint32_t nrays = (uint32_t)(__popc(path_rays) + __popc(shadow_rays));
+        if (nrays != 0) {
+            if (alive && !known) put_ray(s_rays[warp], __popc(path_rays & lower), p.rays + 2 * (size_t)slot, root, lane);
+            if (shadow)
+                put_ray(s_rays[warp], __popc(path_rays) + __popc(shadow_rays & lower), p.shadow_rays + 2 * (size_t)slot, root,
+                        lane | kRayAny);
+            __syncwarp();
+            team_wide<MODE, kTeamPaths, 8>(w, src, WarpQueue<kTeamPaths>{nrays});
+            __syncwarp();
+        }
+        bool keep = false;
+        shadow = false;
+        if (alive) {
+            shade_vertex<false>(p, b, slot, known ? p.hits[slot] : s_hit[warp][lane], keep, shadow);
+            known = false;
+            ++b;
+        }
+        alive = keep;
+        np += keep;
+        ns += shadow;
+        // lanes that ended take further paths
+        if (given < count) {
+            const unsigned idle = __ballot_sync(FULL, !alive && !shadow);
+            if (idle != 0) {
+                uint32_t c = 0;
+                if (lane == 0) c = (uint32_t)atomicAdd(p.work + 64 + b0, (unsigned long long)__popc(idle));
+                c = given + __shfl_sync(FULL, c, 0);
+                if (!alive && !shadow) at = c + __popc(idle & lower);
+                if (c >= count) given = count;
+            }
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        np += __shfl_down_sync(FULL, np, o);
+        ns += __shfl_down_sync(FULL, ns, o);
+    }
+    if (lane == 0 && np + ns) {
+        atomicAdd(p.ray_totals, np);
+        atomicAdd(p.ray_totals + 1, ns);
     }
 }
 
@@ -1047,7 +1214,10 @@ dr_status WaveRunner::prepare(const std::vector<RenderJob> &jobs, const WavePlan
     const size_t need = wave_buffer_bytes(plan.max_slots, gr != nullptr);
     // occupancy of the persistent kernels, queried here so enqueue (which may
     // be under stream capture) only reads the cache
-    for (int mode = 0; mode < 2; ++mode) resident_blocks((const void *)select_p8(mode, cfg.stack), kTraceBlock);
+    for (int mode = 0; mode < 2; ++mode) {
+        resident_blocks((const void *)select_p8(mode, cfg.stack), kTraceBlock);
+        resident_blocks((const void *)(mode ? k_wave_paths<1> : k_wave_paths<0>), kTraceBlock);
+    }
     const uint32_t train_need = gr ? std::max<uint32_t>(1, gr->batch) * std::max<uint32_t>(1, gr->steps) : 0;
     bool grow = jobs.size() > jobs_capacity || plan.segs.size() > segs_capacity || train_need > train_cap;
     for (int k = 0; k < K; ++k) grow = grow || wave_bytes[k] < need;
@@ -1125,6 +1295,8 @@ dr_status WaveRunner::enqueue(const SceneArrays &sc, const WavePlan &plan, const
     const bool wt = tri_mode == DR_TRI_WATERTIGHT, wide = sc.trace.layout == 8;
     const WaveTrace p8 = select_p8(tri_mode, cfg.stack);
     const int trace_per_sm = resident_blocks((const void *)p8, kTraceBlock);
+    const auto paths = wt ? k_wave_paths<1> : k_wave_paths<0>;
+    const int paths_per_sm = resident_blocks((const void *)paths, kTraceBlock);
     DR_CUDA(cudaMemsetAsync(d_totals, 0, 2 * sizeof(unsigned long long), st));
     DR_CUDA(cudaEventRecord(fork, st));
     for (int k = 0; k < K; ++k) DR_CUDA(cudaStreamWaitEvent(stream[k], fork, 0));
@@ -1167,13 +1339,21 @@ dr_status WaveRunner::enqueue(const SceneArrays &sc, const WavePlan &plan, const
         DR_CUDA(cudaMemsetAsync(q.work, 0, 128 * sizeof(unsigned long long), ws));
         if (gr) DR_CUDA(cudaMemsetAsync(q.guide_counts, 0, 64 * sizeof(uint32_t), ws));
         k_camera<<<(W + kRenderBlock - 1) / kRenderBlock, kRenderBlock, 0, ws>>>(q);
-        for (int b = 0; b < (int)plan.max_depth; ++b) {
+        // (binary hierarchies and guided bounces keep the per-bounce kernels)
+        q.path_rays = wide ? (uint32_t)sms * kTailPathsPerSm : 0u;
+        const bool whole = wide && !gr && W <= (uint32_t)sms * kWholePathsPerSm;
+        const unsigned path_grid =
+            (unsigned)std::min<uint64_t>((W + kTraceBlock / 32 - 1) / (kTraceBlock / 32), (uint64_t)sms * paths_per_sm);
+        if (whole) paths<<<path_grid, kTraceBlock, 0, ws>>>(q, 0, false);
+        for (int b = 0; !whole && b < (int)plan.max_depth; ++b) {
+            const bool check = wide && tail_check(b) && b + 2 < (int)plan.max_depth && (!gr || b > (int)gr->bounces);
             if (wide) {
                 p8<<<trace_blocks(b), kTraceBlock, 0, ws>>>(q, b);
             } else {
                 if (wt) k_wave_closest<1, 2><<<trace_grid, kTraceBlock, 0, ws>>>(q, b);
                 else k_wave_closest<0, 2><<<trace_grid, kTraceBlock, 0, ws>>>(q, b);
             }
+            if (check) paths<<<path_grid, kTraceBlock, 0, ws>>>(q, b, true);
             // the guided shading kernel serves the guided bounces and the one
             // after them (its emission weights use the mixture density of the
             // last guided direction, and it closes that vertex's training
@@ -1185,16 +1365,16 @@ dr_status WaveRunner::enqueue(const SceneArrays &sc, const WavePlan &plan, const
                     DR_CUDA(launch_guide_infer(gr->guide, q.guide_pos, q.guide_nrm, q.guide_list, q.guide_counts + b,
                                                W, q.guide_y, ws, DR_GUIDE_DECODED != 0));
                 }
-                k_shade<true><<<shade_grid, kRenderBlock, 0, ws>>>(q, b);
+                k_shade<true><<<shade_grid, kRenderBlock, 0, ws>>>(q, b, 0u);
             } else {
-                k_shade<false><<<shade_grid, kRenderBlock, 0, ws>>>(q, b);
+                k_shade<false><<<shade_grid, kRenderBlock, 0, ws>>>(q, b, check ? q.path_rays + 1 : 0u);
             }
             if (!wide) {
                 if (wt) k_wave_shadow<1, 2><<<trace_grid, kTraceBlock, 0, ws>>>(q, b);
                 else k_wave_shadow<0, 2><<<trace_grid, kTraceBlock, 0, ws>>>(q, b);
             }
         }
-        if (wide) p8<<<trace_blocks((int)plan.max_depth), kTraceBlock, 0, ws>>>(q, (int)plan.max_depth);
+        if (wide && !whole) p8<<<trace_blocks((int)plan.max_depth), kTraceBlock, 0, ws>>>(q, (int)plan.max_depth);
         // images receive the waves in order
         if (w > 0) DR_CUDA(cudaStreamWaitEvent(ws, acc_done[(w - 1) % (uint32_t)K], 0));
         if (learn) {
