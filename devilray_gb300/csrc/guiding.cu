@@ -35,11 +35,6 @@ namespace {
 
 constexpr int kIn = 80, kHid = 64, kOut = 48, kLayers = 5;
 
-// CTAs per SM of the tcgen05 inference launch (at most 3 fit: 62.7 KB of
-// shared memory each).
-#ifndef DR_INFER_CTAS_PER_SM
-#define DR_INFER_CTAS_PER_SM 3
-#endif
 __host__ __device__ constexpr int fan_in(int l) { return l == 0 ? kIn : kHid; }
 __host__ __device__ constexpr int fan_out(int l) { return l == kLayers - 1 ? kOut : kHid; }
 
@@ -91,7 +86,7 @@ __device__ __forceinline__ void encode_pair(const float p[3], const float d[3], 
 {
     if (c < 72) {
         const int a = c / 24, k = (c % 24) >> 1;
-        const float x = ldexpf(p[a], k);  // exact: scaling by a power of two
+        const float x = p[a] * (float)(1 << k);  // exact: a power of two
         sincospif(x, &v0, &v1);
     } else if (c == 72) {
         v0 = d[0];
@@ -267,13 +262,19 @@ __global__ void __launch_bounds__(128) k_guide_infer(const __nv_bfloat16 *wb, co
 
 // ---- inference on the 5th-generation tensor cores (tcgen05) -------------------
 //
-// One CTA of 128 threads carries tiles of 128 rows (the M of one tcgen05.mma)
-// through the network: layer inputs and weights sit in shared memory in the
-// canonical K-major layout without swizzle, the one elected thread issues the
-// K/16 MMAs of a layer into a 128 x N FP32 accumulator in tensor memory and
-// commits them to an mbarrier, and each warp reads its 32 rows back with
-// tcgen05.ld for the bias / ReLU / BF16 epilogue, which writes the next
-// layer's input. Same arithmetic as k_guide_infer (BF16 products, FP32 sums).
+// One CTA per SM holds the weights in shared memory once, in the canonical
+// K-major layout without swizzle, and kInferGroups groups of 128 threads, each
+// with an input tile, 64 tensor-memory columns and an mbarrier of its own. A
+// group carries tiles of 128 rows (the M of one tcgen05.mma) through the
+// network: its first thread issues the K/16 MMAs of a layer into the 128 x N
+// FP32 accumulator and commits them to the mbarrier, and each warp reads its 32
+// rows back with tcgen05.ld for the bias / ReLU / BF16 epilogue, which writes
+// the next layer's input. Groups do not wait for one another: while one is in
+// its chain of MMA, commit, tensor-memory read and barrier, the others encode
+// inputs and run epilogues. Same arithmetic as k_guide_infer (BF16 products,
+// FP32 sums). Bound by that chain's latency with six tiles in flight (0.52 of the
+// issue slots, 0.59 of the shared / tensor memory data path, 0.24 of HBM for
+// 2^20 rows in 118 us; the sines and cosines of the inputs are 19 us of it).
 
 constexpr int kTcRows = 128;
 
@@ -306,7 +307,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t phase)
     return mbar_wait_bounded(mbar, phase, kMbarWaitPolls);
 }
 
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16])
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *v)
 {
     uint32_t r[16];
     asm volatile(
@@ -322,10 +323,16 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16])
 constexpr uint32_t kTcW0 = 0;                        // 64 x 80
 constexpr uint32_t kTcW1 = kTcW0 + 64 * 80 * 2;      // 3 x 64 x 64
 constexpr uint32_t kTcW4 = kTcW1 + 3 * 64 * 64 * 2;  // 48 x 64
-constexpr uint32_t kTcA = kTcW4 + 48 * 64 * 2 + 1024;  // 128 x 80 input / 128 x 64 hidden
-constexpr uint32_t kTcBias = kTcA + kTcRows * kIn * 2;
-constexpr uint32_t kTcBar = kTcBias + (4 * kHid + kOut) * 4;  // MMA mbarrier, TMEM address, copy mbarrier
-constexpr uint32_t kTcSmem = kTcBar + 24;
+constexpr uint32_t kTcA = kTcW4 + 48 * 64 * 2;       // per group: 128 x 80 input / 128 x 64 hidden / 128 x 40 output
+constexpr uint32_t kTcABytes = kTcRows * kIn * 2;
+static_assert(kTcABytes == kTcRows * kGuideOut * 4, "the output rows fit the input tile");
+// Groups per CTA: 6 run at 80 registers (2^20 rows: 118 us), 5 at 96 (128 us),
+// 7 at 72 (119 us), 8 spill at 64 (130 us). Three CTAs of one group each, with
+// their own copies of the weights, took 178 us.
+constexpr int kInferGroups = 6;
+constexpr uint32_t kTcBias = kTcA + kInferGroups * kTcABytes;
+constexpr uint32_t kTcBar = kTcBias + (4 * kHid + kOut) * 4;  // per group: MMA mbarrier; then copy mbarrier, TMEM address
+constexpr uint32_t kTcSmem = kTcBar + 8 * (kInferGroups + 2);
 
 // The weights as the tcgen05 kernels hold them in shared memory, kept in
 // global memory beside the BF16 copy so a CTA fetches them with one bulk
@@ -360,48 +367,76 @@ __device__ __forceinline__ void fetch_weight_image(uint32_t dst, const unsigned 
                  : "memory");
 }
 
-__global__ void __launch_bounds__(128) k_guide_infer_tc(const unsigned char *img, const float *params, GuideParams gp,
-                                                        const float *pos, const float *dir, const uint32_t *list,
-                                                        const uint32_t *count, uint32_t n_fixed, float *y,
-                                                        uint32_t *error, bool decoded)
+// BF16 pair (lo, hi) of max(x, 0), as the layers' inputs are rounded.
+__device__ __forceinline__ uint32_t relu_bf16(float lo, float hi)
+{
+    uint32_t d;
+    asm("cvt.rn.relu.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+    return d;
+}
+
+__device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %0, 128;\n" ::"r"(group + 1) : "memory"); }
+
+template <bool DECODED>
+__global__ void __launch_bounds__(128 * kInferGroups, 1)
+k_guide_infer_tc(const unsigned char *img, const float *params, GuideParams gp, const float *pos, const float *dir,
+                 const uint32_t *list, const uint32_t *count, uint32_t n_fixed, float *y, uint32_t *error)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
-    const int tid = threadIdx.x, warp = tid >> 5;
+    __shared__ int s_failed;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, group = tid >> 7, row = tid & 127;
+    const uint32_t n = count ? *count : n_fixed;
+    if ((uint64_t)blockIdx.x * kTcRows >= n) return;  // the whole block
     // weights in the canonical layout (B operands: N = outputs, K = inputs):
     // the forward part of the weight image, one bulk copy
-    const uint32_t cbar = smem_u32(smem + kTcBar + 16);
-    if (tid == 0) fetch_weight_image(smem_u32(smem + kTcW0), img, kImgFwdBytes, cbar);
-    float *bias = reinterpret_cast<float *>(smem + kTcBias);
-    for (int l = 0; l < kLayers; ++l)
-        for (int i = tid; i < fan_out(l); i += 128) bias[l * kHid + i] = params[b_off(l) + i];
-    const uint32_t mbar = smem_u32(smem + kTcBar);
-    const uint32_t tslot = smem_u32(smem + kTcBar + 8);
+    const uint32_t cbar = smem_u32(smem + kTcBar + 8 * kInferGroups);
+    const uint32_t tslot = cbar + 8, mbar = smem_u32(smem + kTcBar) + 8 * group;
     if (tid == 0) {
+        s_failed = 0;
+        fetch_weight_image(smem_u32(smem + kTcW0), img, kImgFwdBytes, cbar);
+    }
+    if (row == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(mbar) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
+    float *bias = reinterpret_cast<float *>(smem + kTcBias);
+    for (int i = tid; i < 4 * kHid + kOut; i += blockDim.x) bias[i] = params[b_off(i / kHid) + i % kHid];
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 128;\n" ::"r"(tslot) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;\n" ::"r"(tslot) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const uint32_t taddr = *reinterpret_cast<volatile uint32_t *>(smem + kTcBar + 8);
-    const uint32_t a_base = smem_u32(smem + kTcA);
-    const uint32_t w_base[kLayers] = {smem_u32(smem + kTcW0), smem_u32(smem + kTcW1), smem_u32(smem + kTcW1 + 8192),
-                                      smem_u32(smem + kTcW1 + 16384), smem_u32(smem + kTcW4)};
-    const uint32_t n = count ? *count : n_fixed;
+    const uint32_t taddr = *reinterpret_cast<volatile uint32_t *>(smem + kTcBar + 8 * kInferGroups + 8);
+    const uint32_t acc = taddr + 64u * group, lane_addr = acc + ((uint32_t)((warp & 3) * 32) << 16);
+    unsigned char *A = smem + kTcA + group * kTcABytes;
+    const uint32_t a_base = smem_u32(A);
     uint32_t phase = 0;
-    // the weights have landed (bounded wait, one decision for the block)
-    bool ok = __syncthreads_and(mbar_wait(cbar, 0) ? 1 : 0) != 0;
-    if (!ok && tid == 0) atomicOr(error, ERR_TIMEOUT);
-    for (uint32_t tile = blockIdx.x; ok && (uint64_t)tile * kTcRows < n; tile += gridDim.x) {
-        const uint32_t r = tile * kTcRows + tid;
+    // Every wait is bounded. A thread whose wait gives up (or that sees the
+    // block's flag) goes on through its group's barriers without working, so the
+    // block ends together.
+    auto wait = [&](uint32_t bar, uint32_t ph) {
+        if (*reinterpret_cast<volatile int *>(&s_failed)) return false;
+        if (mbar_wait(bar, ph)) return true;
+        *reinterpret_cast<volatile int *>(&s_failed) = 1;
+        atomicOr(error, ERR_TIMEOUT);
+        return false;
+    };
+    bool ok = wait(cbar, 0);  // the weights have landed
+    // tiles go to the blocks first, then to the groups of each block
+    for (uint32_t tile = blockIdx.x + gridDim.x * group; (uint64_t)tile * kTcRows < n; tile += gridDim.x * kInferGroups) {
+        const uint32_t r = tile * kTcRows + row;
         float p[3], d[3];
         uint32_t slot;
         load_row(pos, dir, list, n, r, gp, p, d, slot);
+        // the next tile's rows, while this one is carried through
+        const uint32_t ahead = r + 128u * gridDim.x * kInferGroups;
+        if (ahead < n) {
+            const uint32_t s2 = list ? list[ahead] : ahead;
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(pos + 3 * (size_t)s2));
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(dir + 3 * (size_t)s2));
+        }
         // input row: 10 chunks of 8 encoded columns
 #pragma unroll
         for (int j = 0; j < kIn / 8; ++j) {
@@ -412,80 +447,116 @@ __global__ void __launch_bounds__(128) k_guide_infer_tc(const unsigned char *img
                 encode_pair(p, d, 8 * j + 2 * k, v0, v1);
                 q[k] = pack_bf16(v0, v1);
             }
-            *reinterpret_cast<uint4 *>(smem + kTcA + canon_off(tid, 8 * j, kTcRows)) = make_uint4(q[0], q[1], q[2], q[3]);
+            *reinterpret_cast<uint4 *>(A + canon_off(row, 8 * j, kTcRows)) = make_uint4(q[0], q[1], q[2], q[3]);
         }
+        uint32_t w_base = smem_u32(smem + kTcW0);
+#pragma unroll 1
         for (int l = 0; l < kLayers; ++l) {
+            const int K = fan_in(l), N = fan_out(l);
             asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-            __syncthreads();
-            const int K = fan_in(l), N = fan_out(l);
-            if (tid == 0) {
+            group_sync(group);
+            if (row == 0 && ok) {
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 const uint32_t idesc = idesc_bf16(kTcRows, N);
-                for (int s2 = 0; s2 < K / 16; ++s2) {
-                    const uint64_t ad = smem_desc(a_base + (uint32_t)s2 * 2 * kTcRows * 16, kTcRows * 16, 128);
-                    const uint64_t bd = smem_desc(w_base[l] + (uint32_t)s2 * 2 * N * 16, (uint32_t)N * 16, 128);
+                uint64_t ad = smem_desc(a_base, kTcRows * 16, 128), bd = smem_desc(w_base, (uint32_t)N * 16, 128);
+#pragma unroll
+                for (int s2 = 0; s2 < kIn / 16; ++s2) {
+                    if (16 * s2 >= K) break;
                     asm volatile(
                         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(taddr),
+                        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(acc),
                         "l"(ad), "l"(bd), "r"(idesc), "r"(s2));
+                    ad += 2 * kTcRows * 16 / 16;  // the next 16 columns of both operands
+                    bd += 2 * N * 16 / 16;
                 }
                 asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(mbar)
                              : "memory");
             }
-            // one decision for the whole block: every thread waited (bounded) on the same phase
-            if (!__syncthreads_and(mbar_wait(mbar, phase) ? 1 : 0)) {
-                if (tid == 0) atomicOr(error, ERR_TIMEOUT);
-                ok = false;
-                break;
-            }
+            ok = wait(mbar, phase) && ok;
             phase ^= 1u;
+            w_base += (uint32_t)(K * N * 2);
+            __syncwarp();
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            const uint32_t lane_addr = taddr + ((uint32_t)(warp * 32) << 16);
-            float v[64];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                float t[16];
-                tmem_ld16(lane_addr + 16 * c, t);
-#pragma unroll
-                for (int i = 0; i < 16; ++i) v[16 * c + i] = t[i];
-            }
-            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-            const float *b = bias + l * kHid;
+            const float4 *b = reinterpret_cast<const float4 *>(bias + l * kHid);
             if (l < kLayers - 1) {
 #pragma unroll
-                for (int j = 0; j < kHid / 8; ++j) {
-                    uint32_t q[4];
+                for (int h = 0; h < 2; ++h) {
+                    float v[32];
+                    tmem_ld16(lane_addr + 32 * h, v);
+                    tmem_ld16(lane_addr + 32 * h + 16, v + 16);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        q[k] = pack_bf16(fmaxf(v[8 * j + 2 * k] + b[8 * j + 2 * k], 0.0f),
-                                         fmaxf(v[8 * j + 2 * k + 1] + b[8 * j + 2 * k + 1], 0.0f));
-                    *reinterpret_cast<uint4 *>(smem + kTcA + canon_off(tid, 8 * j, kTcRows)) =
-                        make_uint4(q[0], q[1], q[2], q[3]);
+                    for (int j = 0; j < 4; ++j) {
+                        uint32_t q[4];
+#pragma unroll
+                        for (int k = 0; k < 2; ++k) {
+                            const int i = 8 * j + 4 * k;
+                            const float4 c = b[8 * h + i / 4];
+                            const float2 x = __fadd2_rn(make_float2(v[i], v[i + 1]), make_float2(c.x, c.y));
+                            const float2 z = __fadd2_rn(make_float2(v[i + 2], v[i + 3]), make_float2(c.z, c.w));
+                            q[2 * k] = relu_bf16(x.x, x.y);
+                            q[2 * k + 1] = relu_bf16(z.x, z.y);
+                        }
+                        *reinterpret_cast<uint4 *>(A + canon_off(row, 32 * h + 8 * j, kTcRows)) =
+                            make_uint4(q[0], q[1], q[2], q[3]);
+                    }
                 }
-            } else if (slot != 0xffffffffu && decoded) {
-                float o[kGuideOut];
+            } else {
+                // the output rows, through shared memory (the tile's inputs are
+                // spent): each warp stages its 32 rows and writes them out as
+                // runs of 160 bytes, ten lanes per row
+                float o[48];
+                tmem_ld16(lane_addr, o);
+                tmem_ld16(lane_addr + 16, o + 16);
+                tmem_ld16(lane_addr + 32, o + 32);
+                asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
-                for (int i = 0; i < kGuideOut; ++i) o[i] = v[i] + b[i];
-                guide_store_decoded(y + (size_t)slot * kGuideOut, guide_mix_values(o));
-            } else if (slot != 0xffffffffu) {
-                float4 *dst = reinterpret_cast<float4 *>(y + (size_t)slot * kGuideOut);
+                for (int i = 0; i < kGuideOut / 4; ++i) {
+                    const float4 c = b[i];
+                    o[4 * i] += c.x, o[4 * i + 1] += c.y, o[4 * i + 2] += c.z, o[4 * i + 3] += c.w;
+                }
+                float4 out[kGuideOut / 4];
+                if (DECODED) {
+                    float v[kGuideOut];
 #pragma unroll
-                for (int j = 0; j < kGuideOut / 4; ++j)
-                    dst[j] = make_float4(v[4 * j] + b[4 * j], v[4 * j + 1] + b[4 * j + 1], v[4 * j + 2] + b[4 * j + 2],
-                                         v[4 * j + 3] + b[4 * j + 3]);
+                    for (int i = 0; i < kGuideOut; ++i) v[i] = o[i];
+                    guide_store_decoded(reinterpret_cast<float *>(out), guide_mix_values(v));
+                } else {
+#pragma unroll
+                    for (int j = 0; j < kGuideOut / 4; ++j) out[j] = make_float4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
+                }
+                // rows 4..7 of every 8 are turned by one float4, so that eight
+                // lanes' stores fall in distinct banks
+                constexpr int kQ = kGuideOut / 4;
+                float4 *stage = reinterpret_cast<float4 *>(A + (warp & 3) * 32 * kGuideOut * 4);
+                const int turn = (lane >> 2) & 1;
+#pragma unroll
+                for (int j = 0; j < kQ - 1; ++j) stage[lane * kQ + turn + j] = out[j];
+                stage[lane * kQ + (turn ? 0 : kQ - 1)] = out[kQ - 1];
+                __syncwarp();
+                const int part = lane / kQ, col = lane - part * kQ;
+#pragma unroll
+                for (int j = 0; j < 11; ++j) {
+                    const int at = 3 * j + part;
+                    const uint32_t to = __shfl_sync(0xffffffffu, slot, at & 31);
+                    if (part < 3 && at < 32 && to != 0xffffffffu && ok) {
+                        const int c = col + ((at >> 2) & 1);
+                        reinterpret_cast<float4 *>(y + (size_t)to * kGuideOut)[col] = stage[at * kQ + (c < kQ ? c : 0)];
+                    }
+                }
             }
         }
-        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-        __syncthreads();
+        group_sync(group);  // the staged rows are read before the next tile's inputs replace them
     }
     if (!ok) {
         // MMAs or the weight copy still in flight: wait again (bounded) before freeing their memory
-        mbar_wait(mbar, phase);
+        mbar_wait(mbar, phase ^ 1u);
         mbar_wait(cbar, 0);
     }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 128;\n" ::"r"(taddr) : "memory");
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;\n" ::"r"(taddr) : "memory");
 }
 
 // ---- training -----------------------------------------------------------------
@@ -1233,9 +1304,10 @@ cudaError_t launch_guide_infer(const dr_guide *g, const float *pos, const float 
     if (max_rows == 0) return cudaSuccess;
     if (g->cfg.infer_kernel == DR_GUIDE_INFER_TCGEN05) {
         const unsigned tiles = (max_rows + kTcRows - 1) / kTcRows;
-        const unsigned blocks = std::min<unsigned>(tiles, (unsigned)g->ctx->num_sms * DR_INFER_CTAS_PER_SM);
-        k_guide_infer_tc<<<blocks, 128, kTcSmem, st>>>(g->img, g->params, guide_params(g), pos, dir, list, count,
-                                                       max_rows, y, g->ctx->d_error, decoded);
+        const unsigned blocks = std::min<unsigned>(tiles, (unsigned)g->ctx->num_sms);
+        const auto kernel = decoded ? k_guide_infer_tc<true> : k_guide_infer_tc<false>;
+        kernel<<<blocks, 128 * kInferGroups, kTcSmem, st>>>(g->img, g->params, guide_params(g), pos, dir, list, count,
+                                                            max_rows, y, g->ctx->d_error);
     } else {
         const unsigned tiles = (max_rows + 15) / 16;
         const unsigned blocks = std::min<unsigned>((tiles + 3) / 4, (unsigned)g->ctx->num_sms * 4);
@@ -1271,7 +1343,8 @@ dr_status dr_guide_create(dr_context *ctx, const dr_guide_config *cfg, dr_guide 
     if (!attr) {
         DR_CUDA(cudaFuncSetAttribute(k_guide_infer, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInferSmem));
         DR_CUDA(cudaFuncSetAttribute(k_guide_train_fb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrainSmem));
-        DR_CUDA(cudaFuncSetAttribute(k_guide_infer_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
+        DR_CUDA(cudaFuncSetAttribute(k_guide_infer_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
+        DR_CUDA(cudaFuncSetAttribute(k_guide_infer_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
         DR_CUDA(cudaFuncSetAttribute(k_guide_train_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTfSmem));
         attr = true;
     }

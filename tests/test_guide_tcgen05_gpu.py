@@ -64,3 +64,34 @@ def test_tcgen05_training_matches_mma_sync(native, ctx, n):
     a, b = g_tc.astype(np.float64), g_ms.astype(np.float64)
     rel = np.linalg.norm(a - b) / np.linalg.norm(b)
     assert rel <= 1e-2, rel
+
+
+def test_tcgen05_rows_do_not_depend_on_the_launch(native, ctx):
+    """Row counts around the tiles (128 rows), the blocks (one per SM) and the
+    groups of a block (six): every row has the bits it has in the largest
+    launch, whichever tile, group and pass carries it, and no other row is
+    written; the largest launch agrees with the mma.sync kernel."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    big = 2 * 6 * 128 * sms + 130
+    rng = np.random.default_rng(11)
+    tc = native.Guide(ctx, seed=6, half_extent=10.0, infer_kernel=0)
+    ms = native.Guide(ctx, seed=6, half_extent=10.0, infer_kernel=1)
+    pos = torch.from_numpy(rng.uniform(-11, 11, (big, 3)).astype(np.float32)).cuda()
+    d = rng.normal(size=(big, 3))
+    nrm = torch.from_numpy((d / np.linalg.norm(d, axis=1, keepdims=True)).astype(np.float32)).cuda()
+
+    def run(g, n):
+        y = torch.full((big, 40), float("nan"), dtype=torch.float32, device="cuda")
+        g.infer(pos, nrm, n, y)
+        return y
+
+    want = run(tc, big)
+    assert bool(torch.isfinite(want).all())
+    for n in (1, 127, 128, 129, 128 * sms, 128 * sms + 1, 6 * 128 * sms, 6 * 128 * sms + 1, big - 1):
+        y = run(tc, n)
+        assert torch.equal(y[:n], want[:n]), n
+        assert bool(torch.isnan(y[n:]).all()), n
+    ctx.check()
+    err = (want - run(ms, big)).abs()
+    scale = float(want.abs().max()) + 1e-6
+    assert float(err.median()) <= 1e-6 * scale + 1e-7 and float(err.max()) <= 2e-2 * scale
