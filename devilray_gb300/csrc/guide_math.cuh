@@ -154,6 +154,46 @@ __host__ __device__ inline float guide_loss_grad(const float *y, float wx, float
     return logq;
 }
 
+// The same gradient by lobe, for threads that share a row. The mixture's log
+// density is LSE(u) - LSE(logits), u_j = logit_j + log vMF_j; the caller forms
+// both sums over the lobes (pi = exp(logit - LSE(logits)), resp = exp(u - LSE(u))).
+struct GuideLobeTerm {
+    float u, kappa, cosang, inv_n;  // inv_n = 1 / |mean|, 0 for a mean too short to have a direction
+    float mx, my, mz;
+};
+
+__host__ __device__ inline GuideLobeTerm guide_lobe_term(const float *y, float wx, float wy, float wz)
+{
+    GuideLobeTerm t;
+    const float lk = fminf(fmaxf(y[1], kGuideLogKMin), kGuideLogKMax);
+    const float k = guide_exp(lk);
+    const float n2 = y[2] * y[2] + y[3] * y[3] + y[4] * y[4];
+    const bool deg = n2 < 1e-24f;
+    const float r = deg ? 0.0f : 1.0f / sqrtf(n2);
+    t.kappa = k;
+    t.inv_n = r;
+    t.mx = y[2] * r, t.my = y[3] * r, t.mz = deg ? 1.0f : y[4] * r;
+    t.cosang = t.mx * wx + t.my * wy + t.mz * wz;
+    // log of the normalisation: log kappa - log 2 pi - log(1 - e^{-2 kappa}); kappa >= e^-4 needs no series
+    t.u = y[0] + (lk - 1.83787706641f - log1pf(-guide_exp(-2.0f * k))) + k * (t.cosang - 1.0f);
+    return t;
+}
+
+__host__ __device__ inline void guide_lobe_grad(const float *y, const GuideLobeTerm &t, float pi, float resp, float wx, float wy,
+                                                float wz, float scale, float *dy)
+{
+    const float k = t.kappa;
+    dy[0] = -scale * (resp - pi);
+    const bool clamped = y[1] < kGuideLogKMin || y[1] > kGuideLogKMax;
+    // d log p / d kappa = 1/kappa - 2 / (e^{2 kappa} - 1) + cos - 1
+    const float dk = 1.0f / k - 2.0f / expm1f(2.0f * k) + t.cosang - 1.0f;
+    dy[1] = clamped ? 0.0f : -scale * resp * dk * k;
+    const float g = -scale * resp * k * t.inv_n;
+    dy[2] = g * (wx - t.cosang * t.mx);
+    dy[3] = g * (wy - t.cosang * t.my);
+    dy[4] = g * (wz - t.cosang * t.mz);
+}
+
 #if defined(__CUDACC__)
 // The mixture as the shading kernel uses it: the network output decoded once
 // per vertex, each lobe's vMF normalisation folded into its weight, so that a

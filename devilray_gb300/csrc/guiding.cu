@@ -336,11 +336,9 @@ constexpr uint32_t kTcSmem = kTcBar + 8 * (kInferGroups + 2);
 
 // The weights as the tcgen05 kernels hold them in shared memory, kept in
 // global memory beside the BF16 copy so a CTA fetches them with one bulk
-// asynchronous copy: [0, 40960) the forward operands (kTcW0..kTcW4: W_l as
-// N = out, K = in, canonical K-major), [40960, 71680) the backward operands of
-// layers 1..4 (W_l as N = in 64, K = out).
-constexpr uint32_t kImgFwdBytes = 40960;
-constexpr uint32_t kImgBytes = kImgFwdBytes + 3 * kHid * kHid * 2 + kHid * kOut * 2;
+// asynchronous copy: W_l at kTcW0..kTcW4 as N = out, K = in, canonical K-major
+// (the backward product reads the same bytes MN-major).
+constexpr uint32_t kImgBytes = kNumWeights * 2;
 
 __device__ __forceinline__ void store_weight(__nv_bfloat16 *wb, unsigned char *img, int l, int idx, float p)
 {
@@ -349,10 +347,6 @@ __device__ __forceinline__ void store_weight(__nv_bfloat16 *wb, unsigned char *i
     const int o = idx / fan_in(l), in = idx % fan_in(l);
     const uint32_t fwd = l == 0 ? kTcW0 : l == 4 ? kTcW4 : kTcW1 + (uint32_t)(l - 1) * kHid * kHid * 2;
     *reinterpret_cast<__nv_bfloat16 *>(img + fwd + canon_off(o, in, fan_out(l))) = b;
-    if (l > 0) {
-        const uint32_t bwd = kImgFwdBytes + (uint32_t)(l - 1) * kHid * kHid * 2;
-        *reinterpret_cast<__nv_bfloat16 *>(img + bwd + canon_off(in, o, kHid)) = b;
-    }
 }
 
 // One bulk asynchronous copy of `bytes` of the weight image into shared
@@ -388,12 +382,12 @@ k_guide_infer_tc(const unsigned char *img, const float *params, GuideParams gp, 
     const uint32_t n = count ? *count : n_fixed;
     if ((uint64_t)blockIdx.x * kTcRows >= n) return;  // the whole block
     // weights in the canonical layout (B operands: N = outputs, K = inputs):
-    // the forward part of the weight image, one bulk copy
+    // the weight image, one bulk copy
     const uint32_t cbar = smem_u32(smem + kTcBar + 8 * kInferGroups);
     const uint32_t tslot = cbar + 8, mbar = smem_u32(smem + kTcBar) + 8 * group;
     if (tid == 0) {
         s_failed = 0;
-        fetch_weight_image(smem_u32(smem + kTcW0), img, kImgFwdBytes, cbar);
+        fetch_weight_image(smem_u32(smem + kTcW0), img, kImgBytes, cbar);
     }
     if (row == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(mbar) : "memory");
@@ -746,86 +740,95 @@ __global__ void __launch_bounds__(128) k_guide_train_fb(const __nv_bfloat16 *wb,
     store_t<8>(tb.deltaT[0], tb.rows, r0, dacc, n, kHid);
 }
 
-// Issues the K/16 MMAs of one product into the accumulator at taddr
-// (accumulating from the first when `acc`).
-__device__ __forceinline__ void tc_mma_chain(uint32_t taddr, uint32_t a_base, uint32_t b_base, int M, int N, int K,
-                                             bool acc)
-{
-    const uint32_t idesc = idesc_bf16(M, N);
-    for (int s2 = 0; s2 < K / 16; ++s2) {
-        const uint64_t ad = smem_desc(a_base + (uint32_t)s2 * 2 * M * 16, (uint32_t)M * 16, 128);
-        const uint64_t bd = smem_desc(b_base + (uint32_t)s2 * 2 * N * 16, (uint32_t)N * 16, 128);
-        const uint32_t en = (acc || s2 > 0) ? 1u : 0u;
-        asm volatile(
-            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-            " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(taddr),
-            "l"(ad), "l"(bd), "r"(idesc), "r"(en));
-    }
-}
-
 // ---- training on the 5th-generation tensor cores (tcgen05) ----------------------
 //
-// One CTA of 128 threads carries 128-row tiles through the forward pass, the
-// loss gradient, the backward deltas and the weight gradients, with the same
-// arithmetic as k_guide_train_fb + k_guide_wgrad (BF16 operands, FP32 sums;
-// deltas enter the tensor cores as a BF16 high part plus a BF16 remainder):
-// thread t owns row t of the tile. Forward layer l: D[128 x out] = x_l W_l^T
-// as in k_guide_infer_tc. Backward layer l: D[128 x in] = delta_hi W_l +
-// delta_lo W_l, with W_l staged as the N = in, K = out operand. Every layer
-// input x_l stays in shared memory for the whole tile, and the delta tile
-// holds [delta_hi | delta_lo] as one 128 x 128 matrix. Both serve twice, through two
-// descriptors of the same bytes: K-major (the forward product over inputs,
-// the backward product over outputs) and MN-major (the weight-gradient
-// product over rows): dW_l[128 x (in + 16)] += [delta_hi | delta_lo]^T x_l,
-// whose rows 0-63 and 64-127 are the high and low parts of dW_l. The 16 extra
-// columns of x_l hold 1.0, so column `in` of the product is the bias
-// gradient. The per-layer sums stay in tensor memory across the CTA's tiles
-// and are added to the gradient once, at the end. Measured per Adam step:
-// 16,384 rows 0.108 ms, 65,536 rows 0.166 ms (mma.sync forward/backward plus
-// weight-gradient kernel: 0.180 and 0.545 ms).
+// One CTA of 512 threads per SM carries 128-row tiles through the forward pass,
+// the loss gradient, the backward deltas and the weight gradients, with the
+// same arithmetic as k_guide_train_fb + k_guide_wgrad (BF16 operands, FP32
+// sums; deltas enter the tensor cores as a BF16 high part plus a BF16
+// remainder). Four threads share a row: warp w reads the tensor-memory lanes of
+// rows 32 (w & 3) .., and w >> 2 picks a quarter of the columns (or two of the
+// eight lobes), so the serial work between two matrix products is a quarter of
+// a row's. Forward layer l: D[128 x out] = x_l W_l^T as in k_guide_infer_tc.
+// Backward layer l: D[128 x in] = delta_hi W_l + delta_lo W_l, the forward
+// weights read through an MN-major descriptor. Every layer input x_l stays in
+// shared memory for the whole tile, and a delta tile holds [delta_hi |
+// delta_lo] as one 128 x 128 matrix. Both serve twice, through two descriptors of
+// the same bytes: K-major (the forward product over inputs, the backward
+// product over outputs) and MN-major (the weight-gradient product over rows):
+// dW_l[128 x (in + 16)] += [delta_hi | delta_lo]^T x_l, whose rows 0-63 and
+// 64-127 are the high and low parts of dW_l. The 16 extra columns of x_l hold
+// 1.0, so column `in` of the product is the bias gradient. Two delta tiles
+// alternate between layers, so the weight gradient of a layer runs while the
+// next delta is formed. The per-layer sums stay in tensor memory across the
+// CTA's tiles; each CTA writes its sums to a row of `parts`, and k_guide_adam
+// adds the rows in order, so a step has the same bits every time. Bound by the
+// ten dependent matrix products of a tile (3 us per 128 rows; 0.30 of the issue
+// slots, 0.09 of the tensor pipe). An Adam step of 65,536 rows takes 63 us; with
+// one thread per row, 128 threads per CTA and atomic adds of the sums it took
+// 153 us (20 us of it the atomics).
 
 // Shared memory of k_guide_train_fused (byte offsets).
+constexpr int kTfThreads = 512;
 constexpr uint32_t kTfX0 = 0;                                  // x_0: 128 x (80 + 16)
 constexpr uint32_t kTfX1 = kTfX0 + 12 * 2048;                  // x_1..x_4: 128 x (64 + 16) each
-constexpr uint32_t kTfD = kTfX1 + 4 * 10 * 2048;               // [delta_hi | delta_lo]: 128 x 128
-constexpr uint32_t kTfW = kTfD + 16 * 2048;                    // forward weights, as kTcW0..kTcW4
-constexpr uint32_t kTfWT1 = kTfW + 40960;                      // W_l as [in 64][out 64], l = 1..3
-constexpr uint32_t kTfWT4 = kTfWT1 + 3 * kHid * kHid * 2;      // W_4 as [in 64][out 48]
-constexpr uint32_t kTfBias = kTfWT4 + kHid * kOut * 2;
-constexpr uint32_t kTfBar = kTfBias + (4 * kHid + kOut) * 4;  // MMA mbarrier, TMEM address, copy mbarrier
+constexpr uint32_t kTfD = kTfX1 + 4 * 10 * 2048;               // two tiles [delta_hi | delta_lo]: 128 x 128
+constexpr uint32_t kTfW = kTfD + 2 * 16 * 2048;                // forward weights, as kTcW0..kTcW4
+constexpr uint32_t kTfBias = kTfW + kImgBytes;
+constexpr uint32_t kTfLse = kTfBias + (4 * kHid + kOut) * 4;   // [part][row] running maxima and sums of the loss
+constexpr uint32_t kTfBar = kTfLse + 4 * kTcRows * 16;         // MMA mbarrier, TMEM address, copy mbarrier
 constexpr uint32_t kTfSmem = kTfBar + 24;
-static_assert(kTfWT1 == kTfW + kImgFwdBytes && kTfBias == kTfW + kImgBytes, "the weight image is one copy");
 // tensor-memory columns: [0, 64) the forward / backward product, then dW_l
 __host__ __device__ constexpr uint32_t tf_dcol(int l) { return l == 0 ? 64u : 160u + 80u * (uint32_t)(l - 1); }
+// 16-column chunks of dW_l (weights and the bias column), numbered over all layers
+__host__ __device__ constexpr int tf_chunks(int l) { return fan_in(l) / 16 + 1; }
+__host__ __device__ constexpr int tf_chunk0(int l) { return l == 0 ? 0 : tf_chunk0(l - 1) + tf_chunks(l - 1); }
+constexpr int kTfStage = 20;  // floats per staged row of a chunk: 16 and a pad that spreads the banks
+static_assert(tf_chunk0(kLayers) * 64 * kTfStage * 4 <= (int)kTfW, "the staged gradients fit the tiles");
+// floats of one CTA's row of partial sums: the gradients, the loss
+constexpr int kPartStride = (kNumParams + 1 + 31) & ~31;
+constexpr int kWeightParts = 64;  // blocks of k_guide_weight_sum
 
-// Instruction descriptor of kind::f16 with both operands MN-major (bits 15, 16).
-__host__ __device__ constexpr uint32_t idesc_bf16_mn(int M, int N) { return idesc_bf16(M, N) | (1u << 15) | (1u << 16); }
+__device__ __forceinline__ void tc_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool accumulate)
+{
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"(accumulate ? 1u : 0u));
+}
 
-__global__ void __launch_bounds__(128) k_guide_train_fused(const unsigned char *img, const float *params,
-                                                           GuideParams gp, const float *pos, const float *dir,
-                                                           const float *sdir, const float *weight, uint32_t n,
-                                                           const float *weight_sum, float *grad, float *loss,
-                                                           uint32_t *error)
+// Splits a pair into its BF16 high part and the BF16 rounding of the rest.
+__device__ __forceinline__ void split_bf16(float c0, float c1, uint32_t &hi, uint32_t &lo)
+{
+    const __nv_bfloat162 h = __floats2bfloat162_rn(c0, c1);
+    const float2 hf = __bfloat1622float2(h);
+    hi = *reinterpret_cast<const uint32_t *>(&h);
+    lo = pack_bf16(c0 - hf.x, c1 - hf.y);
+}
+
+__global__ void __launch_bounds__(kTfThreads, 1)
+k_guide_train_fused(const unsigned char *img, const float *params, GuideParams gp, const float *pos, const float *dir,
+                    const float *sdir, const float *weight, uint32_t n, const float *weight_parts, uint32_t nweight,
+                    float *parts, uint32_t *error)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ float s_loss[4];
+    __shared__ int s_failed;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // forward (N = out, K = in) and backward (N = in, K = out) weights: the
-    // weight image, one bulk copy
+    const int row = 32 * (warp & 3) + lane, part = warp >> 2;
     const uint32_t cbar = smem_u32(smem + kTfBar + 16);
+    if (tid == 0) s_failed = 0;
     if (tid == 0) fetch_weight_image(smem_u32(smem + kTfW), img, kImgBytes, cbar);
     float *bias = reinterpret_cast<float *>(smem + kTfBias);
-    for (int l = 0; l < kLayers; ++l)
-        for (int i = tid; i < fan_out(l); i += 128) bias[l * kHid + i] = params[b_off(l) + i];
+    for (int i = tid; i < 4 * kHid + kOut; i += kTfThreads) bias[i] = params[b_off(i / kHid) + i % kHid];
     const uint32_t xoff[kLayers] = {kTfX0, kTfX1, kTfX1 + 20480, kTfX1 + 40960, kTfX1 + 61440};
     // the columns of ones (in .. in + 15) of every x_l
-    {
+    if (part < 2) {
         const uint32_t one2 = 0x3f803f80u;
 #pragma unroll
         for (int l = 0; l < kLayers; ++l)
-#pragma unroll
-            for (int j = 0; j < 2; ++j)
-                *reinterpret_cast<uint4 *>(smem + xoff[l] + canon_off(tid, fan_in(l) + 8 * j, kTcRows)) =
-                    make_uint4(one2, one2, one2, one2);
+            *reinterpret_cast<uint4 *>(smem + xoff[l] + canon_off(row, fan_in(l) + 8 * part, kTcRows)) =
+                make_uint4(one2, one2, one2, one2);
     }
     const uint32_t mbar = smem_u32(smem + kTfBar);
     const uint32_t tslot = smem_u32(smem + kTfBar + 8);
@@ -842,199 +845,272 @@ __global__ void __launch_bounds__(128) k_guide_train_fused(const unsigned char *
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t taddr = *reinterpret_cast<volatile uint32_t *>(smem + kTfBar + 8);
-    const uint32_t d_base = smem_u32(smem + kTfD), dlo_base = d_base + 8 * 2048;
-    uint32_t x_base[kLayers];
-#pragma unroll
-    for (int l = 0; l < kLayers; ++l) x_base[l] = smem_u32(smem + xoff[l]);
-    const uint32_t w_base[kLayers] = {smem_u32(smem + kTfW + kTcW0), smem_u32(smem + kTfW + kTcW1),
-                                      smem_u32(smem + kTfW + kTcW1 + 8192), smem_u32(smem + kTfW + kTcW1 + 16384),
-                                      smem_u32(smem + kTfW + kTcW4)};
-    const uint32_t wt_base[kLayers] = {0, smem_u32(smem + kTfWT1), smem_u32(smem + kTfWT1 + 8192),
-                                       smem_u32(smem + kTfWT1 + 16384), smem_u32(smem + kTfWT4)};
-    const uint32_t lane_addr = taddr + ((uint32_t)(warp * 32) << 16);
-    const float wmean = *weight_sum / (float)n;
+    const uint32_t lane_addr = taddr + ((uint32_t)(32 * (warp & 3)) << 16);
+    const uint32_t d_base = smem_u32(smem + kTfD), w_img = smem_u32(smem + kTfW);
+    // mean sample weight: the same sum in every thread of every block
+    float wsum = (uint32_t)lane < nweight ? weight_parts[lane] : 0.0f;
+    if ((uint32_t)lane + 32 < nweight) wsum += weight_parts[lane + 32];
+    for (int o = 16; o > 0; o >>= 1) wsum += __shfl_xor_sync(0xffffffffu, wsum, o);
+    const float wmean = wsum / (float)n;
+    float loss_sum = 0.0f;  // of the part 0 threads' rows
     uint32_t phase = 0;
-    // the weights have landed (bounded wait, one decision for the block)
-    bool ok = __syncthreads_and(mbar_wait(cbar, 0) ? 1 : 0) != 0, first = true;
-    if (!ok && tid == 0) atomicOr(error, ERR_TIMEOUT);
+    bool first = true;
+    if (!mbar_wait(cbar, 0)) {  // the weights have landed
+        *reinterpret_cast<volatile int *>(&s_failed) = 1;
+        atomicOr(error, ERR_TIMEOUT);
+    }
 
-    auto run = [&](auto issue) -> bool {
+    // The products of one step, issued by one thread once every thread's shared-memory
+    // stores are done; `issue` commits them to the mbarrier.
+    auto launch = [&](auto issue) {
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
         __syncthreads();
         if (tid == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             issue();
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(mbar)
-                         : "memory");
         }
-        if (!__syncthreads_and(mbar_wait(mbar, phase) ? 1 : 0)) {
-            if (tid == 0) atomicOr(error, ERR_TIMEOUT);
-            return false;
+    };
+    auto commit = [&] {
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(mbar) : "memory");
+    };
+    // Waits for the last commit (which covers every product issued before it).
+    // Every wait is bounded; once one gives up the block runs on without waiting,
+    // so that it ends together, and its sums are dropped.
+    auto finish = [&] {
+        if (!*reinterpret_cast<volatile int *>(&s_failed) && !mbar_wait(mbar, phase)) {
+            *reinterpret_cast<volatile int *>(&s_failed) = 1;
+            atomicOr(error, ERR_TIMEOUT);
         }
         phase ^= 1u;
+        __syncwarp();
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        return true;
     };
     // dW_l += [delta_hi | delta_lo]^T x_l over the tile's 128 rows (8 MMAs of
     // 16 rows; MN-major operands: 8-row groups 128 B apart, 8-column groups
     // 2048 B apart)
     auto wgrad = [&](int l, bool acc) {
-        const uint32_t idesc = idesc_bf16_mn(kTcRows, fan_in(l) + 16);
-        for (int s2 = 0; s2 < kTcRows / 16; ++s2) {
-            const uint64_t ad = smem_desc(d_base + (uint32_t)s2 * 256, 128, 2048);
-            const uint64_t bd = smem_desc(x_base[l] + (uint32_t)s2 * 256, 128, 2048);
-            const uint32_t en = (acc || s2 > 0) ? 1u : 0u;
-            asm volatile(
-                "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(taddr + tf_dcol(l)),
-                "l"(ad), "l"(bd), "r"(idesc), "r"(en));
-        }
+        const uint32_t idesc = idesc_bf16(kTcRows, fan_in(l) + 16) | (1u << 15) | (1u << 16);
+        uint64_t a = smem_desc(d_base + (uint32_t)(l & 1) * 32768, 128, 2048), b = smem_desc(smem_u32(smem) + xoff[l], 128, 2048);
+#pragma unroll
+        for (int s2 = 0; s2 < kTcRows / 16; ++s2, a += 16, b += 16) tc_mma(taddr + tf_dcol(l), a, b, idesc, acc || s2 > 0);
     };
-    auto read_acc = [&](float (&v)[64], uint32_t col, int ncols) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            if (16 * c >= ncols) break;
-            float t[16];
-            tmem_ld16(lane_addr + col + 16 * c, t);
-#pragma unroll
-            for (int i = 0; i < 16; ++i) v[16 * c + i] = t[i];
-        }
-        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-    };
-    // [delta_hi | delta_lo] row of this thread: 8-column chunks j of K = ncols
-    auto put_delta = [&](const float *dv, int ncols) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            uint32_t hi[4], lo[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int i0 = 8 * j + 2 * k;
-                const float c0 = i0 < ncols ? dv[i0] : 0.0f, c1 = i0 + 1 < ncols ? dv[i0 + 1] : 0.0f;
-                const __nv_bfloat162 h = __floats2bfloat162_rn(c0, c1);
-                const float2 hf = __bfloat1622float2(h);
-                hi[k] = *reinterpret_cast<const uint32_t *>(&h);
-                lo[k] = pack_bf16(c0 - hf.x, c1 - hf.y);
-            }
-            *reinterpret_cast<uint4 *>(smem + kTfD + canon_off(tid, 8 * j, kTcRows)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-            *reinterpret_cast<uint4 *>(smem + kTfD + canon_off(tid, 64 + 8 * j, kTcRows)) =
-                make_uint4(lo[0], lo[1], lo[2], lo[3]);
-        }
-    };
+    const uint32_t woff[kLayers] = {kTcW0, kTcW1, kTcW1 + 8192, kTcW1 + 16384, kTcW4};
 
-    for (uint32_t tile = blockIdx.x; ok && (uint64_t)tile * kTcRows < n; tile += gridDim.x) {
-        const uint32_t r = tile * kTcRows + tid;
+    for (uint32_t tile = blockIdx.x; (uint64_t)tile * kTcRows < n; tile += gridDim.x) {
+        const uint32_t r = tile * kTcRows + row;
         const bool live = r < n;
         float p[3], d[3];
         uint32_t slot;
         load_row(pos, dir, nullptr, n, r, gp, p, d, slot);
+        // input row: chunks part, part + 4, part + 8 of 8 encoded columns
+        uint32_t in[3][4];
 #pragma unroll
-        for (int j = 0; j < kIn / 8; ++j) {
-            uint32_t q[4];
+        for (int j = 0; j < 3; ++j)
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                float v0, v1;
-                encode_pair(p, d, 8 * j + 2 * k, v0, v1);
-                q[k] = pack_bf16(v0, v1);
+                const int c = 8 * (part + 4 * j) + 2 * k, axis = c / 24;
+                float v0 = 0.0f, v1 = 0.0f;
+                if (c < 72) {
+                    const float x = axis == 0 ? p[0] : axis == 1 ? p[1] : p[2];
+                    sincospif(x * __int_as_float((127 + ((c % 24) >> 1)) << 23), &v0, &v1);
+                } else if (c == 72) {
+                    v0 = d[0], v1 = d[1];
+                } else if (c == 74) {
+                    v0 = d[2];
+                }
+                in[j][k] = pack_bf16(v0, v1);
             }
-            *reinterpret_cast<uint4 *>(smem + kTfX0 + canon_off(tid, 8 * j, kTcRows)) = make_uint4(q[0], q[1], q[2], q[3]);
+        // the previous tile's last weight gradient reads x_0 and a delta tile
+        if (!first) finish();
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+            if (part + 4 * j < kIn / 8)
+                *reinterpret_cast<uint4 *>(smem + kTfX0 + canon_off(row, 8 * (part + 4 * j), kTcRows)) =
+                    make_uint4(in[j][0], in[j][1], in[j][2], in[j][3]);
+        uint64_t mask = 0;  // 16 bits per hidden layer: this thread's columns whose ReLU passes
+#pragma unroll
+        for (int l = 0; l < kLayers - 1; ++l) {
+            launch([&] {
+                const uint32_t idesc = idesc_bf16(kTcRows, kHid);
+                uint64_t a = smem_desc(smem_u32(smem) + xoff[l], kTcRows * 16, 128), b = smem_desc(w_img + woff[l], kHid * 16, 128);
+#pragma unroll
+                for (int s2 = 0; s2 < fan_in(l) / 16; ++s2, a += kTcRows * 2, b += kHid * 2) tc_mma(taddr, a, b, idesc, s2 > 0);
+                commit();
+            });
+            finish();
+            float v[16];
+            tmem_ld16(lane_addr + 16 * part, v);
+            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+            const float4 *b = reinterpret_cast<const float4 *>(bias + l * kHid + 16 * part);
+            uint32_t q[8], m = 0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float4 c = b[i];
+                q[2 * i] = relu_bf16(v[4 * i] + c.x, v[4 * i + 1] + c.y);
+                q[2 * i + 1] = relu_bf16(v[4 * i + 2] + c.z, v[4 * i + 3] + c.w);
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                if (q[i] & 0x7fffu) m |= 1u << (2 * i);
+                if (q[i] & 0x7fff0000u) m |= 2u << (2 * i);
+            }
+            mask |= (uint64_t)m << (16 * l);
+            *reinterpret_cast<uint4 *>(smem + xoff[l + 1] + canon_off(row, 16 * part, kTcRows)) = make_uint4(q[0], q[1], q[2], q[3]);
+            *reinterpret_cast<uint4 *>(smem + xoff[l + 1] + canon_off(row, 16 * part + 8, kTcRows)) =
+                make_uint4(q[4], q[5], q[6], q[7]);
         }
-        uint64_t mask[4] = {0, 0, 0, 0};
-        float v[64];
-        for (int l = 0; l < kLayers && ok; ++l) {
-            const int K = fan_in(l), N = fan_out(l);
-            ok = run([&] { tc_mma_chain(taddr, x_base[l], w_base[l], kTcRows, N, K, false); });
-            if (!ok) break;
-            read_acc(v, 0, N);
-            const float *b = bias + l * kHid;
-            if (l < kLayers - 1) {
+        launch([&] {
+            const uint32_t idesc = idesc_bf16(kTcRows, kOut);
+            uint64_t a = smem_desc(smem_u32(smem) + xoff[4], kTcRows * 16, 128), b = smem_desc(w_img + woff[4], kOut * 16, 128);
 #pragma unroll
-                for (int j = 0; j < kHid / 8; ++j) {
-                    uint32_t q[4];
+            for (int s2 = 0; s2 < kHid / 16; ++s2, a += kTcRows * 2, b += kOut * 2) tc_mma(taddr, a, b, idesc, s2 > 0);
+            commit();
+        });
+        const float c = live && wmean > 0.0f ? weight[r] / wmean : 0.0f;
+        float wx = 0.0f, wy = 0.0f, wz = 1.0f;
+        if (live) wx = sdir[3 * (size_t)r], wy = sdir[3 * (size_t)r + 1], wz = sdir[3 * (size_t)r + 2];
+        finish();
+        {
+            // loss and its gradient: lobes 2 part and 2 part + 1 of the row
+            float v[16], y[10];
+            tmem_ld16(lane_addr + 10 * part, v);
+            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const float h0 = fmaxf(v[8 * j + 2 * k] + b[8 * j + 2 * k], 0.0f);
-                        const float h1 = fmaxf(v[8 * j + 2 * k + 1] + b[8 * j + 2 * k + 1], 0.0f);
-                        q[k] = pack_bf16(h0, h1);
-                        if (q[k] & 0x7fffu) mask[l] |= 1ull << (8 * j + 2 * k);
-                        if (q[k] & 0x7fff0000u) mask[l] |= 1ull << (8 * j + 2 * k + 1);
-                    }
-                    *reinterpret_cast<uint4 *>(smem + xoff[l + 1] + canon_off(tid, 8 * j, kTcRows)) =
-                        make_uint4(q[0], q[1], q[2], q[3]);
-                }
-            } else {
-                float y[kOut], dy[kOut];
+            for (int i = 0; i < 10; ++i) y[i] = v[i] + bias[4 * kHid + 10 * part + i];
+            GuideLobeTerm t[2];
 #pragma unroll
-                for (int i = 0; i < kOut; ++i) {
-                    y[i] = v[i] + b[i];
-                    dy[i] = 0.0f;
-                }
-                float lterm = 0.0f;
-                if (live) {
-                    const float c = wmean > 0.0f ? weight[r] / wmean : 0.0f;
-                    const float lq = guide_loss_grad(y, sdir[3 * (size_t)r], sdir[3 * (size_t)r + 1],
-                                                     sdir[3 * (size_t)r + 2], c / (float)n, dy);
-                    lterm = -c * lq / (float)n;
-                }
-                for (int o = 16; o > 0; o >>= 1) lterm += __shfl_down_sync(0xffffffffu, lterm, o);
-                if (lane == 0) atomicAdd(loss, lterm);
-                put_delta(dy, kOut);
+            for (int j = 0; j < 2; ++j) t[j] = guide_lobe_term(y + 5 * j, wx, wy, wz);
+            const float ml = fmaxf(y[0], y[5]), mu = fmaxf(t[0].u, t[1].u);
+            float4 *lse = reinterpret_cast<float4 *>(smem + kTfLse);
+            lse[part * kTcRows + row] = make_float4(ml, guide_exp(y[0] - ml) + guide_exp(y[5] - ml), mu,
+                                                    guide_exp(t[0].u - mu) + guide_exp(t[1].u - mu));
+            __syncthreads();
+            float4 e[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) e[k] = lse[k * kTcRows + row];
+            const float Ml = fmaxf(fmaxf(e[0].x, e[1].x), fmaxf(e[2].x, e[3].x));
+            const float Mu = fmaxf(fmaxf(e[0].z, e[1].z), fmaxf(e[2].z, e[3].z));
+            float Sl = 0.0f, Su = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                Sl += e[k].y * guide_exp(e[k].x - Ml);
+                Su += e[k].w * guide_exp(e[k].z - Mu);
+            }
+            const float inv_l = 1.0f / Sl, inv_u = 1.0f / Su, scale = live ? c / (float)n : 0.0f;
+            if (part == 0 && live) loss_sum -= scale * ((Mu + logf(Su)) - (Ml + logf(Sl)));
+            float dy[10];
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+                guide_lobe_grad(y + 5 * j, t[j], guide_exp(y[5 * j] - Ml) * inv_l, guide_exp(t[j].u - Mu) * inv_u, wx, wy, wz,
+                                scale, dy + 5 * j);
+#pragma unroll
+            for (int i = 0; i < 5; ++i) {
+                uint32_t hi, lo;
+                split_bf16(live ? dy[2 * i] : 0.0f, live ? dy[2 * i + 1] : 0.0f, hi, lo);
+                *reinterpret_cast<uint32_t *>(smem + kTfD + canon_off(row, 10 * part + 2 * i, kTcRows)) = hi;
+                *reinterpret_cast<uint32_t *>(smem + kTfD + canon_off(row, 64 + 10 * part + 2 * i, kTcRows)) = lo;
+            }
+            if (part < 3) {  // unused outputs
+                *reinterpret_cast<uint4 *>(smem + kTfD + canon_off(row, kGuideOut + 8 * part, kTcRows)) = make_uint4(0, 0, 0, 0);
+                *reinterpret_cast<uint4 *>(smem + kTfD + canon_off(row, 64 + kGuideOut + 8 * part, kTcRows)) =
+                    make_uint4(0, 0, 0, 0);
             }
         }
         // backward: delta_{l-1} = (delta_l W_l) masked by the ReLU of layer
-        // l-1, together with dW_l
-        for (int l = kLayers - 1; l >= 1 && ok; --l) {
-            const int K = fan_out(l);
+        // l - 1; dW_l runs behind it
+#pragma unroll
+        for (int l = kLayers - 1; l >= 1; --l) {
             const bool acc = !first;
-            ok = run([&] {
-                tc_mma_chain(taddr, d_base, wt_base[l], kTcRows, kHid, K, false);
-                tc_mma_chain(taddr, dlo_base, wt_base[l], kTcRows, kHid, K, true);
+            launch([&] {
+                const uint32_t idesc = idesc_bf16(kTcRows, kHid) | (1u << 16);
+                const uint32_t O = l == kLayers - 1 ? kOut : kHid;
+                const uint64_t b0 = smem_desc(w_img + woff[l], 128, O * 16);
+#pragma unroll
+                for (int part2 = 0; part2 < 2; ++part2) {  // high parts, then remainders
+                    uint64_t a = smem_desc(d_base + (uint32_t)(l & 1) * 32768 + part2 * 8 * 2048, kTcRows * 16, 128), b = b0;
+#pragma unroll
+                    for (uint32_t s2 = 0; s2 < O / 16; ++s2, a += kTcRows * 2, b += 16) tc_mma(taddr, a, b, idesc, part2 + s2 > 0);
+                }
+                commit();
                 wgrad(l, acc);
             });
-            if (!ok) break;
-            read_acc(v, 0, kHid);
-            const uint64_t m = mask[l - 1];
-#pragma unroll
-            for (int i = 0; i < kHid; ++i)
-                if (!((m >> i) & 1ull)) v[i] = 0.0f;
-            put_delta(v, kHid);
-        }
-        if (ok) ok = run([&] { wgrad(0, !first); });
-        first = false;
-        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-        __syncthreads();
-    }
-    // add the CTA's weight gradients: rows m < 64 of dW_l carry the high part
-    // of output m, rows 64 + m the low part
-    if (ok && !first) {
-        float *lo = reinterpret_cast<float *>(smem + kTfD);  // [64 rows][96]
-        for (int l = 0; l < kLayers; ++l) {
-            const int in = fan_in(l), N = in + 16, O = fan_out(l);
-            float row[96];
-#pragma unroll
-            for (int c = 0; c < 6; ++c) {
-                if (16 * c >= N) break;
-                float t[16];
-                tmem_ld16(lane_addr + tf_dcol(l) + 16 * c, t);
-#pragma unroll
-                for (int i = 0; i < 16; ++i) row[16 * c + i] = t[i];
-            }
+            finish();
+            float v[16];
+            tmem_ld16(lane_addr + 16 * part, v);
             asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-            __syncthreads();
-            if (tid >= 64)
-                for (int i = 0; i <= in; ++i) lo[(tid - 64) * 96 + i] = row[i];
-            __syncthreads();
-            if (tid < O) {
-                float *G = grad + w_off(l) + (size_t)tid * in;
-                for (int i = 0; i < in; ++i) atomicAdd(G + i, row[i] + lo[tid * 96 + i]);
-                atomicAdd(grad + b_off(l) + tid, row[in] + lo[tid * 96 + in]);
+            const uint32_t m = (uint32_t)(mask >> (16 * (l - 1)));
+            unsigned char *D = smem + kTfD + ((l - 1) & 1) * 32768;
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                uint32_t hi[4], lo[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int i = 8 * j + 2 * k;
+                    split_bf16((m >> i) & 1u ? v[i] : 0.0f, (m >> (i + 1)) & 1u ? v[i + 1] : 0.0f, hi[k], lo[k]);
+                }
+                *reinterpret_cast<uint4 *>(D + canon_off(row, 16 * part + 8 * j, kTcRows)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                *reinterpret_cast<uint4 *>(D + canon_off(row, 64 + 16 * part + 8 * j, kTcRows)) =
+                    make_uint4(lo[0], lo[1], lo[2], lo[3]);
             }
         }
+        launch([&] {
+            wgrad(0, !first);
+            commit();
+        });
+        first = false;
     }
-    if (!ok) {
-        // MMAs or the weight copy still in flight: wait again (bounded) before freeing their memory
+    finish();
+    if (!__syncthreads_or(s_failed)) {
+        // The CTA's sums: rows m < 64 of dW_l carry the high part of output m, rows
+        // 64 + m the low part. They meet in shared memory, chunks of 16 columns
+        // as [chunk][output][16], and leave as whole rows.
+        float *stage = reinterpret_cast<float *>(smem);
+        const int o = row & 63;
+#pragma unroll
+        for (int pass = 0; pass < 2; ++pass) {
+            if ((row >= 64) == (pass == 0))
+#pragma unroll 1
+                for (int l = 0; l < kLayers; ++l)
+#pragma unroll 1
+                    for (int ch = part; ch < tf_chunks(l); ch += 4) {
+                        float v[16];
+                        tmem_ld16(lane_addr + tf_dcol(l) + 16 * ch, v);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+                        float4 *q = reinterpret_cast<float4 *>(stage + ((tf_chunk0(l) + ch) * 64 + o) * kTfStage);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            float4 s = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                            if (pass == 1) {
+                                const float4 low = q[i];
+                                s.x += low.x, s.y += low.y, s.z += low.z, s.w += low.w;
+                            }
+                            q[i] = s;
+                        }
+                    }
+            __syncthreads();
+        }
+        float *out = parts + (size_t)blockIdx.x * kPartStride;
+#pragma unroll
+        for (int l = 0; l < kLayers; ++l) {
+            const int rowv = fan_in(l) / 4;
+            for (int i = tid; i < fan_out(l) * rowv; i += kTfThreads) {
+                const int m = i / rowv, col = 4 * (i % rowv);
+                reinterpret_cast<float4 *>(out + w_off(l))[i] =
+                    *reinterpret_cast<const float4 *>(stage + ((tf_chunk0(l) + col / 16) * 64 + m) * kTfStage + col % 16);
+            }
+            if (tid < fan_out(l)) out[b_off(l) + tid] = stage[((tf_chunk0(l) + fan_in(l) / 16) * 64 + tid) * kTfStage];
+        }
+        for (int k = 16; k > 0; k >>= 1) loss_sum += __shfl_down_sync(0xffffffffu, loss_sum, k);
+        if (part == 0 && lane == 0) s_loss[warp] = loss_sum;
+        __syncthreads();
+        if (tid == 0) out[kNumParams] = (s_loss[0] + s_loss[1]) + (s_loss[2] + s_loss[3]);
+    } else {
+        // MMAs or the weight copy still in flight: wait again (bounded) before
+        // freeing their memory; the sums of this CTA count as nothing
         mbar_wait(mbar, phase);
         mbar_wait(cbar, 0);
+        for (int i = tid; i < kPartStride; i += kTfThreads) parts[(size_t)blockIdx.x * kPartStride + i] = 0.0f;
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
@@ -1112,31 +1188,74 @@ __global__ void __launch_bounds__(128) k_guide_wgrad(TrainBuffers tb, uint32_t n
     }
 }
 
-// Sum of the sample weights into *sum (zeroed before).
-__global__ void k_guide_weight_sum(const float *w, uint32_t n, float *sum)
+// Sums of the sample weights, one per block (gridDim.x <= kWeightParts).
+__global__ void __launch_bounds__(256) k_guide_weight_sum(const float *w, uint32_t n, float *sums)
 {
+    __shared__ float s[8];
     float v = 0.0f;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) v += w[i];
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(sum, v);
+    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x < 8) {
+        v = s[threadIdx.x];
+        for (int o = 4; o > 0; o >>= 1) v += __shfl_down_sync(0xffu, v, o);
+        if (threadIdx.x == 0) sums[blockIdx.x] = v;
+    }
 }
 
-__global__ void k_guide_adam(float *params, float *m, float *v, const float *grad, int t, float lr, float b1, float b2,
-                             float eps, __nv_bfloat16 *wb, unsigned char *img)
+// The blocks' weight sums as one (mma.sync path).
+__global__ void k_guide_add_sums(const float *sums, uint32_t count, float *sum)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= kNumParams) return;
-    const float g = grad[i];
-    const float mi = b1 * m[i] + (1.0f - b1) * g;
-    const float vi = b2 * v[i] + (1.0f - b2) * g * g;
-    m[i] = mi;
-    v[i] = vi;
-    const float c1 = 1.0f - powf(b1, (float)t), c2 = 1.0f - powf(b2, (float)t);
-    const float p = params[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    params[i] = p;
+    const int lane = threadIdx.x;
+    float v = (uint32_t)lane < count ? sums[lane] : 0.0f;
+    if ((uint32_t)lane + 32 < count) v += sums[lane + 32];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if (lane == 0) *sum = v;
+}
+
+// Adds the nparts rows of partial sums (in a fixed order: kAdamSplits
+// interleaved sums, then those) into grad and the loss and, with `adam`, takes
+// the Adam step. 64 entries per block.
+constexpr int kAdamSplits = 8;
+struct AdamArgs {
+    float *params, *m, *v;
+    __nv_bfloat16 *wb;
+    unsigned char *img;
+    int t;
+    float lr, b1, b2, eps;
+};
+__global__ void __launch_bounds__(64 * kAdamSplits) k_guide_adam(const float *parts, int nparts, float *grad, float *loss, bool adam, AdamArgs a)
+{
+    __shared__ float s[kAdamSplits][64];
+    const int i = blockIdx.x * 64 + (threadIdx.x & 63), split = threadIdx.x >> 6;
+    float sum = 0.0f;
+    if (i <= kNumParams) {
+#pragma unroll 8
+        for (int q = split; q < nparts; q += kAdamSplits) sum += parts[(size_t)q * kPartStride + i];
+    }
+    s[split][threadIdx.x & 63] = sum;
+    __syncthreads();
+    if (split != 0 || i > kNumParams) return;
+    float g = 0.0f;
+#pragma unroll
+    for (int q = 0; q < kAdamSplits; ++q) g += s[q][threadIdx.x];
+    if (i == kNumParams) {
+        if (loss) *loss = g;
+        return;
+    }
+    if (grad) grad[i] = g;
+    if (!adam) return;
+    const float mi = a.b1 * a.m[i] + (1.0f - a.b1) * g;
+    const float vi = a.b2 * a.v[i] + (1.0f - a.b2) * g * g;
+    a.m[i] = mi;
+    a.v[i] = vi;
+    const float c1 = 1.0f - powf(a.b1, (float)a.t), c2 = 1.0f - powf(a.b2, (float)a.t);
+    const float p = a.params[i] - a.lr * (mi / c1) / (sqrtf(vi / c2) + a.eps);
+    a.params[i] = p;
     // BF16 weight copy and weight image (biases stay FP32)
     for (int l = 0; l < kLayers; ++l)
-        if (i >= w_off(l) && i < b_off(l)) store_weight(wb, img, l, i - w_off(l), p);
+        if (i >= w_off(l) && i < b_off(l)) store_weight(a.wb, a.img, l, i - w_off(l), p);
 }
 
 __global__ void k_guide_export(const float *params, __nv_bfloat16 *wb, unsigned char *img)
@@ -1182,6 +1301,7 @@ __global__ void k_guide_pdf(const float *y, const float *dir, uint32_t n, uint32
     pdf[i] = guide_pdf(L, dir[3 * (size_t)i], dir[3 * (size_t)i + 1], dir[3 * (size_t)i + 2]);
 }
 
+constexpr size_t kScalarBytes = (4 + kWeightParts) * sizeof(float);
 constexpr size_t kInferSmem = sizeof(SmemWeights);
 constexpr size_t kTrainSmem = sizeof(SmemWeights) + sizeof(SmemWeightsT) + 4 * 16 * kOut * sizeof(float);
 
@@ -1191,10 +1311,12 @@ constexpr size_t kTrainSmem = sizeof(SmemWeights) + sizeof(SmemWeightsT) + 4 * 1
 struct dr_guide {
     dr_context *ctx = nullptr;
     dr_guide_config cfg{};
+    unsigned char *mem = nullptr;  // one allocation; the pointers below point into it
     float *params = nullptr, *m = nullptr, *v = nullptr, *grad = nullptr;
     __nv_bfloat16 *wb = nullptr;
     unsigned char *img = nullptr;  // weight image of the tcgen05 kernels (kImgBytes)
-    float *scalars = nullptr;  // [0] sum of the batch's sample weights, [1] loss
+    float *scalars = nullptr;  // [0] sum of the batch's sample weights (mma.sync path), [1] loss, [4..] weight sums per block
+    float *parts = nullptr;    // partial gradients and loss of the tcgen05 training kernel, one row per CTA
     dr::TrainBuffers tb{};
     void *tb_mem = nullptr;
     uint32_t capacity = 0;
@@ -1216,13 +1338,7 @@ GuideParams guide_params(const dr_guide *g)
 void free_guide(dr_guide *g)
 {
     if (!g) return;
-    cudaFree(g->params);
-    cudaFree(g->m);
-    cudaFree(g->v);
-    cudaFree(g->grad);
-    cudaFree(g->wb);
-    cudaFree(g->img);
-    cudaFree(g->scalars);
+    cudaFree(g->mem);
     cudaFree(g->tb_mem);
     delete g;
 }
@@ -1250,37 +1366,43 @@ dr_status ensure_train_capacity(dr_guide *g, uint32_t n)
     return DR_OK;
 }
 
-// loss and gradients (grad buffer) of one batch
+// Loss and gradients of one batch, as *nparts rows of partial sums at *parts.
 dr_status run_gradients(dr_guide *g, const float *pos, const float *dir, const float *sdir, const float *weight,
-                        uint32_t n, cudaStream_t st)
+                        uint32_t n, cudaStream_t st, const float **parts, int *nparts)
 {
-    // the per-layer delta and activation buffers serve the mma.sync path only
-    // (the tcgen05 kernel keeps them on chip)
-    if (g->cfg.infer_kernel == DR_GUIDE_INFER_MMA_SYNC) {
-        const dr_status r = ensure_train_capacity(g, n);
-        if (r != DR_OK) return r;
-    }
-    DR_CUDA(cudaMemsetAsync(g->grad, 0, kNumParams * sizeof(float), st));
-    DR_CUDA(cudaMemsetAsync(g->scalars, 0, 2 * sizeof(float), st));
-    k_guide_weight_sum<<<std::min<unsigned>((n + 255) / 256, 64), 256, 0, st>>>(weight, n, g->scalars);
     const GuideParams gp = guide_params(g);
+    const unsigned sum_blocks = std::min<unsigned>((n + 255) / 256, kWeightParts);
+    float *sums = g->scalars + 4;
+    k_guide_weight_sum<<<sum_blocks, 256, 0, st>>>(weight, n, sums);
     if (g->cfg.infer_kernel == DR_GUIDE_INFER_TCGEN05) {
         // one CTA per SM (its shared memory and 512 tensor-memory columns)
         const unsigned tiles = (n + kTcRows - 1) / kTcRows;
         const unsigned blocks = std::min<unsigned>(tiles, (unsigned)g->ctx->num_sms);
-        k_guide_train_fused<<<blocks, 128, kTfSmem, st>>>(g->img, g->params, gp, pos, dir, sdir, weight, n,
-                                                           g->scalars, g->grad, g->scalars + 1, g->ctx->d_error);
+        k_guide_train_fused<<<blocks, kTfThreads, kTfSmem, st>>>(g->img, g->params, gp, pos, dir, sdir, weight, n, sums,
+                                                                 sum_blocks, g->parts, g->ctx->d_error);
+        *parts = g->parts;
+        *nparts = (int)blocks;
     } else {
+        // the per-layer delta and activation buffers serve the mma.sync path only
+        // (the tcgen05 kernel keeps them on chip); its sums meet in one row
+        const dr_status r = ensure_train_capacity(g, n);
+        if (r != DR_OK) return r;
+        DR_CUDA(cudaMemsetAsync(g->parts, 0, kPartStride * sizeof(float), st));
+        k_guide_add_sums<<<1, 32, 0, st>>>(sums, sum_blocks, g->scalars);
         k_guide_train_fb<<<(n + 63) / 64, 128, kTrainSmem, st>>>(g->wb, g->params, gp, pos, dir, sdir, weight, n,
-                                                                 g->scalars, g->tb, g->scalars + 1);
+                                                                 g->scalars, g->tb, g->parts + kNumParams);
         int bx = 0;
         for (int l = 0; l < kLayers; ++l) bx = std::max(bx, wgrad_blocks_x(l));
         const dim3 grid((unsigned)bx, (n + kWgradRows - 1) / kWgradRows, (unsigned)kLayers);
-        k_guide_wgrad<<<grid, 128, 0, st>>>(g->tb, n, g->grad);
+        k_guide_wgrad<<<grid, 128, 0, st>>>(g->tb, n, g->parts);
+        *parts = g->parts;
+        *nparts = 1;
     }
     DR_CUDA(cudaGetLastError());
     return DR_OK;
 }
+
+constexpr unsigned kAdamBlocks = (kNumParams + 1 + 63) / 64;
 
 }  // namespace
 
@@ -1361,15 +1483,30 @@ dr_status dr_guide_create(dr_context *ctx, const dr_guide_config *cfg, dr_guide 
         free_guide(g);
         return fail(DR_ERR_INVALID_ARGUMENT, "dr_guide_create: unknown inference kernel");
     }
-    cudaError_t e;
-    if ((e = dev_malloc(&g->params, kNumParams * 4)) != cudaSuccess || (e = dev_malloc(&g->m, kNumParams * 4)) != cudaSuccess ||
-        (e = dev_malloc(&g->v, kNumParams * 4)) != cudaSuccess || (e = dev_malloc(&g->grad, kNumParams * 4)) != cudaSuccess ||
-        (e = dev_malloc(&g->wb, kNumWeights * 2)) != cudaSuccess || (e = dev_malloc(&g->img, kImgBytes)) != cudaSuccess || (e = dev_malloc(&g->scalars, 16)) != cudaSuccess ||
-        (e = cudaMemset(g->m, 0, kNumParams * 4)) != cudaSuccess || (e = cudaMemset(g->v, 0, kNumParams * 4)) != cudaSuccess ||
-        (e = cudaMemset(g->scalars, 0, 16)) != cudaSuccess) {
+    // one allocation, its parts on 256-byte boundaries
+    size_t bytes = 0;
+    auto place = [&](size_t b) {
+        const size_t at = bytes;
+        bytes += (b + 255) & ~size_t(255);
+        return at;
+    };
+    const size_t at_params = place(kNumParams * 4), at_m = place(kNumParams * 4), at_v = place(kNumParams * 4),
+                 at_grad = place(kNumParams * 4), at_wb = place(kNumWeights * 2), at_img = place(kImgBytes),
+                 at_scalars = place(kScalarBytes), at_parts = place((size_t)ctx->num_sms * kPartStride * 4);
+    cudaError_t e = dev_malloc(&g->mem, bytes);
+    if (e == cudaSuccess) e = cudaMemset(g->mem + at_scalars, 0, kScalarBytes);
+    if (e != cudaSuccess) {
         free_guide(g);
         return cuda_fail(e, "dr_guide_create");
     }
+    g->params = reinterpret_cast<float *>(g->mem + at_params);
+    g->m = reinterpret_cast<float *>(g->mem + at_m);
+    g->v = reinterpret_cast<float *>(g->mem + at_v);
+    g->grad = reinterpret_cast<float *>(g->mem + at_grad);
+    g->wb = reinterpret_cast<__nv_bfloat16 *>(g->mem + at_wb);
+    g->img = g->mem + at_img;
+    g->scalars = reinterpret_cast<float *>(g->mem + at_scalars);
+    g->parts = reinterpret_cast<float *>(g->mem + at_parts);
     // He-uniform initialisation (ReLU), last layer scaled by 0.1, zero biases
     std::mt19937_64 rng(g->cfg.seed);
     std::vector<float> p(kNumParams, 0.0f);
@@ -1489,8 +1626,12 @@ dr_status dr_guide_gradients(dr_guide *g, const float *pos_dev, const float *dir
 {
     DR_CHECK_ARG(g && n > 0 && pos_dev && dir_dev && sdir_dev && weight_dev, "dr_guide_gradients: bad argument");
     DR_CUDA(cudaSetDevice(g->ctx->device));
-    dr_status r = run_gradients(g, pos_dev, dir_dev, sdir_dev, weight_dev, n, nullptr);
+    const float *parts = nullptr;
+    int nparts = 0;
+    dr_status r = run_gradients(g, pos_dev, dir_dev, sdir_dev, weight_dev, n, nullptr, &parts, &nparts);
     if (r != DR_OK) return r;
+    k_guide_adam<<<kAdamBlocks, 64 * kAdamSplits>>>(parts, nparts, g->grad, g->scalars + 1, false, AdamArgs{});
+    DR_CUDA(cudaGetLastError());
     DR_CUDA(cudaDeviceSynchronize());
     if (loss_host) DR_CUDA(cudaMemcpy(loss_host, g->scalars + 1, 4, cudaMemcpyDeviceToHost));
     if (grad_host) DR_CUDA(cudaMemcpy(grad_host, g->grad, kNumParams * 4, cudaMemcpyDeviceToHost));
@@ -1504,14 +1645,17 @@ dr_status dr_guide_train_step(dr_guide *g, const float *pos_dev, const float *di
     if (n == 0) return DR_OK;
     DR_CUDA(cudaSetDevice(g->ctx->device));
     auto st = static_cast<cudaStream_t>(stream);
-    dr_status r = run_gradients(g, pos_dev, dir_dev, sdir_dev, weight_dev, n, st);
+    const float *parts = nullptr;
+    int nparts = 0;
+    dr_status r = run_gradients(g, pos_dev, dir_dev, sdir_dev, weight_dev, n, st, &parts, &nparts);
     if (r != DR_OK) return r;
     ++g->step;
     const float lr = g->cfg.warmup_steps && (uint32_t)g->step < g->cfg.warmup_steps
                          ? g->cfg.learning_rate * (float)g->step / (float)g->cfg.warmup_steps
                          : g->cfg.learning_rate;
-    k_guide_adam<<<(kNumParams + 255) / 256, 256, 0, st>>>(g->params, g->m, g->v, g->grad, g->step, lr,
-                                                           g->cfg.beta1, g->cfg.beta2, g->cfg.epsilon, g->wb, g->img);
+    k_guide_adam<<<kAdamBlocks, 64 * kAdamSplits, 0, st>>>(parts, nparts, nullptr, g->scalars + 1, true,
+                                              AdamArgs{g->params, g->m, g->v, g->wb, g->img, g->step, lr, g->cfg.beta1,
+                                                       g->cfg.beta2, g->cfg.epsilon});
     DR_CUDA(cudaGetLastError());
     return DR_OK;
 }

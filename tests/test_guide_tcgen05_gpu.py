@@ -95,3 +95,36 @@ def test_tcgen05_rows_do_not_depend_on_the_launch(native, ctx):
     err = (want - run(ms, big)).abs()
     scale = float(want.abs().max()) + 1e-6
     assert float(err.median()) <= 1e-6 * scale + 1e-7 and float(err.max()) <= 2e-2 * scale
+
+
+@pytest.mark.parametrize("n", [1, 127, 129, 19456, 19457])
+def test_tcgen05_training_at_tile_edges(native, ctx, n):
+    """Row counts around one tile and around one tile per SM: the gradients
+    agree with the mma.sync kernels (the bounds of the test above), and two runs
+    have the same bits."""
+    rng = np.random.default_rng(n + 7)
+    tc = native.Guide(ctx, seed=8, half_extent=10.0, infer_kernel=0)
+    ms = native.Guide(ctx, seed=8, half_extent=10.0, infer_kernel=1)
+    p = tc.params()
+    p[-48:] = rng.normal(0, 0.3, 48)
+    tc.set_params(p)
+    ms.set_params(p)
+
+    def unit(k):
+        d = rng.normal(size=(k, 3))
+        return torch.from_numpy((d / np.linalg.norm(d, axis=1, keepdims=True)).astype(np.float32)).cuda()
+
+    pos = torch.from_numpy(rng.uniform(-10, 10, (n, 3)).astype(np.float32)).cuda()
+    nrm, sdir = unit(n), unit(n)
+    w = torch.from_numpy(rng.lognormal(0.0, 1.0, n).astype(np.float32)).cuda()
+    l_tc, g_tc = tc.gradients(pos, nrm, sdir, w, n)
+    l_2, g_2 = tc.gradients(pos, nrm, sdir, w, n)
+    l_ms, g_ms = ms.gradients(pos, nrm, sdir, w, n)
+    ctx.check()
+    assert l_tc == l_2 and np.array_equal(g_tc, g_2)
+    assert abs(l_tc - l_ms) <= 1e-4 * abs(l_ms)
+    a, b = g_tc.astype(np.float64), g_ms.astype(np.float64)
+    assert np.linalg.norm(a - b) <= 1e-2 * np.linalg.norm(b)
+    # the step uses the same sums: one Adam step from the same parameters agrees
+    tc.train_step(pos, nrm, sdir, w, n)
+    assert tc.last_loss() == l_tc
