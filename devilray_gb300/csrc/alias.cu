@@ -19,9 +19,13 @@
 #include "dr_internal.h"
 #include "alias_kernels.cuh"
 
+#include <cooperative_groups.h>
+
 #include <climits>
 
 namespace dr {
+
+namespace cg = cooperative_groups;
 
 using i128 = __int128;
 
@@ -286,12 +290,36 @@ struct SweepScalars {
     int32_t num_lights;
     int32_t num_heavies;
     i128 D_total;
+    double Wd, inv_W, nd;  // (double)W, 1 / Wd, (double)n
 };
+
+// floor(w 2^shift) of a clamped weight w = m 2^(e - 24), m its
+// 24-bit significand (a denormal one has fewer bits; the value is the same).
+__device__ __forceinline__ long long fixed_weight_bits(float w, int shift)
+{
+    const uint32_t bits = __float_as_uint(w);
+    const int be = (int)(bits >> 23);
+    const long long m = be ? (long long)((bits & 0x7fffffu) | 0x800000u) : (long long)(bits & 0x7fffffu);
+    const int s = (be ? be : 1) - 150 + shift;
+    return s >= 0 ? m << s : s > -64 ? m >> -s : 0;
+}
+
+// The same as a double, by its bits: an FP32 significand always fits, and the
+// conversion from an integer would run at the FP64 rate.
+__device__ __forceinline__ double fixed_weight_double(float w, int shift)
+{
+    const uint32_t bits = __float_as_uint(w), be = bits >> 23;
+    if (be == 0) return (double)fixed_weight_bits(w, shift);
+    const int s = (int)be - 150 + shift;  // shift of the 24-bit significand
+    if (s <= -24) return 0.0;
+    const uint32_t frac = (bits & 0x7fffffu) & (s < 0 ? ~0u << -s : ~0u);
+    return __hiloint2double((int)(((be - 127 + 1023 + (uint32_t)shift) << 20) | (frac >> 3)), (int)(frac << 29));
+}
 
 __device__ __forceinline__ long long fixed_weight(float w, const SweepScalars &sc)
 {
     if (sc.emax == INT_MIN) return 0;
-    return (long long)ldexp((double)clamp_weight(w), sc.shift);
+    return fixed_weight_bits(clamp_weight(w), sc.shift);
 }
 
 __global__ void k_sweep_init(SweepScalars *sc, uint32_t n)
@@ -378,6 +406,9 @@ __global__ void k_sweep_scan_tiles(Agg *tiles, uint32_t num_tiles, SweepScalars 
         sc->num_lights = carry.lights;
         sc->num_heavies = (int32_t)n - carry.lights;
         sc->D_total = carry.D;
+        sc->Wd = (double)sc->W;
+        sc->inv_W = 1.0 / sc->Wd;
+        sc->nd = (double)n;
         const float Wf = sc->emax == INT_MIN ? 0.0f : (float)ldexp((double)sc->W, -sc->shift);
         sc->uniform = !(Wf >= 1e-5f);
     }
@@ -418,41 +449,71 @@ __global__ void k_sweep_scatter(const float *__restrict__ w, uint32_t n, const S
 
 __device__ __forceinline__ float pdf_of(long long m, unsigned long long W) { return (float)((double)m / (double)W); }
 
-__global__ void k_sweep_assign(const float *__restrict__ w, uint32_t n, const SweepScalars *sc,
-                               const int32_t *__restrict__ lights, const i128 *__restrict__ Dexcl,
-                               const int32_t *__restrict__ heavies, const i128 *__restrict__ Sincl,
-                               dr_alias_entry *__restrict__ out)
+// (float)(x / Wd) for x >= 0, with inv = 1 / Wd: the product x inv is within two
+// units of the last place of the quotient, so both round to the same float
+// unless the product's 29 bits below a float's lie that close to half; there
+// (once in 2^26) the division decides. FP64 runs at 1/64 of the FP32 rate, and a
+// division is some ten operations. Below 2^-126, where a float has fewer bits, the
+// division decides as well.
+__device__ __forceinline__ float ratio_f(double x, double Wd, double inv)
 {
-    const SweepScalars s = *sc;
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    if (s.uniform) {
-        out[t] = dr_alias_entry{1.0f, 1.0f / (float)n, 0.0f, (int32_t)t, -1};
-        return;
+    const double q = x * inv;
+    const uint32_t low = (uint32_t)__double2loint(q) & 0x1fffffffu;
+    if (low - 0x0ffffffcu <= 8u || q < 0x1p-126) return (float)(x / Wd);
+    return (float)q;
+}
+
+// First index of the sorted list with list[i] > key (Greater) or >= key, as a
+// binary search that starts from every (count / 256)-th entry, staged in shared
+// memory.
+constexpr int kCoarse = 256;
+template <bool GREATER>
+__device__ __forceinline__ int32_t list_search(const i128 *__restrict__ list, int32_t count, const i128 *coarse, int32_t step, i128 key)
+{
+    // coarse[c] = list[min((c + 1) step, count) - 1]
+    int32_t lo = 0, hi = kCoarse;
+    while (lo < hi) {
+        const int32_t mid = (lo + hi) >> 1;
+        if (GREATER ? coarse[mid] > key : coarse[mid] >= key) hi = mid;
+        else lo = mid + 1;
     }
+    if (lo == kCoarse) return count;
+    hi = min((lo + 1) * step, count) - 1;  // satisfies the condition
+    lo = lo * step;
+    while (lo < hi) {
+        const int32_t mid = (lo + hi) >> 1;
+        if (GREATER ? list[mid] > key : list[mid] >= key) hi = mid;
+        else lo = mid + 1;
+    }
+    return lo;
+}
+
+// The entry of list item t (the lights in order, then the heavies); s_S and s_D
+// are the staged entries of list_search.
+__device__ __forceinline__ void sweep_assign_item(uint32_t t, const float *__restrict__ w, uint32_t n, const SweepScalars &s,
+                                                  const int32_t *lights, const i128 *Dexcl, const int32_t *heavies,
+                                                  const i128 *Sincl, const i128 *s_S, int32_t step_S, const i128 *s_D,
+                                                  int32_t step_D, dr_alias_entry *__restrict__ out)
+{
     const int32_t nl = s.num_lights, nh = s.num_heavies;
-    const double Wd = (double)s.W;
+    const double Wd = s.Wd, inv = s.inv_W;
+    auto fixed_d = [&](int32_t i) { return fixed_weight_double(clamp_weight(w[i]), s.shift); };
+    auto pdf = [&](int32_t i) { return ratio_f(fixed_d(i), Wd, inv); };
     dr_alias_entry e;
     int32_t slot;
     if ((int32_t)t < nl) {
         const int32_t k = (int32_t)t;
         const int32_t i = lights[k];
         slot = i;
-        const long long m = fixed_weight(w[i], s);
-        const i128 d = Dexcl[k];
+        const double m = fixed_d(i);
         // first heavy h with Sincl[h] > d
-        int32_t lo = 0, hi = nh;
-        while (lo < hi) {
-            const int32_t mid = (lo + hi) >> 1;
-            if (Sincl[mid] > d) hi = mid;
-            else lo = mid + 1;
-        }
+        const int32_t h = nh > 0 ? list_search<true>(Sincl, nh, s_S, step_S, Dexcl[k]) : 0;
         e.A = i;
-        e.p_A = (float)((double)((long long)n * m) / Wd);
-        e.pdf_A = pdf_of(m, s.W);
-        if (lo < nh) {
-            e.B = heavies[lo];
-            e.pdf_B = pdf_of(fixed_weight(w[e.B], s), s.W);
+        e.p_A = ratio_f(m * s.nd, Wd, inv);  // n m, rounded to a double once
+        e.pdf_A = ratio_f(m, Wd, inv);
+        if (h < nh) {
+            e.B = heavies[h];
+            e.pdf_B = pdf(e.B);
         } else {
             e.B = -1;
             e.pdf_B = 0.0f;
@@ -464,20 +525,15 @@ __global__ void k_sweep_assign(const float *__restrict__ w, uint32_t n, const Sw
         slot = i;
         const i128 sj = Sincl[j];
         // first light k with Dexcl[k] >= Sincl[j]
-        int32_t lo = 0, hi = nl;
-        while (lo < hi) {
-            const int32_t mid = (lo + hi) >> 1;
-            if (Dexcl[mid] >= sj) hi = mid;
-            else lo = mid + 1;
-        }
-        const i128 Dk = lo < nl ? Dexcl[lo] : s.D_total;
+        const int32_t k = nl > 0 ? list_search<false>(Dexcl, nl, s_D, step_D, sj) : 0;
+        const i128 Dk = k < nl ? Dexcl[k] : s.D_total;
         const long long R = (long long)(sj - Dk);
         e.A = i;
-        e.pdf_A = pdf_of(fixed_weight(w[i], s), s.W);
+        e.pdf_A = pdf(i);
         if (j + 1 < nh) {
-            e.p_A = (float)((double)((long long)s.W + R) / Wd);
+            e.p_A = ratio_f((double)((long long)s.W + R), Wd, inv);
             e.B = heavies[j + 1];
-            e.pdf_B = pdf_of(fixed_weight(w[e.B], s), s.W);
+            e.pdf_B = pdf(e.B);
         } else {
             e.p_A = 1.0f;
             e.B = -1;
@@ -490,6 +546,229 @@ __global__ void k_sweep_assign(const float *__restrict__ w, uint32_t n, const Sw
     }
     ensure_pa_larger(e);
     out[slot] = e;
+}
+
+__device__ __forceinline__ int32_t coarse_step(int32_t count) { return (count + kCoarse - 1) / kCoarse; }
+
+__global__ void __launch_bounds__(kCoarse) k_sweep_assign(const float *__restrict__ w, uint32_t n, const SweepScalars *sc,
+                                                          const int32_t *__restrict__ lights, const i128 *__restrict__ Dexcl,
+                                                          const int32_t *__restrict__ heavies, const i128 *__restrict__ Sincl,
+                                                          dr_alias_entry *__restrict__ out)
+{
+    const SweepScalars s = *sc;
+    const uint32_t t = blockIdx.x * kCoarse + threadIdx.x;
+    if (s.uniform) {
+        if (t < n) out[t] = dr_alias_entry{1.0f, 1.0f / (float)n, 0.0f, (int32_t)t, -1};
+        return;
+    }
+    const int32_t nl = s.num_lights, nh = s.num_heavies;
+    // blocks of lights search the heavies and blocks of heavies the lights; the
+    // one that holds both stages both
+    __shared__ i128 s_S[kCoarse], s_D[kCoarse];
+    const int32_t step_S = coarse_step(nh), step_D = coarse_step(nl), begin = (int32_t)(blockIdx.x * kCoarse);
+    if (begin < nl && nh > 0) s_S[threadIdx.x] = Sincl[min((int32_t)(threadIdx.x + 1) * step_S, nh) - 1];
+    if (begin + kCoarse > nl && nl > 0) s_D[threadIdx.x] = Dexcl[min((int32_t)(threadIdx.x + 1) * step_D, nl) - 1];
+    __syncthreads();
+    if (t < n) sweep_assign_item(t, w, n, s, lights, Dexcl, heavies, Sincl, s_S, step_S, s_D, step_D, out);
+}
+
+// ---- sweep build of one table by one cluster of blocks ---------------------------------
+
+// The first six steps of the parallel build (scalars, exponent, total, tile
+// sums, their scan, the lists) as one launch: every thread keeps up to kListItems
+// consecutive items in registers, and the blocks of one cluster meet through
+// distributed shared memory. The same integers in the same order as the separate
+// kernels, without their launches and re-reads; bound by the latency of its four
+// meetings and of the scattered list stores. Build of 66,356 weights 42.5 ->
+// 29 us, of 1,000 33 -> 18 us, of 3 28 -> 13 us; 131,072 weights 57 -> 41 us (the
+// separate kernels, which take over above, 53 us at 131,073).
+constexpr int kListBlock = 1024, kListItems = 8, kListCluster = 16;
+constexpr uint32_t kListMax = (uint32_t)kListBlock * kListItems * kListCluster;  // 131,072 weights
+// Tables of up to this many weights get their entries from the same launch
+// (100 weights: 16.8 -> 14.0 us; at 1,000 one SM's FP64 units take longer than
+// another launch: 18.3 -> 25.0 us).
+constexpr uint32_t kListWhole = 256;
+static_assert(kListWhole <= kListBlock, "one block");
+
+__global__ void __launch_bounds__(kListBlock) k_sweep_lists(const float *__restrict__ w, uint32_t n, uint32_t per_thread,
+                                                            SweepScalars *sc, int32_t *lights, i128 *Dexcl, int32_t *heavies,
+                                                            i128 *Sincl, dr_alias_entry *__restrict__ out)
+{
+    cg::cluster_group cluster = cg::this_cluster();
+    const unsigned rank = cluster.block_rank(), blocks = cluster.num_blocks();
+    struct Meet {
+        int emax;
+        unsigned long long W;
+        int lights;
+        i128 D, S;
+    };
+    __shared__ Meet s_meet;  // this block's sums, read by the others
+    __shared__ Meet s_all;   // over the cluster (exponent, total), or over the blocks before this one
+    __shared__ int s_all_lights;
+    __shared__ i128 s_all_D;
+    __shared__ unsigned long long s_warp[32];
+    __shared__ int s_cnt[32];
+    __shared__ i128 s_D[32], s_S[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t first = (rank * kListBlock + threadIdx.x) * per_thread;
+    float x[kListItems];
+    int e = INT_MIN;
+#pragma unroll
+    for (int k = 0; k < kListItems; ++k) {
+        x[k] = (uint32_t)k < per_thread && first + k < n ? clamp_weight(w[first + k]) : 0.0f;
+        if (x[k] > 0.0f) e = max(e, float_exponent(x[k]));
+    }
+    // largest exponent: of the block, then one lane per block of the cluster
+    e = __reduce_max_sync(0xffffffffu, e);
+    if (lane == 0) s_cnt[warp] = e;
+    __syncthreads();
+    if (warp == 0) {
+        e = __reduce_max_sync(0xffffffffu, s_cnt[lane]);
+        if (lane == 0) s_meet.emax = e;
+    }
+    cluster.sync();
+    if (warp == 0) {
+        e = (unsigned)lane < blocks ? cluster.map_shared_rank(&s_meet, lane)->emax : INT_MIN;
+        e = __reduce_max_sync(0xffffffffu, e);
+        if (lane == 0) s_all.emax = e;
+    }
+    __syncthreads();
+    e = s_all.emax;
+    const int lg = 32 - __clz((int)n);  // smallest lg with 2^lg >= n + 1
+    const int shift = 61 - lg - e;
+    // total
+    auto weight_of = [&](int k) { return e == INT_MIN ? 0ll : fixed_weight_bits(x[k], shift); };
+    unsigned long long W = 0;
+#pragma unroll
+    for (int k = 0; k < kListItems; ++k) W += (unsigned long long)weight_of(k);
+    for (int off = 16; off > 0; off >>= 1) W += __shfl_xor_sync(0xffffffffu, W, off);
+    if (lane == 0) s_warp[warp] = W;
+    __syncthreads();
+    if (warp == 0) {
+        W = s_warp[lane];
+        for (int off = 16; off > 0; off >>= 1) W += __shfl_xor_sync(0xffffffffu, W, off);
+        if (lane == 0) s_meet.W = W;
+    }
+    cluster.sync();
+    if (warp == 0) {
+        W = (unsigned)lane < blocks ? cluster.map_shared_rank(&s_meet, lane)->W : 0ull;
+        for (int off = 16; off > 0; off >>= 1) W += __shfl_xor_sync(0xffffffffu, W, off);
+        if (lane == 0) s_all.W = W;
+    }
+    __syncthreads();
+    W = s_all.W;
+    // light count, deficit and surplus sums before each thread's items
+    int cnt = 0;
+    i128 D = 0, S = 0;
+#pragma unroll
+    for (int k = 0; k < kListItems; ++k) {
+        if ((uint32_t)k >= per_thread || first + k >= n) break;
+        const long long a = (long long)n * weight_of(k) - (long long)W;
+        if (a < 0) {
+            ++cnt;
+            D += (i128)(-a);
+        } else {
+            S += (i128)a;
+        }
+    }
+    const int c_inc = warp_scan_int(cnt);
+    const i128 d_inc = warp_scan_i128(D), s_inc = warp_scan_i128(S);
+    if (lane == 31) s_cnt[warp] = c_inc, s_D[warp] = d_inc, s_S[warp] = s_inc;
+    __syncthreads();
+    if (warp == 0) {
+        const int c = warp_scan_int(s_cnt[lane]);
+        const i128 d = warp_scan_i128(s_D[lane]), q = warp_scan_i128(s_S[lane]);
+        s_cnt[lane] = c, s_D[lane] = d, s_S[lane] = q;
+        if (lane == 31) s_meet.lights = c, s_meet.D = d, s_meet.S = q;
+    }
+    cluster.sync();
+    if (warp == 0) {
+        int c = 0;
+        i128 d = 0, q = 0;
+        if ((unsigned)lane < blocks) {
+            const Meet *o = cluster.map_shared_rank(&s_meet, lane);
+            c = o->lights, d = o->D, q = o->S;
+        }
+        const int ci = warp_scan_int(c);
+        const i128 di = warp_scan_i128(d), qi = warp_scan_i128(q);
+        if ((unsigned)lane == rank) s_all.lights = ci - c, s_all.D = di - d, s_all.S = qi - q;
+        if (lane == 31) s_all_lights = ci, s_all_D = di;
+    }
+    cluster.sync();  // no block leaves while another reads its sums
+    int rank_l = s_all.lights + c_inc - cnt + (warp > 0 ? s_cnt[warp - 1] : 0);
+    i128 Db = s_all.D + d_inc - D + (warp > 0 ? s_D[warp - 1] : (i128)0);
+    i128 Sb = s_all.S + s_inc - S + (warp > 0 ? s_S[warp - 1] : (i128)0);
+    // the lists, in index order, with their running sums
+#pragma unroll
+    for (int k = 0; k < kListItems; ++k) {
+        if ((uint32_t)k >= per_thread || first + k >= n) break;
+        const long long a = (long long)n * weight_of(k) - (long long)W;
+        if (a < 0) {
+            lights[rank_l] = (int32_t)(first + k);
+            Dexcl[rank_l] = Db;
+            ++rank_l;
+            Db += (i128)(-a);
+        } else {
+            const int32_t h = (int32_t)(first + k) - rank_l;
+            Sb += (i128)a;
+            heavies[h] = (int32_t)(first + k);
+            Sincl[h] = Sb;
+        }
+    }
+    __shared__ SweepScalars s_sc;
+    if (threadIdx.x == 0) {
+        const float Wf = e == INT_MIN ? 0.0f : (float)ldexp((double)W, -shift);
+        s_sc.emax = e;
+        s_sc.lg = lg;
+        s_sc.shift = shift;
+        s_sc.uniform = !(Wf >= 1e-5f);
+        s_sc.W = W;
+        s_sc.num_lights = s_all_lights;
+        s_sc.num_heavies = (int32_t)n - s_all_lights;
+        s_sc.D_total = s_all_D;
+        s_sc.Wd = (double)W;
+        s_sc.inv_W = 1.0 / s_sc.Wd;
+        s_sc.nd = (double)n;
+        if (rank == 0) *sc = s_sc;
+    }
+    if (n > kListWhole) return;
+    // a small table's entries too, without another launch
+    __shared__ i128 s_fine_S[kCoarse], s_fine_D[kCoarse];
+    __syncthreads();
+    const SweepScalars &s = s_sc;
+    const int32_t step_S = coarse_step(s.num_heavies), step_D = coarse_step(s.num_lights), c = (int32_t)threadIdx.x;
+    if (c < kCoarse && s.num_heavies > 0) s_fine_S[c] = Sincl[min((c + 1) * step_S, s.num_heavies) - 1];
+    if (c < kCoarse && s.num_lights > 0) s_fine_D[c] = Dexcl[min((c + 1) * step_D, s.num_lights) - 1];
+    __syncthreads();
+    for (uint32_t t = threadIdx.x; t < n; t += kListBlock) {
+        if (s.uniform) out[t] = dr_alias_entry{1.0f, 1.0f / (float)n, 0.0f, (int32_t)t, -1};
+        else sweep_assign_item(t, w, n, s, lights, Dexcl, heavies, Sincl, s_fine_S, step_S, s_fine_D, step_D, out);
+    }
+}
+
+static cudaError_t launch_sweep_lists(const float *w, uint32_t n, SweepScalars *sc, int32_t *lights, i128 *Dexcl, int32_t *heavies,
+                                      i128 *Sincl, dr_alias_entry *out, cudaStream_t st)
+{
+    // as few blocks as give every thread one item, up to the cluster's 16; then more items
+    unsigned blocks = 1;
+    while (blocks < kListCluster && (uint64_t)blocks * kListBlock < n) blocks *= 2;
+    const uint32_t per_thread = (n + blocks * kListBlock - 1) / (blocks * kListBlock);
+    cudaError_t e = cudaFuncSetAttribute(k_sweep_lists, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(kListBlock);
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = blocks;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, k_sweep_lists, w, n, per_thread, sc, lights, Dexcl, heavies, Sincl, out);
+    if (e != cudaSuccess || n <= kListWhole) return e;
+    k_sweep_assign<<<(n + kCoarse - 1) / kCoarse, kCoarse, 0, st>>>(w, n, sc, lights, Dexcl, heavies, Sincl, out);
+    return cudaGetLastError();
 }
 
 // ---- sweep build of many small tables, one thread per table ---------------------------
@@ -661,6 +940,7 @@ cudaError_t launch_alias_build(const float *w, uint32_t n, dr_alias_entry *out, 
     i128 *Sincl = Dexcl + n;
     int32_t *lights = reinterpret_cast<int32_t *>(Sincl + n);
     int32_t *heavies = lights + n;
+    if (n <= kListMax) return launch_sweep_lists(w, n, sc, lights, Dexcl, heavies, Sincl, out, st);
     const int grid = (int)std::min<uint32_t>((n + 255) / 256, (uint32_t)num_sms * 8);
     k_sweep_init<<<1, 32, 0, st>>>(sc, n);
     k_sweep_exponent<<<grid, 256, 0, st>>>(w, n, sc);
@@ -668,7 +948,7 @@ cudaError_t launch_alias_build(const float *w, uint32_t n, dr_alias_entry *out, 
     k_sweep_tile_aggregates<<<tiles, kSweepBlock, 0, st>>>(w, n, sc, tile_agg);
     k_sweep_scan_tiles<<<1, kSweepBlock, 0, st>>>(tile_agg, tiles, sc, n);
     k_sweep_scatter<<<tiles, kSweepBlock, 0, st>>>(w, n, sc, tile_agg, lights, Dexcl, heavies, Sincl);
-    k_sweep_assign<<<(n + 255) / 256, 256, 0, st>>>(w, n, sc, lights, Dexcl, heavies, Sincl, out);
+    k_sweep_assign<<<(n + kCoarse - 1) / kCoarse, kCoarse, 0, st>>>(w, n, sc, lights, Dexcl, heavies, Sincl, out);
     return cudaGetLastError();
 }
 

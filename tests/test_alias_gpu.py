@@ -90,3 +90,23 @@ def test_device_sampling_matches_oracle(native, ctx, oracle, mode):
     # empirical frequencies follow the weights
     freq = np.bincount(idx, minlength=n) / len(u)
     assert np.abs(freq - w / w.sum()).max() < 2e-3
+
+
+@pytest.mark.parametrize("n", [31, 1024, 1025, 2049, 16384, 16385, 32769, 66356, 131071, 131072, 131073])
+@pytest.mark.parametrize("kind", ["lognormal", "wide", "one"])
+def test_sweep_mode_at_cluster_sizes(native, ctx, oracle, n, kind):
+    """Sizes where the one-launch list build takes another block or item per
+    thread, and the first size of the separate kernels; weights over the whole
+    exponent range (denormal ones among them), and a single non-zero weight."""
+    rng = np.random.default_rng(n)
+    if kind == "lognormal":
+        w = rng.lognormal(0, 1.5, n).astype(np.float32)
+    elif kind == "wide":
+        w = np.ldexp(rng.uniform(0.5, 1.0, n), rng.integers(-148, 128, n)).astype(np.float32)
+        w[rng.random(n) < 0.5] = 0.0
+        w[n // 2] = 1.0
+    else:
+        w = np.zeros(n, np.float32)
+        w[n - 1] = 2.5
+    tab = device_build(ctx, native, w, native.DR_ALIAS_SWEEP)
+    assert tab.tobytes() == oracle.alias_build_sweep(w).tobytes()
