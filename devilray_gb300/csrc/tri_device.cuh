@@ -24,10 +24,20 @@ struct DevRay {
 };
 
 // Reciprocal that maps a zero (or denormal) direction component to +-1e30 so
-// slab times stay finite and ordered.
+// slab times stay finite and ordered. Only the box tests use it, where its error
+// scales every slab time of an axis alike: on the device the hardware's
+// reciprocal (one ulp) instead of a division, well inside their relative margin
+// of 2^-19 (kBoxFarScale).
 __host__ __device__ __forceinline__ float safe_rcp(float x)
 {
-    return 1.0f / (fabsf(x) >= 1e-30f ? x : copysignf(1e-30f, x));
+    const float y = fabsf(x) >= 1e-30f ? x : copysignf(1e-30f, x);
+#if defined(__CUDA_ARCH__)
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
+    return r;
+#else
+    return 1.0f / y;
+#endif
 }
 
 // Ray from values (origin, direction, tmax); false for a non-finite origin or
@@ -39,11 +49,20 @@ __host__ __device__ __forceinline__ bool make_dev_ray(float3 o, float3 v, float 
     r.v = v;
     r.inv = make_float3(safe_rcp(v.x), safe_rcp(v.y), safe_rcp(v.z));
     r.ooi = make_float3(o.x * r.inv.x, o.y * r.inv.y, o.z * r.inv.z);
+#if defined(__CUDA_ARCH__)
+    // largest magnitudes, NaN if any component is
+    float mo, mv;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(mo) : "f"(fabsf(o.x)), "f"(fabsf(o.y)), "f"(fabsf(o.z)));
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(mv) : "f"(fabsf(v.x)), "f"(fabsf(v.y)), "f"(fabsf(v.z)));
+    const float inf = __int_as_float(0x7f800000);
+    return mo < inf && mv < inf && mv > 0.0f;
+#else
     using std::isfinite;
     const bool finite = isfinite(o.x) && isfinite(o.y) && isfinite(o.z) && isfinite(v.x) && isfinite(v.y) &&
                         isfinite(v.z);
     const bool nonzero = !(v.x == 0.0f && v.y == 0.0f && v.z == 0.0f);
     return finite && nonzero;
+#endif
 }
 
 // Ray i of a GLOBAL-memory dr_ray array (read through the read-only path).
