@@ -19,6 +19,17 @@
 // scenes (dr_batch): every slot carries its job (image), pixel and sample, and
 // the job names the hierarchy root, light tables and camera it uses.
 
+// The renderer's traversal runs the slab FMAs of a pair of slots as scalar FMAs
+// (packed pairs spill at its 64 registers), fetches at most 32 rays at once
+// (its launches are smaller and their rays longer than the public ones) and goes
+// on with extra node tests while 12 lanes can. Measured against packed pairs, 64
+// rays and 16 lanes (box room 256x256, 16 spp / many-light 1080p, 4 spp / guided
+// 480x270): scalar 1,846 -> 1,839 us / 9.95 -> 9.79 ms / 13.39 -> 13.32 ms; with 32
+// rays 1,793 us / 9.70 / 13.19 ms; with 12 lanes 1,790 us / 9.69 / 13.21 ms.
+#define DR_HALF_SCALAR 1
+#define DR_PERSISTENT_CHUNK 32
+#define DR_INNER_MIN_LANES_LANE 12
+
 #include "dr_internal.h"
 #include "render_internal.h"
 #include "alias_kernels.cuh"

@@ -86,8 +86,11 @@ constexpr int kWideStack = 64;
 #define DR_HIT_CHAINS 1
 #endif
 // The FP16 path's slab FMAs as scalar FMAs instead of packed pairs (fewer
-// registers). Measured: 3.283 ms at 7 blocks per SM, 3.371 ms at 8 (64
-// registers, spills); packed pairs 3.192 ms at 7 blocks, 3.308 ms at 8.
+// registers). Public closest hit: 3.283 ms at 7 blocks per SM, 3.371 ms at 8 (64
+// registers, spills); packed pairs 3.192 ms at 7 blocks, 3.308 ms at 8. The
+// renderer, at 64 registers, turns it on (render.cu). (Hit bits from the signs
+// of packed differences through funnel shifts instead of the compare and FMA
+// per slot: 3.130 against 3.132 ms, so dropped.)
 #ifndef DR_HALF_SCALAR
 #define DR_HALF_SCALAR 0
 #endif
