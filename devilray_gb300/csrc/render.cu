@@ -226,6 +226,25 @@ __device__ __forceinline__ uint32_t find_segment(const WaveSegment *segs, uint32
     return lo;
 }
 
+// The image, pixel and sample of a path slot. A wave of one segment (every wave of
+// dr_render) computes them; others read what k_camera stored.
+struct SlotId {
+    uint32_t job, pixel, sample;
+};
+__device__ __forceinline__ SlotId slot_id(const RenderParams &p, uint32_t slot)
+{
+    if (p.nsegs == 1) {
+        const WaveSegment &sg = p.segs[0];
+        const uint32_t local = slot - sg.slot_begin, q = local / sg.npix;
+        return SlotId{sg.job, local - q * sg.npix, p.jobs[sg.job].sample_offset + sg.sample_rel + q};
+    }
+    return SlotId{p.slot_job[slot], p.slot_pix[slot], p.slot_sample[slot]};
+}
+__device__ __forceinline__ uint32_t slot_root(const RenderParams &p, uint32_t slot)
+{
+    return p.jobs[p.nsegs == 1 ? p.segs[0].job : p.slot_job[slot]].root;
+}
+
 // Guided directions drawn below the surface are mirrored into the upper
 // hemisphere (w - 2 (w.n) n) instead of ending the path. With it the density
 // of the guided part at an upper-hemisphere direction w is q(w) + q(R w), R
@@ -371,14 +390,13 @@ __global__ void __launch_bounds__(kRenderBlock) k_camera(RenderParams p)
     camera_ray(J, pixel, sample, o, d);
     p.rays[2 * i] = make_float4(o.x, o.y, o.z, __int_as_float(0x7f800000));
     p.rays[2 * i + 1] = make_float4(d.x, d.y, d.z, 0.0f);
-    p.thr[i] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
     p.color[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    p.prev_p[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // w = 0: no diffuse vertex before
-    p.stack[i] = make_int4(0, 0, 0, 0);                 // w = size
-    p.casts[i] = 0;
-    p.slot_job[i] = sg.job;
-    p.slot_pix[i] = pixel;
-    p.slot_sample[i] = sample;
+    p.stack[i] = make_int4(0, 0, 0, 0);  // w = size
+    if (p.nsegs > 1) {
+        p.slot_job[i] = sg.job;
+        p.slot_pix[i] = pixel;
+        p.slot_sample[i] = sample;
+    }
     if (p.rec_n) p.rec_n[i] = 0;
     p.list[0][i] = i;
 }
@@ -454,14 +472,15 @@ struct BounceSource {
     float2 *hits;
     float4 *color;
     const float4 *pending;
-    const uint32_t *slot_job;
+    const uint32_t *slot_job;  // NULL: every slot has the root `root`
     const RenderJob *jobs;
+    uint32_t root;
     __device__ __forceinline__ bool is_any(uint64_t i) const { return i >= npaths; }
     __device__ __forceinline__ uint32_t slot(uint64_t i) const { return is_any(i) ? shadows[i - npaths] : paths[i]; }
-    __device__ __forceinline__ bool load(uint64_t i, DevRay &r, uint32_t &root) const
+    __device__ __forceinline__ bool load(uint64_t i, DevRay &r, uint32_t &ray_root) const
     {
         const uint32_t s = slot(i);
-        root = jobs[slot_job[s]].root;
+        ray_root = slot_job ? jobs[slot_job[s]].root : root;
         return load_ray(reinterpret_cast<const dr_ray *>(is_any(i) ? shadow_rays : rays), s, r);
     }
     __device__ __forceinline__ void closest(uint64_t i, float t, int32_t prim) const
@@ -494,8 +513,9 @@ __global__ void __launch_bounds__(kTraceBlock, kP8MinBlocks) k_wave_trace_p8(Ren
     const Wide8Args w{p.trace.nodes8, p.trace.tri_ref, p.trace.tri_wt, p.trace.prim, p.trace.num_nodes, p.trace.error,
                       p.trace.stack_limit};
     const uint32_t npaths = b < p.max_depth ? p.counts[b] : 0u, nshadows = b > 0 ? p.counts[64 + b - 1] : 0u;
+    const bool one = p.nsegs == 1;
     const BounceSource src{p.list[b & 1], p.shadow_list, npaths, p.rays, p.shadow_rays, p.hits, p.color, p.pending,
-                           p.slot_job, p.jobs};
+                           one ? nullptr : p.slot_job, p.jobs, one ? p.jobs[p.segs[0].job].root : kNoRoot};
     const uint64_t n = (uint64_t)npaths + nshadows;
     unsigned long long nn = 0, nb = 0, nt = 0, nh = 0;
     persistent_wide<MODE, Query::kMixed, false, false, STACK>(w, src, n, p.work + b, nn, nb, nt, nh, p.chunk);
@@ -527,7 +547,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_wave_closest(RenderParams p, in
         float t = r.tmax;
         int32_t prim = INT_MAX;
         TraceStats st;
-        if (valid) scene_closest<MODE, false, LAYOUT>(p.trace, r, p.jobs[p.slot_job[slot]].root, t, prim, st);
+        if (valid) scene_closest<MODE, false, LAYOUT>(p.trace, r, slot_root(p, slot), t, prim, st);
         p.hits[slot] = prim != INT_MAX ? make_float2(t, __int_as_float(prim))
                                        : make_float2(__int_as_float(0x7f800000), __int_as_float(-1));
     }
@@ -546,8 +566,8 @@ template <bool GUIDED>
 __device__ __forceinline__ void shade_vertex(const RenderParams &p, int b, uint32_t slot, float2 h, bool &keep, bool &shadow)
 {
     bool dead = false;
-    p.casts[slot] += 1;
-    const RenderJob &J = p.jobs[p.slot_job[slot]];
+    const SlotId id = slot_id(p, slot);
+    const RenderJob &J = p.jobs[id.job];
     float *closed = nullptr;  // guided: the record this vertex closes
     if (GUIDED && p.rec_n) {
         // the radiance gathered before this vertex closes the last record
@@ -575,10 +595,10 @@ __device__ __forceinline__ void shade_vertex(const RenderParams &p, int b, uint3
         F3 hp = add(ro, mul(rv, t));
         hp = f3(hp.x * 1.0f + 0.0f, hp.y * 1.0f + 0.0f, hp.z * 1.0f + 0.0f);
         const dr_material &M = p.materials[mat_id];
-        float4 thr = p.thr[slot];
-        float4 col = p.color[slot];
-        const float4 pp4 = p.prev_p[slot];
-        const uint32_t pixel = p.slot_pix[slot], sample = p.slot_sample[slot];
+        // the camera leaves no state: the first vertex has throughput 1 and no
+        // diffuse vertex before it
+        float4 thr = b > 0 ? p.thr[slot] : make_float4(1.0f, 1.0f, 1.0f, 0.0f);
+        const uint32_t pixel = id.pixel, sample = id.sample;
         float u[12];
         const uint32_t g = 1u + 3u * (uint32_t)b;
         uniforms4(J, pixel, sample, g, u);
@@ -588,8 +608,20 @@ __device__ __forceinline__ void shade_vertex(const RenderParams &p, int b, uint3
             const float4 E = make_float4(M.emission[0], M.emission[1], M.emission[2], M.emission[3]);
             const float4 alb = make_float4(M.albedo[0], M.albedo[1], M.albedo[2], M.albedo[3]);
             // misWeightedEmission (PathGeneration.hpp:306-318) with the
-            // pdfs of computeNextBounceMisPdfs (:320-334) for (prev, this)
-            if (pp4.w == 0.0f) {
+            // pdfs of computeNextBounceMisPdfs (:320-334) for (prev, this).
+            // A surface that does not emit adds zeros, which leave the colour as
+            // it is while the throughput is finite: most vertices neither read
+            // nor write it
+            const float inf = __int_as_float(0x7f800000);
+            const bool emits = !(E.x == 0.0f && E.y == 0.0f && E.z == 0.0f && E.w == 0.0f && fabsf(thr.x) < inf &&
+                                 fabsf(thr.y) < inf && fabsf(thr.z) < inf && fabsf(thr.w) < inf);
+            float4 pp4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), col = pp4;
+            if (emits) {
+                col = p.color[slot];
+                if (b > 0) pp4 = p.prev_p[slot];
+            }
+            if (!emits) {
+            } else if (pp4.w == 0.0f) {
                 col = add4(col, mul4(E, thr));
             } else {
                 const float4 pn4 = p.prev_n[slot];
@@ -609,6 +641,7 @@ __device__ __forceinline__ void shade_vertex(const RenderParams &p, int b, uint3
 #endif
                 }
             }
+            if (emits) p.color[slot] = col;
             const float alpha = GUIDED && b < p.guide_bounces ? p.guide_alpha : 0.0f;
 #if DR_GUIDE_DECODED
             const float *lobes = GUIDED ? p.guide_y + (size_t)slot * kGuideOut : nullptr;
@@ -763,15 +796,15 @@ __device__ __forceinline__ void shade_vertex(const RenderParams &p, int b, uint3
             }
             new_o = hp;
             p.stack[slot] = make_int4(stk[0], stk[1], stk[2], ss);
-            p.prev_p[slot] = make_float4(hp.x, hp.y, hp.z, 0.0f);
+            reinterpret_cast<float *>(p.prev_p + slot)[3] = 0.0f;  // no diffuse vertex before the next one
         }
         new_o = add(new_o, mul(normal, 1e-5f));
         p.rays[2 * slot] = make_float4(new_o.x, new_o.y, new_o.z, __int_as_float(0x7f800000));
         p.rays[2 * slot + 1] = make_float4(new_v.x, new_v.y, new_v.z, 0.0f);
-        p.thr[slot] = thr;
-        p.color[slot] = col;
+        if (b == 0 || M.kind == DR_MAT_DIFFUSE) p.thr[slot] = thr;
         keep = b + 1 < (int)J.max_depth && !dead;
     }
+    if (!keep) p.casts[slot] = (uint32_t)b + 1u;  // the path's rays, written where it ends
 }
 
 template <bool GUIDED>
@@ -893,7 +926,7 @@ __global__ void __launch_bounds__(kTraceBlock, 5) k_wave_paths(RenderParams p, i
             alive = true;
             known = traced;
             s_slot[warp][lane] = slot;
-            root = p.jobs[p.slot_job[slot]].root;
+            root = slot_root(p, slot);
         }
         const unsigned path_rays = __ballot_sync(FULL, alive && !known), shadow_rays = __ballot_sync(FULL, shadow);
         if (__ballot_sync(FULL, alive || shadow) == 0) break;
@@ -1063,7 +1096,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_wave_shadow(RenderParams p, int
         const uint32_t slot = p.shadow_list[i];
         DevRay r;
         const bool valid = load_ray(reinterpret_cast<const dr_ray *>(p.shadow_rays), slot, r);
-        const bool occluded = valid && scene_any<MODE, LAYOUT>(p.trace, r, p.jobs[p.slot_job[slot]].root);
+        const bool occluded = valid && scene_any<MODE, LAYOUT>(p.trace, r, slot_root(p, slot));
         if (!occluded) p.color[slot] = add4(p.color[slot], p.pending[slot]);
     }
 }
