@@ -80,36 +80,64 @@ __constant__ float kSrgbStep[255] = {
 // product and of the sum), so the byte is certain unless 255 s lies within
 // kSrgbDoubt of a rounding boundary n + 1/2 (0.2 % of values); there the exact
 // step decides. The double power that this replaces ran at 1/64 of the FP32
-// rate and bound the whole conversion: 1080p 1,036 us with it, 18.4 us now
+// rate and bound the whole conversion: 1080p 1,036 us with it, 18.4 us without
 // (equal bytes for every FP32 value in [0, 1]).
 constexpr float kSrgbDoubt = 1e-3f;
-__device__ __forceinline__ uint32_t srgb_byte(float linear)
+// The byte of the channel sum / samples, inv within an ulp of 1 / samples: the
+// estimate takes the product, the steps the quotient itself.
+__device__ __forceinline__ uint32_t srgb_byte(float sum, float samples, float inv)
 {
-    const float r = fminf(fmaxf(linear, 0.f), 1.f);
+    const float r = fminf(fmaxf(sum * inv, 0.f), 1.f);
     const float v = r < 0.0031308f ? r * (12.92f * 255.0f)
                                    : exp2f(__log2f(r) * (1 / 2.4f)) * (1.055f * 255.0f) - 0.055f * 255.0f;
     const float n = floorf(v);
-    if (fabsf(v - n - 0.5f) < kSrgbDoubt) return (uint32_t)n + (r >= kSrgbStep[(int)n] ? 1u : 0u);
+    if (fabsf(v - n - 0.5f) < kSrgbDoubt) {
+        const float q = fminf(fmaxf(sum / samples, 0.f), 1.f);
+        return (uint32_t)n + (q >= kSrgbStep[(int)n] ? 1u : 0u);
+    }
     return (uint32_t)(v + 0.5f);
 }
 
-// One pixel per thread; memory-bound (16 bytes in, 4 out).
-template <bool GAMMA>
-__global__ void k_tonemap(const float4 *__restrict__ accum, int32_t w, int32_t h, uint32_t *__restrict__ out)
+__device__ __forceinline__ uint32_t tonemap_pixel(const float4 p, bool gamma)
 {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
-    if (x >= w || y >= h) return;
-    const float4 p = accum[x + (size_t)y * w];
-    float r = 0.f, g = 0.f, b = 0.f;
-    if (p.w != 0.f) {
-        r = p.x / p.w;
-        g = p.y / p.w;
-        b = p.z / p.w;
+    if (p.w == 0.f) return 255u << 24;
+    const float r = p.x / p.w, g = p.y / p.w, b = p.z / p.w;
+    if (!gamma) return (255u << 24) | to_u32(r * 255) | (to_u32(g * 255) << 8) | (to_u32(b * 255) << 16);
+    // quotients that are exact: for counts whose reciprocal is no normal number
+    return (255u << 24) | srgb_byte(r, 1.0f, 1.0f) | (srgb_byte(g, 1.0f, 1.0f) << 8) | (srgb_byte(b, 1.0f, 1.0f) << 16);
+}
+
+// kPixels neighbouring columns per thread, each a coalesced load of its own, so
+// that a thread has several pixels in flight; bound by memory (16 bytes in, 4 out
+// per pixel) and the launch. 1 / 2 / 4 pixels: 1080p 12.3 / 10.3 / 11.3 us, 3840x2160
+// 40.8 / 32.8 / 34.9 us (0.75 of the measured HBM rate). With three divisions per
+// pixel, one pixel per thread: 16.5 and 58.3 us.
+constexpr int kPixels = 2;
+template <bool GAMMA>
+__global__ void __launch_bounds__(128) k_tonemap(const float4 *__restrict__ accum, int32_t w, int32_t h, uint32_t *__restrict__ out)
+{
+    const int x0 = blockIdx.x * (128 * kPixels) + threadIdx.x, y = blockIdx.y;
+    float4 p[kPixels];
+#pragma unroll
+    for (int k = 0; k < kPixels; ++k) {
+        const int x = x0 + 128 * k;
+        if (x < w) p[k] = __ldcs(accum + x + (size_t)y * w);
     }
-    uint32_t v = 255u << 24;
-    if (GAMMA) v |= srgb_byte(r) | (srgb_byte(g) << 8) | (srgb_byte(b) << 16);
-    else v |= to_u32(r * 255) | (to_u32(g * 255) << 8) | (to_u32(b * 255) << 16);
-    out[x + (size_t)(h - y - 1) * w] = v;
+#pragma unroll
+    for (int k = 0; k < kPixels; ++k) {
+        const int x = x0 + 128 * k;
+        if (x >= w) break;
+        uint32_t v;
+        if (GAMMA && p[k].w >= 1e-30f && p[k].w <= 1e30f) {
+            float inv;
+            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(p[k].w));
+            v = (255u << 24) | srgb_byte(p[k].x, p[k].w, inv) | (srgb_byte(p[k].y, p[k].w, inv) << 8) |
+                (srgb_byte(p[k].z, p[k].w, inv) << 16);
+        } else {
+            v = tonemap_pixel(p[k], GAMMA);
+        }
+        __stcs(out + x + (size_t)(h - y - 1) * w, v);
+    }
 }
 
 __global__ void k_resolve(const float4 *__restrict__ accum, uint64_t n, float *__restrict__ rgb)
@@ -216,7 +244,7 @@ dr_status dr_tonemap(const float *accum_dev, int32_t width, int32_t height, int3
     DR_CHECK_ARG(accum_dev && rgba_dev && width > 0 && height > 0, "dr_tonemap: bad argument");
     DR_CHECK_ARG(height <= 65535 && (uint64_t)width * (uint64_t)height < (1ull << 31), "dr_tonemap: image too large");
     DR_CHECK_ARG(((uintptr_t)accum_dev & 15) == 0, "dr_tonemap: accum_dev must be 16-byte aligned");
-    const dim3 grid((width + 127) / 128, height);
+    const dim3 grid((width + 128 * kPixels - 1) / (128 * kPixels), height);
     const auto st = static_cast<cudaStream_t>(stream);
     const auto *accum = reinterpret_cast<const float4 *>(accum_dev);
     if (gamma_corrected) k_tonemap<true><<<grid, 128, 0, st>>>(accum, width, height, rgba_dev);
