@@ -272,9 +272,11 @@ __global__ void __launch_bounds__(128) k_guide_infer(const __nv_bfloat16 *wb, co
 // the next layer's input. Groups do not wait for one another: while one is in
 // its chain of MMA, commit, tensor-memory read and barrier, the others encode
 // inputs and run epilogues. Same arithmetic as k_guide_infer (BF16 products,
-// FP32 sums). Bound by that chain's latency with six tiles in flight (0.52 of the
-// issue slots, 0.59 of the shared / tensor memory data path, 0.24 of HBM for
-// 2^20 rows in 118 us; the sines and cosines of the inputs are 19 us of it).
+// FP32 sums). Bound by the shared / tensor memory data path (0.59 of it by loads
+// and stores, the operands of the MMAs beside them) and by that chain's latency;
+// 0.52 of the issue slots, 0.26 of HBM for 2^20 rows in 108 us. The sines and cosines
+// of the inputs are 19 us of it; outputs of whole tiles leave as one bulk copy
+// (117 us when every tile's rows went through loads and stores).
 
 constexpr int kTcRows = 128;
 
@@ -326,9 +328,9 @@ constexpr uint32_t kTcW4 = kTcW1 + 3 * 64 * 64 * 2;  // 48 x 64
 constexpr uint32_t kTcA = kTcW4 + 48 * 64 * 2;       // per group: 128 x 80 input / 128 x 64 hidden / 128 x 40 output
 constexpr uint32_t kTcABytes = kTcRows * kIn * 2;
 static_assert(kTcABytes == kTcRows * kGuideOut * 4, "the output rows fit the input tile");
-// Groups per CTA: 6 run at 80 registers (2^20 rows: 118 us), 5 at 96 (128 us),
-// 7 at 72 (119 us), 8 spill at 64 (130 us). Three CTAs of one group each, with
-// their own copies of the weights, took 178 us.
+// Groups per CTA: 6 run at 80 registers (2^20 rows: 108 us), 5 at 96 (114 us),
+// 7 at 72 with spills (106 us; 200,000 rows 29.4 against 29.0 us), 8 spill at 64.
+// Three CTAs of one group each, with their own copies of the weights, took 178 us.
 constexpr int kInferGroups = 6;
 constexpr uint32_t kTcBias = kTcA + kInferGroups * kTcABytes;
 constexpr uint32_t kTcBar = kTcBias + (4 * kHid + kOut) * 4;  // per group: MMA mbarrier; then copy mbarrier, TMEM address
@@ -376,6 +378,7 @@ __global__ void __launch_bounds__(128 * kInferGroups, 1)
 k_guide_infer_tc(const unsigned char *img, const float *params, GuideParams gp, const float *pos, const float *dir,
                  const uint32_t *list, const uint32_t *count, uint32_t n_fixed, float *y, uint32_t *error)
 {
+    constexpr int kCols = 16;  // accumulator columns an epilogue holds at once
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ int s_failed;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, group = tid >> 7, row = tid & 127;
@@ -443,6 +446,7 @@ k_guide_infer_tc(const unsigned char *img, const float *params, GuideParams gp, 
             }
             *reinterpret_cast<uint4 *>(A + canon_off(row, 8 * j, kTcRows)) = make_uint4(q[0], q[1], q[2], q[3]);
         }
+        const bool run = !DECODED && !list && (tile + 1) * kTcRows <= n;  // the tile's outputs are one run of memory
         uint32_t w_base = smem_u32(smem + kTcW0);
 #pragma unroll 1
         for (int l = 0; l < kLayers; ++l) {
@@ -475,24 +479,24 @@ k_guide_infer_tc(const unsigned char *img, const float *params, GuideParams gp, 
             const float4 *b = reinterpret_cast<const float4 *>(bias + l * kHid);
             if (l < kLayers - 1) {
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    float v[32];
-                    tmem_ld16(lane_addr + 32 * h, v);
-                    tmem_ld16(lane_addr + 32 * h + 16, v + 16);
+                for (int h = 0; h < 64 / kCols; ++h) {
+                    float v[kCols];
+#pragma unroll
+                    for (int c = 0; c < kCols; c += 16) tmem_ld16(lane_addr + kCols * h + c, v + c);
                     asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
+                    for (int j = 0; j < kCols / 8; ++j) {
                         uint32_t q[4];
 #pragma unroll
                         for (int k = 0; k < 2; ++k) {
                             const int i = 8 * j + 4 * k;
-                            const float4 c = b[8 * h + i / 4];
+                            const float4 c = b[kCols / 4 * h + i / 4];
                             const float2 x = __fadd2_rn(make_float2(v[i], v[i + 1]), make_float2(c.x, c.y));
                             const float2 z = __fadd2_rn(make_float2(v[i + 2], v[i + 3]), make_float2(c.z, c.w));
                             q[2 * k] = relu_bf16(x.x, x.y);
                             q[2 * k + 1] = relu_bf16(z.x, z.y);
                         }
-                        *reinterpret_cast<uint4 *>(A + canon_off(row, 32 * h + 8 * j, kTcRows)) =
+                        *reinterpret_cast<uint4 *>(A + canon_off(row, kCols * h + 8 * j, kTcRows)) =
                             make_uint4(q[0], q[1], q[2], q[3]);
                     }
                 }
@@ -500,34 +504,66 @@ k_guide_infer_tc(const unsigned char *img, const float *params, GuideParams gp, 
                 // the output rows, through shared memory (the tile's inputs are
                 // spent): each warp stages its 32 rows and writes them out as
                 // runs of 160 bytes, ten lanes per row
-                float o[48];
-                tmem_ld16(lane_addr, o);
-                tmem_ld16(lane_addr + 16, o + 16);
-                tmem_ld16(lane_addr + 32, o + 32);
-                asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-#pragma unroll
-                for (int i = 0; i < kGuideOut / 4; ++i) {
-                    const float4 c = b[i];
-                    o[4 * i] += c.x, o[4 * i + 1] += c.y, o[4 * i + 2] += c.z, o[4 * i + 3] += c.w;
-                }
-                float4 out[kGuideOut / 4];
-                if (DECODED) {
-                    float v[kGuideOut];
-#pragma unroll
-                    for (int i = 0; i < kGuideOut; ++i) v[i] = o[i];
-                    guide_store_decoded(reinterpret_cast<float *>(out), guide_mix_values(v));
-                } else {
-#pragma unroll
-                    for (int j = 0; j < kGuideOut / 4; ++j) out[j] = make_float4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
-                }
                 // rows 4..7 of every 8 are turned by one float4, so that eight
                 // lanes' stores fall in distinct banks
                 constexpr int kQ = kGuideOut / 4;
                 float4 *stage = reinterpret_cast<float4 *>(A + (warp & 3) * 32 * kGuideOut * 4);
                 const int turn = (lane >> 2) & 1;
+                auto put = [&](int j, float4 q) { stage[lane * kQ + (j < kQ - 1 ? turn + j : turn ? 0 : kQ - 1)] = q; };
+                if (DECODED) {
+                    float o[48], out[kGuideOut];
 #pragma unroll
-                for (int j = 0; j < kQ - 1; ++j) stage[lane * kQ + turn + j] = out[j];
-                stage[lane * kQ + (turn ? 0 : kQ - 1)] = out[kQ - 1];
+                    for (int c = 0; c < 48; c += 16) tmem_ld16(lane_addr + c, o + c);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+                    float v[kGuideOut];
+#pragma unroll
+                    for (int i = 0; i < kQ; ++i) {
+                        const float4 c = b[i];
+                        v[4 * i] = o[4 * i] + c.x, v[4 * i + 1] = o[4 * i + 1] + c.y;
+                        v[4 * i + 2] = o[4 * i + 2] + c.z, v[4 * i + 3] = o[4 * i + 3] + c.w;
+                    }
+                    guide_store_decoded(out, guide_mix_values(v));
+#pragma unroll
+                    for (int j = 0; j < kQ; ++j) put(j, reinterpret_cast<const float4 *>(out)[j]);
+                } else {
+float o[kGuideOut];
+                    {
+                        float v[48];
+#pragma unroll
+                        for (int c = 0; c < 48; c += 16) tmem_ld16(lane_addr + c, v + c);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+                        for (int i = 0; i < kQ; ++i) {
+                            const float4 c = b[i];
+                            o[4 * i] = v[4 * i] + c.x, o[4 * i + 1] = v[4 * i + 1] + c.y;
+                            o[4 * i + 2] = v[4 * i + 2] + c.z, o[4 * i + 3] = v[4 * i + 3] + c.w;
+                        }
+                    }
+                    const float4 *q = reinterpret_cast<const float4 *>(o);
+                    if (run) {
+                        // rows in place; lanes 4..7 of every 8 are one float4 ahead,
+                        // so that eight lanes' stores fall in distinct banks
+#pragma unroll
+                        for (int j = 0; j < kQ; ++j) {
+                            const float4 v0 = q[j], v1 = q[(j + 1) % kQ];
+                            stage[lane * kQ + (turn ? (j + 1) % kQ : j)] =
+                                make_float4(turn ? v1.x : v0.x, turn ? v1.y : v0.y, turn ? v1.z : v0.z, turn ? v1.w : v0.w);
+                        }
+                        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                        group_sync(group);
+                        if (row == 0 && ok) {
+                            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(
+                                             y + (size_t)tile * kTcRows * kGuideOut),
+                                         "r"(a_base), "r"(kTcABytes)
+                                         : "memory");
+                            asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+                            asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
+                        }
+                        break;  // the last layer
+                    }
+#pragma unroll
+                    for (int j = 0; j < kQ; ++j) put(j, q[j]);
+                }
                 __syncwarp();
                 const int part = lane / kQ, col = lane - part * kQ;
 #pragma unroll
