@@ -20,6 +20,7 @@
 #include "mbarrier.cuh"
 #include "guide_math.cuh"
 #include "guide_internal.h"
+#include "launch.cuh"
 
 #include <cuda_bf16.h>
 
@@ -800,9 +801,10 @@ __global__ void __launch_bounds__(128) k_guide_train_fb(const __nv_bfloat16 *wb,
 // CTA's tiles; each CTA writes its sums to a row of `parts`, and k_guide_adam
 // adds the rows in order, so a step has the same bits every time. Bound by the
 // ten dependent matrix products of a tile (3 us per 128 rows; 0.30 of the issue
-// slots, 0.09 of the tensor pipe). An Adam step of 65,536 rows takes 63 us; with
-// one thread per row, 128 threads per CTA and atomic adds of the sums it took
-// 153 us (20 us of it the atomics).
+// slots, 0.09 of the tensor pipe). An Adam step of 65,536 rows takes 57 us (63 us
+// without the programmatic launches of its three kernels); with one thread per
+// row, 128 threads per CTA and atomic adds of the sums it took 153 us (20 us of it
+// the atomics).
 
 // Shared memory of k_guide_train_fused (byte offsets).
 constexpr int kTfThreads = 512;
@@ -853,10 +855,7 @@ k_guide_train_fused(const unsigned char *img, const float *params, GuideParams g
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int row = 32 * (warp & 3) + lane, part = warp >> 2;
     const uint32_t cbar = smem_u32(smem + kTfBar + 16);
-    if (tid == 0) s_failed = 0;
-    if (tid == 0) fetch_weight_image(smem_u32(smem + kTfW), img, kImgBytes, cbar);
     float *bias = reinterpret_cast<float *>(smem + kTfBias);
-    for (int i = tid; i < 4 * kHid + kOut; i += kTfThreads) bias[i] = params[b_off(i / kHid) + i % kHid];
     const uint32_t xoff[kLayers] = {kTfX0, kTfX1, kTfX1 + 20480, kTfX1 + 40960, kTfX1 + 61440};
     // the columns of ones (in .. in + 15) of every x_l
     if (part < 2) {
@@ -876,6 +875,10 @@ k_guide_train_fused(const unsigned char *img, const float *params, GuideParams g
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;\n" ::"r"(tslot) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
+    wait_previous();  // the parameters and the weight sums
+    if (tid == 0) s_failed = 0;
+    if (tid == 0) fetch_weight_image(smem_u32(smem + kTfW), img, kImgBytes, cbar);
+    for (int i = tid; i < 4 * kHid + kOut; i += kTfThreads) bias[i] = params[b_off(i / kHid) + i % kHid];
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
@@ -1096,6 +1099,7 @@ k_guide_train_fused(const unsigned char *img, const float *params, GuideParams g
         });
         first = false;
     }
+    allow_next();
     finish();
     if (!__syncthreads_or(s_failed)) {
         // The CTA's sums: rows m < 64 of dW_l carry the high part of output m, rows
@@ -1229,6 +1233,8 @@ __global__ void __launch_bounds__(256) k_guide_weight_sum(const float *w, uint32
 {
     __shared__ float s[8];
     float v = 0.0f;
+    wait_previous();  // the sums' last reader, and whatever wrote the weights
+    allow_next();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) v += w[i];
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
@@ -1266,6 +1272,8 @@ __global__ void __launch_bounds__(64 * kAdamSplits) k_guide_adam(const float *pa
     __shared__ float s[kAdamSplits][64];
     const int i = blockIdx.x * 64 + (threadIdx.x & 63), split = threadIdx.x >> 6;
     float sum = 0.0f;
+    wait_previous();
+    allow_next();
     if (i <= kNumParams) {
 #pragma unroll 8
         for (int q = split; q < nparts; q += kAdamSplits) sum += parts[(size_t)q * kPartStride + i];
@@ -1409,13 +1417,13 @@ dr_status run_gradients(dr_guide *g, const float *pos, const float *dir, const f
     const GuideParams gp = guide_params(g);
     const unsigned sum_blocks = std::min<unsigned>((n + 255) / 256, kWeightParts);
     float *sums = g->scalars + 4;
-    k_guide_weight_sum<<<sum_blocks, 256, 0, st>>>(weight, n, sums);
+    DR_CUDA(launch_after(k_guide_weight_sum, sum_blocks, 256, 0, st, weight, n, sums));
     if (g->cfg.infer_kernel == DR_GUIDE_INFER_TCGEN05) {
         // one CTA per SM (its shared memory and 512 tensor-memory columns)
         const unsigned tiles = (n + kTcRows - 1) / kTcRows;
         const unsigned blocks = std::min<unsigned>(tiles, (unsigned)g->ctx->num_sms);
-        k_guide_train_fused<<<blocks, kTfThreads, kTfSmem, st>>>(g->img, g->params, gp, pos, dir, sdir, weight, n, sums,
-                                                                 sum_blocks, g->parts, g->ctx->d_error);
+        DR_CUDA(launch_after(k_guide_train_fused, blocks, kTfThreads, kTfSmem, st, g->img, g->params, gp, pos, dir, sdir, weight, n,
+                             sums, sum_blocks, g->parts, g->ctx->d_error));
         *parts = g->parts;
         *nparts = (int)blocks;
     } else {
@@ -1689,9 +1697,9 @@ dr_status dr_guide_train_step(dr_guide *g, const float *pos_dev, const float *di
     const float lr = g->cfg.warmup_steps && (uint32_t)g->step < g->cfg.warmup_steps
                          ? g->cfg.learning_rate * (float)g->step / (float)g->cfg.warmup_steps
                          : g->cfg.learning_rate;
-    k_guide_adam<<<kAdamBlocks, 64 * kAdamSplits, 0, st>>>(parts, nparts, nullptr, g->scalars + 1, true,
-                                              AdamArgs{g->params, g->m, g->v, g->wb, g->img, g->step, lr, g->cfg.beta1,
-                                                       g->cfg.beta2, g->cfg.epsilon});
+    DR_CUDA(launch_after(k_guide_adam, kAdamBlocks, 64 * kAdamSplits, 0, st, parts, nparts, (float *)nullptr, g->scalars + 1, true,
+                         AdamArgs{g->params, g->m, g->v, g->wb, g->img, g->step, lr, g->cfg.beta1, g->cfg.beta2,
+                                  g->cfg.epsilon}));
     DR_CUDA(cudaGetLastError());
     return DR_OK;
 }
