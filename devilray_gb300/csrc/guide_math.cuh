@@ -154,44 +154,45 @@ __host__ __device__ inline float guide_loss_grad(const float *y, float wx, float
     return logq;
 }
 
-// The same gradient by lobe, for threads that share a row. The mixture's log
-// density is LSE(u) - LSE(logits), u_j = logit_j + log vMF_j; the caller forms
-// both sums over the lobes (pi = exp(logit - LSE(logits)), resp = exp(u - LSE(u))).
+// The same gradient by lobe, for threads that share a row: guide_loss_grad's
+// own operations in its order, so that both give the same numbers. The caller
+// forms the sums over the lobes (pi and log q).
 struct GuideLobeTerm {
-    float u, kappa, cosang, inv_n;  // inv_n = 1 / |mean|, 0 for a mean too short to have a direction
+    float t, kappa, cosang, n;  // t = log(pi vMF), n = |mean|
     float mx, my, mz;
 };
 
-__host__ __device__ inline GuideLobeTerm guide_lobe_term(const float *y, float wx, float wy, float wz)
+__host__ __device__ inline GuideLobeTerm guide_lobe_term(const float *y, float pi, float wx, float wy, float wz)
 {
-    GuideLobeTerm t;
-    const float lk = fminf(fmaxf(y[1], kGuideLogKMin), kGuideLogKMax);
-    const float k = guide_exp(lk);
+    GuideLobeTerm T;
+    const float k = guide_exp(fminf(fmaxf(y[1], kGuideLogKMin), kGuideLogKMax));
     const float n2 = y[2] * y[2] + y[3] * y[3] + y[4] * y[4];
+    T.kappa = k;
+    T.n = sqrtf(n2);
     const bool deg = n2 < 1e-24f;
-    const float r = deg ? 0.0f : 1.0f / sqrtf(n2);
-    t.kappa = k;
-    t.inv_n = r;
-    t.mx = y[2] * r, t.my = y[3] * r, t.mz = deg ? 1.0f : y[4] * r;
-    t.cosang = t.mx * wx + t.my * wy + t.mz * wz;
-    // log of the normalisation: log kappa - log 2 pi - log(1 - e^{-2 kappa}); kappa >= e^-4 needs no series
-    t.u = y[0] + (lk - 1.83787706641f - log1pf(-guide_exp(-2.0f * k))) + k * (t.cosang - 1.0f);
-    return t;
+    const float r = 1.0f / T.n;
+    T.mx = deg ? 0.0f : y[2] * r, T.my = deg ? 0.0f : y[3] * r, T.mz = deg ? 1.0f : y[4] * r;
+    T.cosang = T.mx * wx + T.my * wy + T.mz * wz;
+    // kappa >= e^-4: 1 - e^{-2 kappa} needs no series
+    const float lognorm = logf(k) - 1.83787706641f - log1pf(-guide_exp(-2.0f * k));
+    T.t = logf(pi) + lognorm + k * (T.cosang - 1.0f);
+    return T;
 }
 
-__host__ __device__ inline void guide_lobe_grad(const float *y, const GuideLobeTerm &t, float pi, float resp, float wx, float wy,
+__host__ __device__ inline void guide_lobe_grad(const float *y, const GuideLobeTerm &T, float pi, float logq, float wx, float wy,
                                                 float wz, float scale, float *dy)
 {
-    const float k = t.kappa;
+    const float k = T.kappa, resp = guide_exp(T.t - logq);
     dy[0] = -scale * (resp - pi);
     const bool clamped = y[1] < kGuideLogKMin || y[1] > kGuideLogKMax;
     // d log p / d kappa = 1/kappa - 2 / (e^{2 kappa} - 1) + cos - 1
-    const float dk = 1.0f / k - 2.0f / expm1f(2.0f * k) + t.cosang - 1.0f;
+    const float dk = 1.0f / k - 2.0f / expm1f(2.0f * k) + T.cosang - 1.0f;
     dy[1] = clamped ? 0.0f : -scale * resp * dk * k;
-    const float g = -scale * resp * k * t.inv_n;
-    dy[2] = g * (wx - t.cosang * t.mx);
-    dy[3] = g * (wy - t.cosang * t.my);
-    dy[4] = g * (wz - t.cosang * t.mz);
+    const bool deg = T.n < 1e-12f;
+    const float g = -scale * resp * k / T.n;
+    dy[2] = deg ? 0.0f : g * (wx - T.cosang * T.mx);
+    dy[3] = deg ? 0.0f : g * (wy - T.cosang * T.my);
+    dy[4] = deg ? 0.0f : g * (wz - T.cosang * T.mz);
 }
 
 #if defined(__CUDACC__)

@@ -322,6 +322,13 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *v)
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+__device__ __forceinline__ float tmem_ld1(uint32_t taddr)
+{
+    uint32_t r;
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];\n" : "=r"(r) : "r"(taddr));
+    return __uint_as_float(r);
+}
+
 // Shared memory of k_guide_infer_tc (byte offsets).
 constexpr uint32_t kTcW0 = 0;                        // 64 x 80
 constexpr uint32_t kTcW1 = kTcW0 + 64 * 80 * 2;      // 3 x 64 x 64
@@ -801,7 +808,7 @@ __global__ void __launch_bounds__(128) k_guide_train_fb(const __nv_bfloat16 *wb,
 // CTA's tiles; each CTA writes its sums to a row of `parts`, and k_guide_adam
 // adds the rows in order, so a step has the same bits every time. Bound by the
 // ten dependent matrix products of a tile (3 us per 128 rows; 0.30 of the issue
-// slots, 0.09 of the tensor pipe). An Adam step of 65,536 rows takes 57 us (63 us
+// slots, 0.09 of the tensor pipe). An Adam step of 65,536 rows takes 58 us (64 us
 // without the programmatic launches of its three kernels); with one thread per
 // row, 128 threads per CTA and atomic adds of the sums it took 153 us (20 us of it
 // the atomics).
@@ -813,8 +820,8 @@ constexpr uint32_t kTfX1 = kTfX0 + 12 * 2048;                  // x_1..x_4: 128 
 constexpr uint32_t kTfD = kTfX1 + 4 * 10 * 2048;               // two tiles [delta_hi | delta_lo]: 128 x 128
 constexpr uint32_t kTfW = kTfD + 2 * 16 * 2048;                // forward weights, as kTcW0..kTcW4
 constexpr uint32_t kTfBias = kTfW + kImgBytes;
-constexpr uint32_t kTfLse = kTfBias + (4 * kHid + kOut) * 4;   // [part][row] running maxima and sums of the loss
-constexpr uint32_t kTfBar = kTfLse + 4 * kTcRows * 16;         // MMA mbarrier, TMEM address, copy mbarrier
+constexpr uint32_t kTfLse = kTfBias + (4 * kHid + kOut) * 4;   // [part][row] log densities of two lobes
+constexpr uint32_t kTfBar = kTfLse + 4 * kTcRows * 8;          // MMA mbarrier, TMEM address, copy mbarrier
 constexpr uint32_t kTfSmem = kTfBar + 24;
 // tensor-memory columns: [0, 64) the forward / backward product, then dW_l
 __host__ __device__ constexpr uint32_t tf_dcol(int l) { return l == 0 ? 64u : 160u + 80u * (uint32_t)(l - 1); }
@@ -1012,37 +1019,45 @@ k_guide_train_fused(const unsigned char *img, const float *params, GuideParams g
         finish();
         {
             // loss and its gradient: lobes 2 part and 2 part + 1 of the row
-            float v[16], y[10];
+            float v[16], y[10], z[kGuideLobes];
             tmem_ld16(lane_addr + 10 * part, v);
+#pragma unroll
+            for (int j = 0; j < kGuideLobes; ++j) z[j] = tmem_ld1(lane_addr + 5 * j);
             asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
             for (int i = 0; i < 10; ++i) y[i] = v[i] + bias[4 * kHid + 10 * part + i];
+            // mixture weights: every thread of a row takes the sum over all lobes
+            float mx = z[0] = z[0] + bias[4 * kHid];
+#pragma unroll
+            for (int j = 1; j < kGuideLobes; ++j) mx = fmaxf(mx, z[j] = z[j] + bias[4 * kHid + 5 * j]);
+            float s = 0.0f;
+#pragma unroll
+            for (int j = 0; j < kGuideLobes; ++j) s += guide_exp(z[j] - mx);
+            const float inv = 1.0f / s, pi[2] = {guide_exp(y[0] - mx) * inv, guide_exp(y[5] - mx) * inv};
             GuideLobeTerm t[2];
 #pragma unroll
-            for (int j = 0; j < 2; ++j) t[j] = guide_lobe_term(y + 5 * j, wx, wy, wz);
-            const float ml = fmaxf(y[0], y[5]), mu = fmaxf(t[0].u, t[1].u);
-            float4 *lse = reinterpret_cast<float4 *>(smem + kTfLse);
-            lse[part * kTcRows + row] = make_float4(ml, guide_exp(y[0] - ml) + guide_exp(y[5] - ml), mu,
-                                                    guide_exp(t[0].u - mu) + guide_exp(t[1].u - mu));
+            for (int j = 0; j < 2; ++j) t[j] = guide_lobe_term(y + 5 * j, pi[j], wx, wy, wz);
+            float2 *lse = reinterpret_cast<float2 *>(smem + kTfLse);
+            lse[part * kTcRows + row] = make_float2(t[0].t, t[1].t);
             __syncthreads();
-            float4 e[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) e[k] = lse[k * kTcRows + row];
-            const float Ml = fmaxf(fmaxf(e[0].x, e[1].x), fmaxf(e[2].x, e[3].x));
-            const float Mu = fmaxf(fmaxf(e[0].z, e[1].z), fmaxf(e[2].z, e[3].z));
-            float Sl = 0.0f, Su = 0.0f;
+            float2 e[4];
+            mx = -3.0e38f;
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                Sl += e[k].y * guide_exp(e[k].x - Ml);
-                Su += e[k].w * guide_exp(e[k].z - Mu);
+                e[k] = lse[k * kTcRows + row];
+                mx = fmaxf(mx, fmaxf(e[k].x, e[k].y));
             }
-            const float inv_l = 1.0f / Sl, inv_u = 1.0f / Su, scale = live ? c / (float)n : 0.0f;
-            if (part == 0 && live) loss_sum -= scale * ((Mu + logf(Su)) - (Ml + logf(Sl)));
+            s = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                s += guide_exp(e[k].x - mx);
+                s += guide_exp(e[k].y - mx);
+            }
+            const float logq = mx + logf(s), scale = c / (float)n;
+            if (part == 0 && live) loss_sum += -c * logq / (float)n;
             float dy[10];
 #pragma unroll
-            for (int j = 0; j < 2; ++j)
-                guide_lobe_grad(y + 5 * j, t[j], guide_exp(y[5 * j] - Ml) * inv_l, guide_exp(t[j].u - Mu) * inv_u, wx, wy, wz,
-                                scale, dy + 5 * j);
+            for (int j = 0; j < 2; ++j) guide_lobe_grad(y + 5 * j, t[j], pi[j], logq, wx, wy, wz, scale, dy + 5 * j);
 #pragma unroll
             for (int i = 0; i < 5; ++i) {
                 uint32_t hi, lo;
