@@ -390,6 +390,8 @@ k_guide_infer_tc(const unsigned char *img, const float *params, GuideParams gp, 
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ int s_failed;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, group = tid >> 7, row = tid & 127;
+    allow_next();
+    wait_previous();
     const uint32_t n = count ? *count : n_fixed;
     if ((uint64_t)blockIdx.x * kTcRows >= n) return;  // the whole block
     // weights in the canonical layout (B operands: N = outputs, K = inputs):
@@ -1487,8 +1489,9 @@ cudaError_t launch_guide_infer(const dr_guide *g, const float *pos, const float 
         const unsigned tiles = (max_rows + kTcRows - 1) / kTcRows;
         const unsigned blocks = std::min<unsigned>(tiles, (unsigned)g->ctx->num_sms);
         const auto kernel = decoded ? k_guide_infer_tc<true> : k_guide_infer_tc<false>;
-        kernel<<<blocks, 128 * kInferGroups, kTcSmem, st>>>(g->img, g->params, guide_params(g), pos, dir, list, count,
-                                                            max_rows, y, g->ctx->d_error);
+        const cudaError_t e = launch_after(kernel, blocks, 128 * kInferGroups, kTcSmem, st, g->img, g->params, guide_params(g),
+                                           pos, dir, list, count, max_rows, y, g->ctx->d_error);
+        if (e != cudaSuccess) return e;
     } else {
         const unsigned tiles = (max_rows + 15) / 16;
         const unsigned blocks = std::min<unsigned>((tiles + 3) / 4, (unsigned)g->ctx->num_sms * 4);

@@ -18,8 +18,9 @@ namespace dr {
 __device__ __forceinline__ void allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// `early` = false: the ordinary launch, for callers that choose by their stream.
 template <typename... P, typename... A>
-cudaError_t launch_after(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... args)
+cudaError_t launch_next(bool early, void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
@@ -30,8 +31,14 @@ cudaError_t launch_after(void (*kernel)(P...), unsigned grid, unsigned block, si
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = early ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+template <typename... P, typename... A>
+cudaError_t launch_after(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... args)
+{
+    return launch_next(true, kernel, grid, block, smem, st, args...);
 }
 
 }  // namespace dr

@@ -33,6 +33,7 @@
 #include "dr_internal.h"
 #include "render_internal.h"
 #include "alias_kernels.cuh"
+#include "launch.cuh"
 #include "ptmath.cuh"
 #include "trace_device.cuh"
 #include "persistent.cuh"
@@ -379,7 +380,15 @@ __device__ __forceinline__ F3 guide_draw(const GuideMix &M, float u0, float u1, 
 __global__ void __launch_bounds__(kRenderBlock) k_camera(RenderParams p)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) p.counts[0] = p.wave;
+    allow_next();
+    // the wave's counters, which no kernel touches before the next one (waves
+    // smaller than the tables: this block's threads take several entries)
+    if (blockIdx.x == 0)
+        for (uint32_t k = threadIdx.x; k < 128; k += blockDim.x) {
+            p.counts[k] = k == 0 ? p.wave : 0u;
+            p.work[k] = 0;
+            if (p.guide_counts && k < 64) p.guide_counts[k] = 0;
+        }
     if (i >= p.wave) return;
     const WaveSegment sg = p.segs[find_segment<0>(p.segs, p.nsegs, i)];
     const RenderJob &J = p.jobs[sg.job];
@@ -481,7 +490,10 @@ struct BounceSource {
     {
         const uint32_t s = slot(i);
         ray_root = slot_job ? jobs[slot_job[s]].root : root;
-        return load_ray(reinterpret_cast<const dr_ray *>(is_any(i) ? shadow_rays : rays), s, r);
+        // plain loads: the kernel is launched while the one that writes the rays
+        // still runs, which rules out the read-only path
+        const float4 *q = (is_any(i) ? shadow_rays : rays) + 2 * (size_t)s, o = q[0], v = q[1];
+        return make_dev_ray(make_float3(o.x, o.y, o.z), make_float3(v.x, v.y, v.z), o.w, r);
     }
     __device__ __forceinline__ void closest(uint64_t i, float t, int32_t prim) const
     {
@@ -512,11 +524,14 @@ __global__ void __launch_bounds__(kTraceBlock, kP8MinBlocks) k_wave_trace_p8(Ren
 {
     const Wide8Args w{p.trace.nodes8, p.trace.tri_ref, p.trace.tri_wt, p.trace.prim, p.trace.num_nodes, p.trace.error,
                       p.trace.stack_limit};
+    allow_next();
+    wait_previous();
     const uint32_t npaths = b < p.max_depth ? p.counts[b] : 0u, nshadows = b > 0 ? p.counts[64 + b - 1] : 0u;
     const bool one = p.nsegs == 1;
     const BounceSource src{p.list[b & 1], p.shadow_list, npaths, p.rays, p.shadow_rays, p.hits, p.color, p.pending,
                            one ? nullptr : p.slot_job, p.jobs, one ? p.jobs[p.segs[0].job].root : kNoRoot};
     const uint64_t n = (uint64_t)npaths + nshadows;
+    if (n == 0) return;  // k_wave_paths has finished the wave
     unsigned long long nn = 0, nb = 0, nt = 0, nh = 0;
     persistent_wide<MODE, Query::kMixed, false, false, STACK>(w, src, n, p.work + b, nn, nb, nt, nh, p.chunk);
 }
@@ -810,6 +825,8 @@ __device__ __forceinline__ void shade_vertex(const RenderParams &p, int b, uint3
 template <bool GUIDED>
 __global__ void __launch_bounds__(kRenderBlock, GUIDED ? DR_GUIDE_SHADE_BLOCKS : kShadeMinBlocks) k_shade(RenderParams p, int b, uint32_t at_least)
 {
+    allow_next();
+    wait_previous();
     const uint32_t count = p.counts[b];
     if (count < at_least) return;  // k_wave_paths has taken these paths to their ends
     const uint32_t *list = p.list[b & 1];
@@ -897,6 +914,8 @@ __global__ void __launch_bounds__(kTraceBlock, 5) k_wave_paths(RenderParams p, i
 {
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int W = kTraceBlock / 32;
+    allow_next();
+    wait_previous();
     const uint32_t count = p.counts[b0];
     if (b0 > 0 && count > p.path_rays) return;
     __shared__ WarpRays s_rays[W];
@@ -976,6 +995,8 @@ __global__ void __launch_bounds__(kTraceBlock, 5) k_wave_paths(RenderParams p, i
 // the incoming ray, as the shading computes them) and their slot list.
 __global__ void __launch_bounds__(kRenderBlock) k_guide_prepare(RenderParams p, int b)
 {
+    allow_next();
+    wait_previous();
     const uint32_t count = p.counts[b];
     const uint32_t *list = p.list[b & 1];
     const uint32_t warp_first = (blockIdx.x * blockDim.x + (threadIdx.x & ~31u));
@@ -1106,6 +1127,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_wave_shadow(RenderParams p, int
 // in sample order. Waves run this pass one after another.
 __global__ void __launch_bounds__(256) k_accumulate_wave(RenderParams p)
 {
+    wait_previous();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= p.wave_pix) return;
     const WaveSegment sg = p.segs[find_segment<1>(p.segs, p.nsegs, t)];
@@ -1341,6 +1363,13 @@ dr_status WaveRunner::enqueue(const SceneArrays &sc, const WavePlan &plan, const
     const int trace_per_sm = resident_blocks((const void *)p8, kTraceBlock);
     const auto paths = wt ? k_wave_paths<1> : k_wave_paths<0>;
     const int paths_per_sm = resident_blocks((const void *)paths, kTraceBlock);
+    // With one stream the kernels of a wave are launched before their
+    // predecessors end (launch.cuh): box room 16 spp 1.735 -> 1.688 ms, 1080p
+    // 1 spp 3.86 -> 3.80 ms. Blocks that wait hold places on the SMs, which the
+    // waves of other streams could use (many-light 1080p, 4 spp: 9.44 -> 9.98 ms,
+    // so not there); and the whole-path kernel, whose few long blocks are spread
+    // best over empty SMs, starts after the camera rays (432 against 486 us).
+    const bool early = K == 1;
     DR_CUDA(cudaMemsetAsync(d_totals, 0, 2 * sizeof(unsigned long long), st));
     DR_CUDA(cudaEventRecord(fork, st));
     for (int k = 0; k < K; ++k) DR_CUDA(cudaStreamWaitEvent(stream[k], fork, 0));
@@ -1379,25 +1408,22 @@ dr_status WaveRunner::enqueue(const SceneArrays &sc, const WavePlan &plan, const
             const uint64_t rays = (uint64_t)W * (b > 0 && b < (int)plan.max_depth ? 2 : 1);
             return (unsigned)std::min<uint64_t>((rays + kTraceBlock - 1) / kTraceBlock, (uint64_t)sms * trace_per_sm);
         };
-        DR_CUDA(cudaMemsetAsync(q.counts, 0, 128 * sizeof(uint32_t), ws));
-        DR_CUDA(cudaMemsetAsync(q.work, 0, 128 * sizeof(unsigned long long), ws));
-        if (gr) DR_CUDA(cudaMemsetAsync(q.guide_counts, 0, 64 * sizeof(uint32_t), ws));
         k_camera<<<(W + kRenderBlock - 1) / kRenderBlock, kRenderBlock, 0, ws>>>(q);
         // (binary hierarchies and guided bounces keep the per-bounce kernels)
         q.path_rays = wide ? (uint32_t)sms * kTailPathsPerSm : 0u;
         const bool whole = wide && !gr && W <= (uint32_t)sms * kWholePathsPerSm;
         const unsigned path_grid =
             (unsigned)std::min<uint64_t>((W + kTraceBlock / 32 - 1) / (kTraceBlock / 32), (uint64_t)sms * paths_per_sm);
-        if (whole) paths<<<path_grid, kTraceBlock, 0, ws>>>(q, 0, false);
+        if (whole) DR_CUDA(launch_next(false, paths, path_grid, kTraceBlock, 0, ws, q, 0, false));
         for (int b = 0; !whole && b < (int)plan.max_depth; ++b) {
             const bool check = wide && tail_check(b) && b + 2 < (int)plan.max_depth && (!gr || b > (int)gr->bounces);
             if (wide) {
-                p8<<<trace_blocks(b), kTraceBlock, 0, ws>>>(q, b);
+                DR_CUDA(launch_next(early, p8, trace_blocks(b), kTraceBlock, 0, ws, q, b));
             } else {
                 if (wt) k_wave_closest<1, 2><<<trace_grid, kTraceBlock, 0, ws>>>(q, b);
                 else k_wave_closest<0, 2><<<trace_grid, kTraceBlock, 0, ws>>>(q, b);
             }
-            if (check) paths<<<path_grid, kTraceBlock, 0, ws>>>(q, b, true);
+            if (check) DR_CUDA(launch_next(early, paths, path_grid, kTraceBlock, 0, ws, q, b, true));
             // the guided shading kernel serves the guided bounces and the one
             // after them (its emission weights use the mixture density of the
             // last guided direction, and it closes that vertex's training
@@ -1405,27 +1431,28 @@ dr_status WaveRunner::enqueue(const SceneArrays &sc, const WavePlan &plan, const
             // kernel does
             if (gr && b <= (int)gr->bounces) {
                 if (b < (int)gr->bounces) {
-                    k_guide_prepare<<<shade_grid, kRenderBlock, 0, ws>>>(q, b);
+                    DR_CUDA(launch_next(early, k_guide_prepare, shade_grid, kRenderBlock, 0, ws, q, b));
                     DR_CUDA(launch_guide_infer(gr->guide, q.guide_pos, q.guide_nrm, q.guide_list, q.guide_counts + b,
                                                W, q.guide_y, ws, DR_GUIDE_DECODED != 0));
                 }
-                k_shade<true><<<shade_grid, kRenderBlock, 0, ws>>>(q, b, 0u);
+                DR_CUDA(launch_next(early, k_shade<true>, shade_grid, kRenderBlock, 0, ws, q, b, 0u));
             } else {
-                k_shade<false><<<shade_grid, kRenderBlock, 0, ws>>>(q, b, check ? q.path_rays + 1 : 0u);
+                DR_CUDA(launch_next(early, k_shade<false>, shade_grid, kRenderBlock, 0, ws, q, b, check ? q.path_rays + 1 : 0u));
             }
             if (!wide) {
                 if (wt) k_wave_shadow<1, 2><<<trace_grid, kTraceBlock, 0, ws>>>(q, b);
                 else k_wave_shadow<0, 2><<<trace_grid, kTraceBlock, 0, ws>>>(q, b);
             }
         }
-        if (wide && !whole) p8<<<trace_blocks((int)plan.max_depth), kTraceBlock, 0, ws>>>(q, (int)plan.max_depth);
+        if (wide && !whole)
+            DR_CUDA(launch_next(early, p8, trace_blocks((int)plan.max_depth), kTraceBlock, 0, ws, q, (int)plan.max_depth));
         // images receive the waves in order
         if (w > 0) DR_CUDA(cudaStreamWaitEvent(ws, acc_done[(w - 1) % (uint32_t)K], 0));
         if (learn) {
             DR_CUDA(cudaMemsetAsync(q.train_head + 1, 0, sizeof(uint32_t), ws));
             k_guide_collect<<<(W + 255) / 256, 256, 0, ws>>>(q);
         }
-        k_accumulate_wave<<<(q.wave_pix + 255) / 256, 256, 0, ws>>>(q);
+        DR_CUDA(launch_next(early, k_accumulate_wave, (q.wave_pix + 255) / 256, 256, 0, ws, q));
         DR_CUDA(cudaGetLastError());
         if (learn)
             for (uint32_t t = 0; t < gr->steps && (gr->budget == 0 || guide_steps(gr->guide) < gr->budget); ++t) {
