@@ -18,6 +18,7 @@
 
 #include "dr_internal.h"
 #include "alias_kernels.cuh"
+#include "launch.cuh"
 
 #include <cooperative_groups.h>
 
@@ -551,10 +552,12 @@ __device__ __forceinline__ void sweep_assign_item(uint32_t t, const float *__res
 __device__ __forceinline__ int32_t coarse_step(int32_t count) { return (count + kCoarse - 1) / kCoarse; }
 
 __global__ void __launch_bounds__(kCoarse) k_sweep_assign(const float *__restrict__ w, uint32_t n, const SweepScalars *sc,
-                                                          const int32_t *__restrict__ lights, const i128 *__restrict__ Dexcl,
-                                                          const int32_t *__restrict__ heavies, const i128 *__restrict__ Sincl,
-                                                          dr_alias_entry *__restrict__ out)
+                                                          const int32_t *lights, const i128 *Dexcl, const int32_t *heavies,
+                                                          const i128 *Sincl, dr_alias_entry *__restrict__ out)
 {
+    // the lists may still be written when this kernel is launched, so they are
+    // not read through the read-only path
+    wait_previous();
     const SweepScalars s = *sc;
     const uint32_t t = blockIdx.x * kCoarse + threadIdx.x;
     if (s.uniform) {
@@ -580,13 +583,13 @@ __global__ void __launch_bounds__(kCoarse) k_sweep_assign(const float *__restric
 // distributed shared memory. The same integers in the same order as the separate
 // kernels, without their launches and re-reads; bound by the latency of its four
 // meetings and of the scattered list stores. Build of 66,356 weights 42.5 ->
-// 29 us, of 1,000 33 -> 18 us, of 3 28 -> 13 us; 131,072 weights 57 -> 41 us (the
+// 29 us, of 1,000 33 -> 17 us, of 3 28 -> 13 us; 131,072 weights 57 -> 39 us (the
 // separate kernels, which take over above, 53 us at 131,073).
 constexpr int kListBlock = 1024, kListItems = 8, kListCluster = 16;
 constexpr uint32_t kListMax = (uint32_t)kListBlock * kListItems * kListCluster;  // 131,072 weights
 // Tables of up to this many weights get their entries from the same launch
 // (100 weights: 16.8 -> 14.0 us; at 1,000 one SM's FP64 units take longer than
-// another launch: 18.3 -> 25.0 us).
+// another launch: 16.8 -> 25.0 us).
 constexpr uint32_t kListWhole = 256;
 static_assert(kListWhole <= kListBlock, "one block");
 
@@ -611,6 +614,7 @@ __global__ void __launch_bounds__(kListBlock) k_sweep_lists(const float *__restr
     __shared__ i128 s_D[32], s_S[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t first = (rank * kListBlock + threadIdx.x) * per_thread;
+    allow_next();
     float x[kListItems];
     int e = INT_MIN;
 #pragma unroll
@@ -767,8 +771,7 @@ static cudaError_t launch_sweep_lists(const float *w, uint32_t n, SweepScalars *
     cfg.numAttrs = 1;
     e = cudaLaunchKernelEx(&cfg, k_sweep_lists, w, n, per_thread, sc, lights, Dexcl, heavies, Sincl, out);
     if (e != cudaSuccess || n <= kListWhole) return e;
-    k_sweep_assign<<<(n + kCoarse - 1) / kCoarse, kCoarse, 0, st>>>(w, n, sc, lights, Dexcl, heavies, Sincl, out);
-    return cudaGetLastError();
+    return launch_after(k_sweep_assign, (n + kCoarse - 1) / kCoarse, kCoarse, 0, st, w, n, sc, lights, Dexcl, heavies, Sincl, out);
 }
 
 // ---- sweep build of many small tables, one thread per table ---------------------------

@@ -87,3 +87,30 @@ def test_whole_paths_equal_waves(native, ctx, oracle, mode, kind, w, h, depth):
         acc = images[0][0].cpu().numpy()
         assert np.array_equal(acc[pix].view(np.uint32), oacc[pix].view(np.uint32))
         assert np.array_equal(images[0][1].cpu().numpy()[pix], ocasts[pix].astype(np.int64))
+
+
+@pytest.mark.parametrize("streams", [1, 2])
+def test_captured_waves_equal_a_plain_render(native, ctx, streams):
+    """Waves above the whole-path limit as one captured schedule: with one
+    stream their kernels are launched before their predecessors end, with more
+    they are not. Two replays against one plain render of twice the samples."""
+    scene = native.Scene.from_spec(ctx, scenes.box_room(2))
+    cam, depth, n = scenes.camera(405, 384), 7, 405 * 384
+    images = []
+    for replays in (2, 0):
+        acc = torch.zeros((n, 4), dtype=torch.float32, device="cuda")
+        casts = torch.zeros(n, dtype=torch.int32, device="cuda")
+        if replays:
+            job = native.make_job(scene, cam, acc, casts, spp=4, max_depth=depth, seed=6)
+            batch = native.Batch(ctx, [job], wave_paths=2 * n, streams=streams, use_graph=True)
+            for _ in range(replays):
+                batch.render()
+            torch.cuda.synchronize()
+            assert batch.info().num_waves == 2
+            batch.close()
+        else:
+            scene.render(cam, acc, casts, spp=8, max_depth=depth, seed=6)
+            torch.cuda.synchronize()
+        images.append((acc, casts))
+    assert torch.equal(images[0][0].view(torch.int32), images[1][0].view(torch.int32))
+    assert torch.equal(images[0][1], images[1][1])
