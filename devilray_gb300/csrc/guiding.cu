@@ -788,7 +788,7 @@ __global__ void __launch_bounds__(128) k_guide_train_fb(const __nv_bfloat16 *wb,
 
 // ---- training on the 5th-generation tensor cores (tcgen05) ----------------------
 //
-// One CTA of 512 threads per SM carries 128-row tiles through the forward pass,
+// One CTA of 512 workers per SM carries 128-row tiles through the forward pass,
 // the loss gradient, the backward deltas and the weight gradients, with the
 // same arithmetic as k_guide_train_fb + k_guide_wgrad (BF16 operands, FP32
 // sums; deltas enter the tensor cores as a BF16 high part plus a BF16
@@ -808,15 +808,22 @@ __global__ void __launch_bounds__(128) k_guide_train_fb(const __nv_bfloat16 *wb,
 // alternate between layers, so the weight gradient of a layer runs while the
 // next delta is formed. The per-layer sums stay in tensor memory across the
 // CTA's tiles; each CTA writes its sums to a row of `parts`, and k_guide_adam
-// adds the rows in order, so a step has the same bits every time. Bound by the
-// ten dependent matrix products of a tile (3 us per 128 rows; 0.30 of the issue
-// slots, 0.09 of the tensor pipe). An Adam step of 65,536 rows takes 58 us (64 us
-// without the programmatic launches of its three kernels); with one thread per
-// row, 128 threads per CTA and atomic adds of the sums it took 153 us (20 us of it
-// the atomics).
+// adds the rows in order, so a step has the same bits every time.
+//
+// Bound by the serial chain of a tile, 16,500 cycles: five forward steps of 950
+// cycles (operands ready, four products, epilogue), the loss gradient 4,700
+// (issue slots), four backward steps of 1,450 (eight products behind the eight
+// of the last weight gradient), the last weight gradient. Shared memory holds
+// one tile, so nothing else can run meanwhile but the encoding of the next
+// tile's rows, which is spread over the waits. The products are issued by a
+// warp of their own, which alone waits for all workers. An Adam step of 65,536
+// rows takes 51 us (58 us with the products issued by a worker and the encoding
+// between the tiles, 64 us without the programmatic launches of its three
+// kernels); with one thread per row, 128 threads per CTA and atomic adds of the
+// sums it took 153 us (20 us of it the atomics).
 
 // Shared memory of k_guide_train_fused (byte offsets).
-constexpr int kTfThreads = 512;
+constexpr int kTfThreads = 512;  // workers; one more warp issues the products
 constexpr uint32_t kTfX0 = 0;                                  // x_0: 128 x (80 + 16)
 constexpr uint32_t kTfX1 = kTfX0 + 12 * 2048;                  // x_1..x_4: 128 x (64 + 16) each
 constexpr uint32_t kTfD = kTfX1 + 4 * 10 * 2048;               // two tiles [delta_hi | delta_lo]: 128 x 128
@@ -827,11 +834,10 @@ constexpr uint32_t kTfBar = kTfLse + 4 * kTcRows * 8;          // MMA mbarrier, 
 constexpr uint32_t kTfSmem = kTfBar + 24;
 // tensor-memory columns: [0, 64) the forward / backward product, then dW_l
 __host__ __device__ constexpr uint32_t tf_dcol(int l) { return l == 0 ? 64u : 160u + 80u * (uint32_t)(l - 1); }
-// 16-column chunks of dW_l (weights and the bias column), numbered over all layers
-__host__ __device__ constexpr int tf_chunks(int l) { return fan_in(l) / 16 + 1; }
-__host__ __device__ constexpr int tf_chunk0(int l) { return l == 0 ? 0 : tf_chunk0(l - 1) + tf_chunks(l - 1); }
-constexpr int kTfStage = 20;  // floats per staged row of a chunk: 16 and a pad that spreads the banks
-static_assert(tf_chunk0(kLayers) * 64 * kTfStage * 4 <= (int)kTfW, "the staged gradients fit the tiles");
+// 16-column chunks of the dW_l (weights and the bias column), in order of their columns
+constexpr int kTfChunks = 6 + 4 * 5;
+static_assert(tf_dcol(1) == 64 + 16 * 6 && tf_dcol(4) + 80 == 64 + 16 * kTfChunks, "chunk f begins at column 64 + 16 f");
+static_assert(2 * kTfChunks * 64 * 64 <= (int)kTfBias, "the staged sums fit the tiles and the weights");
 // floats of one CTA's row of partial sums: the gradients, the loss
 constexpr int kPartStride = (kNumParams + 1 + 31) & ~31;
 constexpr int kWeightParts = 64;  // blocks of k_guide_weight_sum
@@ -853,7 +859,25 @@ __device__ __forceinline__ void split_bf16(float c0, float c1, uint32_t &hi, uin
     lo = pack_bf16(c0 - hf.x, c1 - hf.y);
 }
 
-__global__ void __launch_bounds__(kTfThreads, 1)
+// Named barriers of k_guide_train_fused (0 is __syncthreads).
+constexpr int kTfRowBar = 1;    // + row group: the four threads of each of 32 rows
+constexpr int kTfReadyBar = 5;  // the operands of the next products are in shared memory
+constexpr int kTfWorkBar = 6;   // all workers
+__device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id, int threads)
+{
+    asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
+}
+
+// True in one lane of a converged warp, always the same one.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t one;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+    return one != 0;
+}
+
+__global__ void __launch_bounds__(kTfThreads + 32, 1)
 k_guide_train_fused(const unsigned char *img, const float *params, GuideParams gp, const float *pos, const float *dir,
                     const float *sdir, const float *weight, uint32_t n, const float *weight_parts, uint32_t nweight,
                     float *parts, uint32_t *error)
@@ -861,8 +885,9 @@ k_guide_train_fused(const unsigned char *img, const float *params, GuideParams g
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ float s_loss[4];
     __shared__ int s_failed;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int row = 32 * (warp & 3) + lane, part = warp >> 2;
+    const bool worker = warp < kTfThreads / 32;  // the last warp issues the products
     const uint32_t cbar = smem_u32(smem + kTfBar + 16);
     float *bias = reinterpret_cast<float *>(smem + kTfBias);
     const uint32_t xoff[kLayers] = {kTfX0, kTfX1, kTfX1 + 20480, kTfX1 + 40960, kTfX1 + 61440};
@@ -887,287 +912,316 @@ k_guide_train_fused(const unsigned char *img, const float *params, GuideParams g
     wait_previous();  // the parameters and the weight sums
     if (tid == 0) s_failed = 0;
     if (tid == 0) fetch_weight_image(smem_u32(smem + kTfW), img, kImgBytes, cbar);
-    for (int i = tid; i < 4 * kHid + kOut; i += kTfThreads) bias[i] = params[b_off(i / kHid) + i % kHid];
+    for (int i = tid; i < 4 * kHid + kOut; i += kTfThreads + 32) bias[i] = params[b_off(i / kHid) + i % kHid];
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t taddr = *reinterpret_cast<volatile uint32_t *>(smem + kTfBar + 8);
-    const uint32_t lane_addr = taddr + ((uint32_t)(32 * (warp & 3)) << 16);
-    const uint32_t d_base = smem_u32(smem + kTfD), w_img = smem_u32(smem + kTfW);
-    // mean sample weight: the same sum in every thread of every block
-    float wsum = (uint32_t)lane < nweight ? weight_parts[lane] : 0.0f;
-    if ((uint32_t)lane + 32 < nweight) wsum += weight_parts[lane + 32];
-    for (int o = 16; o > 0; o >>= 1) wsum += __shfl_xor_sync(0xffffffffu, wsum, o);
-    const float wmean = wsum / (float)n;
-    float loss_sum = 0.0f;  // of the part 0 threads' rows
-    uint32_t phase = 0;
-    bool first = true;
+    const uint32_t d_base = smem_u32(smem + kTfD), w_img = smem_u32(smem + kTfW), x_base = smem_u32(smem);
+    const uint32_t woff[kLayers] = {kTcW0, kTcW1, kTcW1 + 8192, kTcW1 + 16384, kTcW4};
     if (!mbar_wait(cbar, 0)) {  // the weights have landed
         *reinterpret_cast<volatile int *>(&s_failed) = 1;
         atomicOr(error, ERR_TIMEOUT);
     }
 
-    // The products of one step, issued by one thread once every thread's shared-memory
-    // stores are done; `issue` commits them to the mbarrier.
-    auto launch = [&](auto issue) {
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-        __syncthreads();
-        if (tid == 0) {
+    if (!worker) {
+        // The products of every step, by one lane of a warp of their own: in a
+        // worker's warp their issue (up to 1,000 cycles a step, as the tensor
+        // pipe takes them) would keep that warp's rows waiting.
+        const bool leader = elect_one();
+        auto ready = [&] {
+            bar_sync(kTfReadyBar, kTfThreads + 32);
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            issue();
-        }
-    };
-    auto commit = [&] {
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(mbar) : "memory");
-    };
-    // Waits for the last commit (which covers every product issued before it).
-    // Every wait is bounded; once one gives up the block runs on without waiting,
-    // so that it ends together, and its sums are dropped.
-    auto finish = [&] {
-        if (!*reinterpret_cast<volatile int *>(&s_failed) && !mbar_wait(mbar, phase)) {
-            *reinterpret_cast<volatile int *>(&s_failed) = 1;
-            atomicOr(error, ERR_TIMEOUT);
-        }
-        phase ^= 1u;
-        __syncwarp();
-        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    };
-    // dW_l += [delta_hi | delta_lo]^T x_l over the tile's 128 rows (8 MMAs of
-    // 16 rows; MN-major operands: 8-row groups 128 B apart, 8-column groups
-    // 2048 B apart)
-    auto wgrad = [&](int l, bool acc) {
-        const uint32_t idesc = idesc_bf16(kTcRows, fan_in(l) + 16) | (1u << 15) | (1u << 16);
-        uint64_t a = smem_desc(d_base + (uint32_t)(l & 1) * 32768, 128, 2048), b = smem_desc(smem_u32(smem) + xoff[l], 128, 2048);
+        };
+        auto commit = [&] {
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(mbar)
+                         : "memory");
+        };
+        // dW_l += [delta_hi | delta_lo]^T x_l over the tile's 128 rows (8 MMAs of
+        // 16 rows; MN-major operands: 8-row groups 128 B apart, 8-column groups
+        // 2048 B apart)
+        auto wgrad = [&](int l, bool acc) {
+            const uint32_t idesc = idesc_bf16(kTcRows, fan_in(l) + 16) | (1u << 15) | (1u << 16);
+            uint64_t a = smem_desc(d_base + (uint32_t)(l & 1) * 32768, 128, 2048), b = smem_desc(x_base + xoff[l], 128, 2048);
 #pragma unroll
-        for (int s2 = 0; s2 < kTcRows / 16; ++s2, a += 16, b += 16) tc_mma(taddr + tf_dcol(l), a, b, idesc, acc || s2 > 0);
-    };
-    const uint32_t woff[kLayers] = {kTcW0, kTcW1, kTcW1 + 8192, kTcW1 + 16384, kTcW4};
-
-    for (uint32_t tile = blockIdx.x; (uint64_t)tile * kTcRows < n; tile += gridDim.x) {
-        const uint32_t r = tile * kTcRows + row;
-        const bool live = r < n;
+            for (int s2 = 0; s2 < kTcRows / 16; ++s2, a += 16, b += 16) tc_mma(taddr + tf_dcol(l), a, b, idesc, acc || s2 > 0);
+        };
+        bool first = true;
+        for (uint32_t tile = blockIdx.x; (uint64_t)tile * kTcRows < n; tile += gridDim.x) {
+#pragma unroll
+            for (int l = 0; l < kLayers; ++l) {  // forward
+                ready();
+                if (leader) {
+                    const uint32_t N = fan_out(l), idesc = idesc_bf16(kTcRows, N);
+                    uint64_t a = smem_desc(x_base + xoff[l], kTcRows * 16, 128), b = smem_desc(w_img + woff[l], N * 16, 128);
+#pragma unroll
+                    for (uint32_t s2 = 0; s2 < fan_in(l) / 16; ++s2, a += kTcRows * 2, b += N * 2) tc_mma(taddr, a, b, idesc, s2 > 0);
+                    commit();
+                }
+                __syncwarp();
+            }
+            // backward: delta_{l-1} = (delta_l W_l) masked by the ReLU of layer
+            // l - 1; dW_l runs behind it
+#pragma unroll
+            for (int l = kLayers - 1; l >= 1; --l) {
+                ready();
+                if (leader) {
+                    const uint32_t O = fan_out(l), idesc = idesc_bf16(kTcRows, kHid) | (1u << 16);
+                    const uint64_t b0 = smem_desc(w_img + woff[l], 128, O * 16);
+#pragma unroll
+                    for (int half = 0; half < 2; ++half) {  // high parts, then remainders
+                        uint64_t a = smem_desc(d_base + (uint32_t)(l & 1) * 32768 + half * 8 * 2048, kTcRows * 16, 128), b = b0;
+#pragma unroll
+                        for (uint32_t s2 = 0; s2 < O / 16; ++s2, a += kTcRows * 2, b += 16) tc_mma(taddr, a, b, idesc, half + s2 > 0);
+                    }
+                    commit();
+                    wgrad(l, !first);
+                }
+                __syncwarp();
+            }
+            ready();
+            if (leader) {
+                wgrad(0, !first);
+                commit();
+            }
+            __syncwarp();
+            first = false;
+        }
+        allow_next();
+    } else {
+        const uint32_t lane_addr = taddr + ((uint32_t)(32 * (warp & 3)) << 16);
+        // mean sample weight: the same sum in every thread of every block
+        float wsum = (uint32_t)lane < nweight ? weight_parts[lane] : 0.0f;
+        if ((uint32_t)lane + 32 < nweight) wsum += weight_parts[lane + 32];
+        for (int o = 16; o > 0; o >>= 1) wsum += __shfl_xor_sync(0xffffffffu, wsum, o);
+        const float wmean = wsum / (float)n;
+        float loss_sum = 0.0f;  // of the part 0 threads' rows
+        uint32_t phase = 0;
+        bool failed = false;  // warp-uniform
+        // this thread's shared-memory stores (and tensor-memory loads) are done
+        auto ready = [&] {
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+            if (failed) bar_sync(kTfReadyBar, kTfThreads + 32);
+            else bar_arrive(kTfReadyBar, kTfThreads + 32);
+        };
+        // Waits for the last commit (which covers every product issued before it).
+        // Every wait is bounded; once one gives up the block runs on without waiting
+        // (but in step, at the barrier), so that it ends together, and its sums are
+        // dropped.
+        auto finish = [&] {
+            bool bad = *reinterpret_cast<volatile int *>(&s_failed) != 0;
+            if (!bad && !mbar_wait(mbar, phase)) {
+                *reinterpret_cast<volatile int *>(&s_failed) = 1;
+                atomicOr(error, ERR_TIMEOUT);
+                bad = true;
+            }
+            phase ^= 1u;
+            failed = __any_sync(0xffffffffu, bad);
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        };
+        // Pair k of the encoded columns of chunk part + 4 j (8 columns) of a row.
+        // A tile's rows are loaded a tile ahead and encoded while the products of
+        // the tile before run (3,700 cycles a tile otherwise).
         float p[3], d[3];
-        uint32_t slot;
-        load_row(pos, dir, nullptr, n, r, gp, p, d, slot);
-        // input row: chunks part, part + 4, part + 8 of 8 encoded columns
         uint32_t in[3][4];
-#pragma unroll
-        for (int j = 0; j < 3; ++j)
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int c = 8 * (part + 4 * j) + 2 * k, axis = c / 24;
-                float v0 = 0.0f, v1 = 0.0f;
-                if (c < 72) {
-                    const float x = axis == 0 ? p[0] : axis == 1 ? p[1] : p[2];
-                    sincospif(x * __int_as_float((127 + ((c % 24) >> 1)) << 23), &v0, &v1);
-                } else if (c == 72) {
-                    v0 = d[0], v1 = d[1];
-                } else if (c == 74) {
-                    v0 = d[2];
-                }
-                in[j][k] = pack_bf16(v0, v1);
+        auto encode = [&](int j, int k) {
+            const int c = 8 * (part + 4 * j) + 2 * k, axis = c / 24;
+            float v0 = 0.0f, v1 = 0.0f;
+            if (c < 72) {
+                const float x = axis == 0 ? p[0] : axis == 1 ? p[1] : p[2];
+                sincospif(x * __int_as_float((127 + ((c % 24) >> 1)) << 23), &v0, &v1);
+            } else if (c == 72) {
+                v0 = d[0], v1 = d[1];
+            } else if (c == 74) {
+                v0 = d[2];
             }
-        // the previous tile's last weight gradient reads x_0 and a delta tile
-        if (!first) finish();
+            in[j][k] = pack_bf16(v0, v1);
+        };
+        uint32_t tile = blockIdx.x, slot;
+        if ((uint64_t)tile * kTcRows < n) {
+            load_row(pos, dir, nullptr, n, tile * kTcRows + row, gp, p, d, slot);
 #pragma unroll
-        for (int j = 0; j < 3; ++j)
-            if (part + 4 * j < kIn / 8)
-                *reinterpret_cast<uint4 *>(smem + kTfX0 + canon_off(row, 8 * (part + 4 * j), kTcRows)) =
-                    make_uint4(in[j][0], in[j][1], in[j][2], in[j][3]);
-        uint64_t mask = 0;  // 16 bits per hidden layer: this thread's columns whose ReLU passes
-#pragma unroll
-        for (int l = 0; l < kLayers - 1; ++l) {
-            launch([&] {
-                const uint32_t idesc = idesc_bf16(kTcRows, kHid);
-                uint64_t a = smem_desc(smem_u32(smem) + xoff[l], kTcRows * 16, 128), b = smem_desc(w_img + woff[l], kHid * 16, 128);
-#pragma unroll
-                for (int s2 = 0; s2 < fan_in(l) / 16; ++s2, a += kTcRows * 2, b += kHid * 2) tc_mma(taddr, a, b, idesc, s2 > 0);
-                commit();
-            });
-            finish();
-            float v[16];
-            tmem_ld16(lane_addr + 16 * part, v);
-            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-            const float4 *b = reinterpret_cast<const float4 *>(bias + l * kHid + 16 * part);
-            uint32_t q[8], m = 0;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float4 c = b[i];
-                q[2 * i] = relu_bf16(v[4 * i] + c.x, v[4 * i + 1] + c.y);
-                q[2 * i + 1] = relu_bf16(v[4 * i + 2] + c.z, v[4 * i + 3] + c.w);
-            }
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                if (q[i] & 0x7fffu) m |= 1u << (2 * i);
-                if (q[i] & 0x7fff0000u) m |= 2u << (2 * i);
-            }
-            mask |= (uint64_t)m << (16 * l);
-            *reinterpret_cast<uint4 *>(smem + xoff[l + 1] + canon_off(row, 16 * part, kTcRows)) = make_uint4(q[0], q[1], q[2], q[3]);
-            *reinterpret_cast<uint4 *>(smem + xoff[l + 1] + canon_off(row, 16 * part + 8, kTcRows)) =
-                make_uint4(q[4], q[5], q[6], q[7]);
+            for (int i = 0; i < 12; ++i) encode(i / 4, i % 4);
         }
-        launch([&] {
-            const uint32_t idesc = idesc_bf16(kTcRows, kOut);
-            uint64_t a = smem_desc(smem_u32(smem) + xoff[4], kTcRows * 16, 128), b = smem_desc(w_img + woff[4], kOut * 16, 128);
+        for (; (uint64_t)tile * kTcRows < n; tile += gridDim.x) {
+            const uint32_t r = tile * kTcRows + row;
+            const bool live = r < n;
 #pragma unroll
-            for (int s2 = 0; s2 < kHid / 16; ++s2, a += kTcRows * 2, b += kOut * 2) tc_mma(taddr, a, b, idesc, s2 > 0);
-            commit();
-        });
-        const float c = live && wmean > 0.0f ? weight[r] / wmean : 0.0f;
-        float wx = 0.0f, wy = 0.0f, wz = 1.0f;
-        if (live) wx = sdir[3 * (size_t)r], wy = sdir[3 * (size_t)r + 1], wz = sdir[3 * (size_t)r + 2];
-        finish();
-        {
-            // loss and its gradient: lobes 2 part and 2 part + 1 of the row
-            float v[16], y[10], z[kGuideLobes];
-            tmem_ld16(lane_addr + 10 * part, v);
+            for (int j = 0; j < 3; ++j)
+                if (part + 4 * j < kIn / 8)
+                    *reinterpret_cast<uint4 *>(smem + kTfX0 + canon_off(row, 8 * (part + 4 * j), kTcRows)) =
+                        make_uint4(in[j][0], in[j][1], in[j][2], in[j][3]);
+            const uint64_t ahead = ((uint64_t)tile + gridDim.x) * kTcRows + row;
 #pragma unroll
-            for (int j = 0; j < kGuideLobes; ++j) z[j] = tmem_ld1(lane_addr + 5 * j);
-            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+            for (int l = 0; l < kLayers - 1; ++l) {
+                ready();
+                if (l == 0) load_row(pos, dir, nullptr, n, (uint32_t)min((uint64_t)n, ahead), gp, p, d, slot);
+                else encode(0, l - 1);
+                finish();
+                float v[16];
+                tmem_ld16(lane_addr + 16 * part, v);
+                asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+                const float4 *b = reinterpret_cast<const float4 *>(bias + l * kHid + 16 * part);
+                uint32_t q[8];
 #pragma unroll
-            for (int i = 0; i < 10; ++i) y[i] = v[i] + bias[4 * kHid + 10 * part + i];
-            // mixture weights: every thread of a row takes the sum over all lobes
-            float mx = z[0] = z[0] + bias[4 * kHid];
-#pragma unroll
-            for (int j = 1; j < kGuideLobes; ++j) mx = fmaxf(mx, z[j] = z[j] + bias[4 * kHid + 5 * j]);
-            float s = 0.0f;
-#pragma unroll
-            for (int j = 0; j < kGuideLobes; ++j) s += guide_exp(z[j] - mx);
-            const float inv = 1.0f / s, pi[2] = {guide_exp(y[0] - mx) * inv, guide_exp(y[5] - mx) * inv};
-            GuideLobeTerm t[2];
-#pragma unroll
-            for (int j = 0; j < 2; ++j) t[j] = guide_lobe_term(y + 5 * j, pi[j], wx, wy, wz);
-            float2 *lse = reinterpret_cast<float2 *>(smem + kTfLse);
-            lse[part * kTcRows + row] = make_float2(t[0].t, t[1].t);
-            __syncthreads();
-            float2 e[4];
-            mx = -3.0e38f;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                e[k] = lse[k * kTcRows + row];
-                mx = fmaxf(mx, fmaxf(e[k].x, e[k].y));
-            }
-            s = 0.0f;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                s += guide_exp(e[k].x - mx);
-                s += guide_exp(e[k].y - mx);
-            }
-            const float logq = mx + logf(s), scale = c / (float)n;
-            if (part == 0 && live) loss_sum += -c * logq / (float)n;
-            float dy[10];
-#pragma unroll
-            for (int j = 0; j < 2; ++j) guide_lobe_grad(y + 5 * j, t[j], pi[j], logq, wx, wy, wz, scale, dy + 5 * j);
-#pragma unroll
-            for (int i = 0; i < 5; ++i) {
-                uint32_t hi, lo;
-                split_bf16(live ? dy[2 * i] : 0.0f, live ? dy[2 * i + 1] : 0.0f, hi, lo);
-                *reinterpret_cast<uint32_t *>(smem + kTfD + canon_off(row, 10 * part + 2 * i, kTcRows)) = hi;
-                *reinterpret_cast<uint32_t *>(smem + kTfD + canon_off(row, 64 + 10 * part + 2 * i, kTcRows)) = lo;
-            }
-            if (part < 3) {  // unused outputs
-                *reinterpret_cast<uint4 *>(smem + kTfD + canon_off(row, kGuideOut + 8 * part, kTcRows)) = make_uint4(0, 0, 0, 0);
-                *reinterpret_cast<uint4 *>(smem + kTfD + canon_off(row, 64 + kGuideOut + 8 * part, kTcRows)) =
-                    make_uint4(0, 0, 0, 0);
-            }
-        }
-        // backward: delta_{l-1} = (delta_l W_l) masked by the ReLU of layer
-        // l - 1; dW_l runs behind it
-#pragma unroll
-        for (int l = kLayers - 1; l >= 1; --l) {
-            const bool acc = !first;
-            launch([&] {
-                const uint32_t idesc = idesc_bf16(kTcRows, kHid) | (1u << 16);
-                const uint32_t O = l == kLayers - 1 ? kOut : kHid;
-                const uint64_t b0 = smem_desc(w_img + woff[l], 128, O * 16);
-#pragma unroll
-                for (int part2 = 0; part2 < 2; ++part2) {  // high parts, then remainders
-                    uint64_t a = smem_desc(d_base + (uint32_t)(l & 1) * 32768 + part2 * 8 * 2048, kTcRows * 16, 128), b = b0;
-#pragma unroll
-                    for (uint32_t s2 = 0; s2 < O / 16; ++s2, a += kTcRows * 2, b += 16) tc_mma(taddr, a, b, idesc, part2 + s2 > 0);
+                for (int i = 0; i < 4; ++i) {
+                    const float4 c = b[i];
+                    const float2 x = __fadd2_rn(make_float2(v[4 * i], v[4 * i + 1]), make_float2(c.x, c.y));
+                    const float2 z = __fadd2_rn(make_float2(v[4 * i + 2], v[4 * i + 3]), make_float2(c.z, c.w));
+                    q[2 * i] = relu_bf16(x.x, x.y);
+                    q[2 * i + 1] = relu_bf16(z.x, z.y);
                 }
-                commit();
-                wgrad(l, acc);
-            });
+                *reinterpret_cast<uint4 *>(smem + xoff[l + 1] + canon_off(row, 16 * part, kTcRows)) = make_uint4(q[0], q[1], q[2], q[3]);
+                *reinterpret_cast<uint4 *>(smem + xoff[l + 1] + canon_off(row, 16 * part + 8, kTcRows)) =
+                    make_uint4(q[4], q[5], q[6], q[7]);
+            }
+            ready();
+            const float c = live && wmean > 0.0f ? weight[r] / wmean : 0.0f;
+            float wx = 0.0f, wy = 0.0f, wz = 1.0f;
+            if (live) wx = sdir[3 * (size_t)r], wy = sdir[3 * (size_t)r + 1], wz = sdir[3 * (size_t)r + 2];
             finish();
-            float v[16];
-            tmem_ld16(lane_addr + 16 * part, v);
-            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-            const uint32_t m = (uint32_t)(mask >> (16 * (l - 1)));
-            unsigned char *D = smem + kTfD + ((l - 1) & 1) * 32768;
+            {
+                // loss and its gradient: lobes 2 part and 2 part + 1 of the row
+                float v[16], y[10], z[kGuideLobes];
+                tmem_ld16(lane_addr + 10 * part, v);
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                uint32_t hi[4], lo[4];
+                for (int j = 0; j < kGuideLobes; ++j) z[j] = tmem_ld1(lane_addr + 5 * j);
+                asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+                for (int i = 0; i < 10; ++i) y[i] = v[i] + bias[4 * kHid + 10 * part + i];
+                // mixture weights: every thread of a row takes the sum over all lobes
+                float mx = z[0] = z[0] + bias[4 * kHid];
+#pragma unroll
+                for (int j = 1; j < kGuideLobes; ++j) mx = fmaxf(mx, z[j] = z[j] + bias[4 * kHid + 5 * j]);
+                float s = 0.0f;
+#pragma unroll
+                for (int j = 0; j < kGuideLobes; ++j) s += guide_exp(z[j] - mx);
+                const float inv = 1.0f / s, pi[2] = {guide_exp(y[0] - mx) * inv, guide_exp(y[5] - mx) * inv};
+                GuideLobeTerm t[2];
+#pragma unroll
+                for (int j = 0; j < 2; ++j) t[j] = guide_lobe_term(y + 5 * j, pi[j], wx, wy, wz);
+                float2 *lse = reinterpret_cast<float2 *>(smem + kTfLse);
+                lse[part * kTcRows + row] = make_float2(t[0].t, t[1].t);
+                bar_sync(kTfRowBar + (warp & 3), 128);
+                float2 e[4];
+                mx = -3.0e38f;
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    const int i = 8 * j + 2 * k;
-                    split_bf16((m >> i) & 1u ? v[i] : 0.0f, (m >> (i + 1)) & 1u ? v[i + 1] : 0.0f, hi[k], lo[k]);
+                    e[k] = lse[k * kTcRows + row];
+                    mx = fmaxf(mx, fmaxf(e[k].x, e[k].y));
                 }
-                *reinterpret_cast<uint4 *>(D + canon_off(row, 16 * part + 8 * j, kTcRows)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                *reinterpret_cast<uint4 *>(D + canon_off(row, 64 + 16 * part + 8 * j, kTcRows)) =
-                    make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                s = 0.0f;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    s += guide_exp(e[k].x - mx);
+                    s += guide_exp(e[k].y - mx);
+                }
+                const float logq = mx + logf(s), scale = c / (float)n;
+                if (part == 0 && live) loss_sum += -c * logq / (float)n;
+                float dy[10];
+#pragma unroll
+                for (int j = 0; j < 2; ++j) guide_lobe_grad(y + 5 * j, t[j], pi[j], logq, wx, wy, wz, scale, dy + 5 * j);
+#pragma unroll
+                for (int i = 0; i < 5; ++i) {
+                    uint32_t hi, lo;
+                    split_bf16(live ? dy[2 * i] : 0.0f, live ? dy[2 * i + 1] : 0.0f, hi, lo);
+                    *reinterpret_cast<uint32_t *>(smem + kTfD + canon_off(row, 10 * part + 2 * i, kTcRows)) = hi;
+                    *reinterpret_cast<uint32_t *>(smem + kTfD + canon_off(row, 64 + 10 * part + 2 * i, kTcRows)) = lo;
+                }
+                if (part < 3) {  // unused outputs
+                    *reinterpret_cast<uint4 *>(smem + kTfD + canon_off(row, kGuideOut + 8 * part, kTcRows)) = make_uint4(0, 0, 0, 0);
+                    *reinterpret_cast<uint4 *>(smem + kTfD + canon_off(row, 64 + kGuideOut + 8 * part, kTcRows)) =
+                        make_uint4(0, 0, 0, 0);
+                }
             }
-        }
-        launch([&] {
-            wgrad(0, !first);
-            commit();
-        });
-        first = false;
-    }
-    allow_next();
-    finish();
-    if (!__syncthreads_or(s_failed)) {
-        // The CTA's sums: rows m < 64 of dW_l carry the high part of output m, rows
-        // 64 + m the low part. They meet in shared memory, chunks of 16 columns
-        // as [chunk][output][16], and leave as whole rows.
-        float *stage = reinterpret_cast<float *>(smem);
-        const int o = row & 63;
 #pragma unroll
-        for (int pass = 0; pass < 2; ++pass) {
-            if ((row >= 64) == (pass == 0))
-#pragma unroll 1
-                for (int l = 0; l < kLayers; ++l)
-#pragma unroll 1
-                    for (int ch = part; ch < tf_chunks(l); ch += 4) {
-                        float v[16];
-                        tmem_ld16(lane_addr + tf_dcol(l) + 16 * ch, v);
-                        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-                        float4 *q = reinterpret_cast<float4 *>(stage + ((tf_chunk0(l) + ch) * 64 + o) * kTfStage);
+            for (int l = kLayers - 1; l >= 1; --l) {
+                ready();
+                if (l == kLayers - 1) encode(0, 3);
+                else encode(1, kLayers - 2 - l);
+                finish();
+                float v[16];
+                tmem_ld16(lane_addr + 16 * part, v);
+                asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+                // the ReLU of layer l - 1 passes where its output x_l is not zero
+                unsigned char *D = smem + kTfD + ((l - 1) & 1) * 32768;
+                const __nv_bfloat162 zero2 = __floats2bfloat162_rn(0.0f, 0.0f);
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            float4 s = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-                            if (pass == 1) {
-                                const float4 low = q[i];
-                                s.x += low.x, s.y += low.y, s.z += low.z, s.w += low.w;
-                            }
-                            q[i] = s;
-                        }
+                for (int j = 0; j < 2; ++j) {
+                    const uint4 x = *reinterpret_cast<const uint4 *>(smem + xoff[l] + canon_off(row, 16 * part + 8 * j, kTcRows));
+                    const uint32_t q[4] = {x.x, x.y, x.z, x.w};
+                    uint32_t hi[4], lo[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const int i = 8 * j + 2 * k;
+                        const uint32_t pass = __hneu2_mask(*reinterpret_cast<const __nv_bfloat162 *>(&q[k]), zero2);
+                        split_bf16(v[i], v[i + 1], hi[k], lo[k]);
+                        hi[k] &= pass, lo[k] &= pass;
                     }
-            __syncthreads();
-        }
-        float *out = parts + (size_t)blockIdx.x * kPartStride;
-#pragma unroll
-        for (int l = 0; l < kLayers; ++l) {
-            const int rowv = fan_in(l) / 4;
-            for (int i = tid; i < fan_out(l) * rowv; i += kTfThreads) {
-                const int m = i / rowv, col = 4 * (i % rowv);
-                reinterpret_cast<float4 *>(out + w_off(l))[i] =
-                    *reinterpret_cast<const float4 *>(stage + ((tf_chunk0(l) + col / 16) * 64 + m) * kTfStage + col % 16);
+                    *reinterpret_cast<uint4 *>(D + canon_off(row, 16 * part + 8 * j, kTcRows)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                    *reinterpret_cast<uint4 *>(D + canon_off(row, 64 + 16 * part + 8 * j, kTcRows)) =
+                        make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                }
             }
-            if (tid < fan_out(l)) out[b_off(l) + tid] = stage[((tf_chunk0(l) + fan_in(l) / 16) * 64 + tid) * kTfStage];
+            ready();
+            encode(1, 3);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) encode(2, k);
+            finish();  // the last weight gradient reads x_0 and a delta tile
         }
-        for (int k = 16; k > 0; k >>= 1) loss_sum += __shfl_down_sync(0xffffffffu, loss_sum, k);
-        if (part == 0 && lane == 0) s_loss[warp] = loss_sum;
-        __syncthreads();
-        if (tid == 0) out[kNumParams] = (s_loss[0] + s_loss[1]) + (s_loss[2] + s_loss[3]);
-    } else {
-        // MMAs or the weight copy still in flight: wait again (bounded) before
-        // freeing their memory; the sums of this CTA count as nothing
-        mbar_wait(mbar, phase);
-        mbar_wait(cbar, 0);
-        for (int i = tid; i < kPartStride; i += kTfThreads) parts[(size_t)blockIdx.x * kPartStride + i] = 0.0f;
+        allow_next();
+        bar_sync(kTfWorkBar, kTfThreads);
+        float *out = parts + (size_t)blockIdx.x * kPartStride;
+        if (!*reinterpret_cast<volatile int *>(&s_failed)) {
+            // The CTA's sums: rows m < 64 of dW_l carry the high part of output m, rows
+            // 64 + m the low part. Both go to shared memory as [half][chunk][output][16]
+            // (chunk f: tensor-memory columns 64 + 16 f ..; layers 1 to 4 have 5 each)
+            // and leave, added, as whole rows. The 16-byte pieces are turned so that
+            // neither side has bank conflicts.
+            const int half = row >> 6, o = row & 63;
+            auto piece = [&](int h, int f, int m, int q) {
+                return reinterpret_cast<float4 *>(smem + ((h * kTfChunks + f) * 64 + (m ^ (f & 1))) * 64 + 16 * (q ^ ((m >> 1) & 3)));
+            };
+#pragma unroll 1
+            for (int f0 = part; f0 < kTfChunks; f0 += 8) {  // two at a time
+                float v[2][16];
+                tmem_ld16(lane_addr + 64 + 16 * f0, v[0]);
+                if (f0 + 4 < kTfChunks) tmem_ld16(lane_addr + 64 + 16 * (f0 + 4), v[1]);
+                asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+                for (int k = 0; k < 2; ++k)
+                    if (f0 + 4 * k < kTfChunks)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            *piece(half, f0 + 4 * k, o, i) = make_float4(v[k][4 * i], v[k][4 * i + 1], v[k][4 * i + 2], v[k][4 * i + 3]);
+            }
+            bar_sync(kTfWorkBar, kTfThreads);
+            auto sum = [&](int f, int m, int q) {
+                const float4 hi = *piece(0, f, m, q), lo = *piece(1, f, m, q);
+                return make_float4(hi.x + lo.x, hi.y + lo.y, hi.z + lo.z, hi.w + lo.w);
+            };
+#pragma unroll
+            for (int l = 0; l < kLayers; ++l) {
+                const int rowv = fan_in(l) / 4, f = ((int)tf_dcol(l) - 64) / 16;
+                for (int i = tid; i < fan_out(l) * rowv; i += kTfThreads) {
+                    const int m = i / rowv, q = i % rowv;
+                    reinterpret_cast<float4 *>(out + w_off(l))[i] = sum(f + q / 4, m, q % 4);
+                }
+                if (tid < fan_out(l)) out[b_off(l) + tid] = sum(f + fan_in(l) / 16, tid, 0).x;
+            }
+            for (int k = 16; k > 0; k >>= 1) loss_sum += __shfl_down_sync(0xffffffffu, loss_sum, k);
+            if (part == 0 && lane == 0) s_loss[warp] = loss_sum;
+            bar_sync(kTfWorkBar, kTfThreads);
+            if (tid == 0) out[kNumParams] = (s_loss[0] + s_loss[1]) + (s_loss[2] + s_loss[3]);
+        } else {
+            // MMAs or the weight copy still in flight: wait again (bounded) before
+            // freeing their memory; the sums of this CTA count as nothing
+            mbar_wait(mbar, phase);
+            mbar_wait(cbar, 0);
+            for (int i = tid; i < kPartStride; i += kTfThreads) out[i] = 0.0f;
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
@@ -1275,8 +1329,9 @@ __global__ void k_guide_add_sums(const float *sums, uint32_t count, float *sum)
 
 // Adds the nparts rows of partial sums (in a fixed order: kAdamSplits
 // interleaved sums, then those) into grad and the loss and, with `adam`, takes
-// the Adam step. 64 entries per block.
-constexpr int kAdamSplits = 8;
+// the Adam step. 64 entries per block, four per thread and load, so that a
+// block's loads are all in flight at once.
+constexpr int kAdamSplits = 32;
 struct AdamArgs {
     float *params, *m, *v;
     __nv_bfloat16 *wb;
@@ -1284,23 +1339,28 @@ struct AdamArgs {
     int t;
     float lr, b1, b2, eps;
 };
-__global__ void __launch_bounds__(64 * kAdamSplits) k_guide_adam(const float *parts, int nparts, float *grad, float *loss, bool adam, AdamArgs a)
+__global__ void __launch_bounds__(16 * kAdamSplits) k_guide_adam(const float *parts, int nparts, float *grad, float *loss, bool adam, AdamArgs a)
 {
-    __shared__ float s[kAdamSplits][64];
-    const int i = blockIdx.x * 64 + (threadIdx.x & 63), split = threadIdx.x >> 6;
-    float sum = 0.0f;
+    __shared__ float4 s[kAdamSplits][16];
+    const int quad = threadIdx.x & 15, split = threadIdx.x >> 4;
+    float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     wait_previous();
     allow_next();
-    if (i <= kNumParams) {
+    if (blockIdx.x * 64 + 4 * quad < kPartStride) {
+        const float4 *p = reinterpret_cast<const float4 *>(parts) + blockIdx.x * 16 + quad;
 #pragma unroll 8
-        for (int q = split; q < nparts; q += kAdamSplits) sum += parts[(size_t)q * kPartStride + i];
+        for (int q = split; q < nparts; q += kAdamSplits) {
+            const float4 x = p[(size_t)q * (kPartStride / 4)];
+            sum.x += x.x, sum.y += x.y, sum.z += x.z, sum.w += x.w;
+        }
     }
-    s[split][threadIdx.x & 63] = sum;
+    s[split][quad] = sum;
     __syncthreads();
-    if (split != 0 || i > kNumParams) return;
+    const int i = blockIdx.x * 64 + (int)threadIdx.x;
+    if (threadIdx.x >= 64 || i > kNumParams) return;
     float g = 0.0f;
 #pragma unroll
-    for (int q = 0; q < kAdamSplits; ++q) g += s[q][threadIdx.x];
+    for (int q = 0; q < kAdamSplits; ++q) g += reinterpret_cast<const float *>(s[q])[threadIdx.x];
     if (i == kNumParams) {
         if (loss) *loss = g;
         return;
@@ -1439,7 +1499,7 @@ dr_status run_gradients(dr_guide *g, const float *pos, const float *dir, const f
         // one CTA per SM (its shared memory and 512 tensor-memory columns)
         const unsigned tiles = (n + kTcRows - 1) / kTcRows;
         const unsigned blocks = std::min<unsigned>(tiles, (unsigned)g->ctx->num_sms);
-        DR_CUDA(launch_after(k_guide_train_fused, blocks, kTfThreads, kTfSmem, st, g->img, g->params, gp, pos, dir, sdir, weight, n,
+        DR_CUDA(launch_after(k_guide_train_fused, blocks, kTfThreads + 32, kTfSmem, st, g->img, g->params, gp, pos, dir, sdir, weight, n,
                              sums, sum_blocks, g->parts, g->ctx->d_error));
         *parts = g->parts;
         *nparts = (int)blocks;
@@ -1692,7 +1752,7 @@ dr_status dr_guide_gradients(dr_guide *g, const float *pos_dev, const float *dir
     int nparts = 0;
     dr_status r = run_gradients(g, pos_dev, dir_dev, sdir_dev, weight_dev, n, nullptr, &parts, &nparts);
     if (r != DR_OK) return r;
-    k_guide_adam<<<kAdamBlocks, 64 * kAdamSplits>>>(parts, nparts, g->grad, g->scalars + 1, false, AdamArgs{});
+    k_guide_adam<<<kAdamBlocks, 16 * kAdamSplits>>>(parts, nparts, g->grad, g->scalars + 1, false, AdamArgs{});
     DR_CUDA(cudaGetLastError());
     DR_CUDA(cudaDeviceSynchronize());
     if (loss_host) DR_CUDA(cudaMemcpy(loss_host, g->scalars + 1, 4, cudaMemcpyDeviceToHost));
@@ -1715,7 +1775,7 @@ dr_status dr_guide_train_step(dr_guide *g, const float *pos_dev, const float *di
     const float lr = g->cfg.warmup_steps && (uint32_t)g->step < g->cfg.warmup_steps
                          ? g->cfg.learning_rate * (float)g->step / (float)g->cfg.warmup_steps
                          : g->cfg.learning_rate;
-    DR_CUDA(launch_after(k_guide_adam, kAdamBlocks, 64 * kAdamSplits, 0, st, parts, nparts, (float *)nullptr, g->scalars + 1, true,
+    DR_CUDA(launch_after(k_guide_adam, kAdamBlocks, 16 * kAdamSplits, 0, st, parts, nparts, (float *)nullptr, g->scalars + 1, true,
                          AdamArgs{g->params, g->m, g->v, g->wb, g->img, g->step, lr, g->cfg.beta1, g->cfg.beta2,
                                   g->cfg.epsilon}));
     DR_CUDA(cudaGetLastError());
