@@ -267,17 +267,19 @@ __global__ void __launch_bounds__(128) k_guide_infer(const __nv_bfloat16 *wb, co
 // K-major layout without swizzle, and kInferGroups groups of 128 threads, each
 // with an input tile, 64 tensor-memory columns and an mbarrier of its own. A
 // group carries tiles of 128 rows (the M of one tcgen05.mma) through the
-// network: its first thread issues the K/16 MMAs of a layer into the 128 x N
-// FP32 accumulator and commits them to the mbarrier, and each warp reads its 32
-// rows back with tcgen05.ld for the bias / ReLU / BF16 epilogue, which writes
+// network: one lane of its first warp, elected while the warp is converged,
+// issues the K/16 MMAs of a layer into the 128 x N FP32 accumulator and commits
+// them to the mbarrier (chosen by its thread index instead, it moved every
+// operand to the uniform registers by itself: 106 against 95 us), and each warp
+// reads its 32 rows back with tcgen05.ld for the bias / ReLU / BF16 epilogue, which writes
 // the next layer's input. Groups do not wait for one another: while one is in
 // its chain of MMA, commit, tensor-memory read and barrier, the others encode
 // inputs and run epilogues. Same arithmetic as k_guide_infer (BF16 products,
-// FP32 sums). Bound by the shared / tensor memory data path (0.59 of it by loads
+// FP32 sums). Bound by the shared / tensor memory data path (0.6 of it by loads
 // and stores, the operands of the MMAs beside them) and by that chain's latency;
-// 0.52 of the issue slots, 0.26 of HBM for 2^20 rows in 108 us. The sines and cosines
-// of the inputs are 19 us of it; outputs of whole tiles leave as one bulk copy
-// (117 us when every tile's rows went through loads and stores).
+// 0.58 of the issue slots, 0.3 of HBM for 2^20 rows in 95 us. The sines and cosines
+// of the inputs are some 19 us of it; outputs of whole tiles leave as one bulk copy
+// (117 against 108 us when every tile's rows went through loads and stores).
 
 constexpr int kTcRows = 128;
 
@@ -310,6 +312,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t phase)
     return mbar_wait_bounded(mbar, phase, kMbarWaitPolls);
 }
 
+// True in one lane of a converged warp, always the same one.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t one;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+    return one != 0;
+}
+
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *v)
 {
     uint32_t r[16];
@@ -336,9 +346,9 @@ constexpr uint32_t kTcW4 = kTcW1 + 3 * 64 * 64 * 2;  // 48 x 64
 constexpr uint32_t kTcA = kTcW4 + 48 * 64 * 2;       // per group: 128 x 80 input / 128 x 64 hidden / 128 x 40 output
 constexpr uint32_t kTcABytes = kTcRows * kIn * 2;
 static_assert(kTcABytes == kTcRows * kGuideOut * 4, "the output rows fit the input tile");
-// Groups per CTA: 6 run at 80 registers (2^20 rows: 108 us), 5 at 96 (114 us),
-// 7 at 72 with spills (106 us; 200,000 rows 29.4 against 29.0 us), 8 spill at 64.
-// Three CTAs of one group each, with their own copies of the weights, took 178 us.
+// Groups per CTA: 6 run at 80 registers (2^20 rows: 95 us; 200,000 rows 23.8),
+// 5 at 96 (101; 27.0), 7 and 8 spill at 72 and 64 (94; 24.7 and 25.7). Three CTAs
+// of one group each, with their own copies of the weights, took 178 us.
 constexpr int kInferGroups = 6;
 constexpr uint32_t kTcBias = kTcA + kInferGroups * kTcABytes;
 constexpr uint32_t kTcBar = kTcBias + (4 * kHid + kOut) * 4;  // per group: MMA mbarrier; then copy mbarrier, TMEM address
@@ -389,7 +399,7 @@ k_guide_infer_tc(const unsigned char *img, const float *params, GuideParams gp, 
     constexpr int kCols = 16;  // accumulator columns an epilogue holds at once
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ int s_failed;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, group = tid >> 7, row = tid & 127;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, group = warp >> 2, row = tid & 127;
     allow_next();
     wait_previous();
     const uint32_t n = count ? *count : n_fixed;
@@ -464,22 +474,25 @@ k_guide_infer_tc(const unsigned char *img, const float *params, GuideParams gp, 
             asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
             group_sync(group);
-            if (row == 0 && ok) {
-                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                const uint32_t idesc = idesc_bf16(kTcRows, N);
-                uint64_t ad = smem_desc(a_base, kTcRows * 16, 128), bd = smem_desc(w_base, (uint32_t)N * 16, 128);
+            if ((warp & 3) == 0) {
+                if (__all_sync(0xffffffffu, ok) && elect_one()) {
+                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                    const uint32_t idesc = idesc_bf16(kTcRows, N);
+                    uint64_t ad = smem_desc(a_base, kTcRows * 16, 128), bd = smem_desc(w_base, (uint32_t)N * 16, 128);
 #pragma unroll
-                for (int s2 = 0; s2 < kIn / 16; ++s2) {
-                    if (16 * s2 >= K) break;
-                    asm volatile(
-                        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(acc),
-                        "l"(ad), "l"(bd), "r"(idesc), "r"(s2));
-                    ad += 2 * kTcRows * 16 / 16;  // the next 16 columns of both operands
-                    bd += 2 * N * 16 / 16;
+                    for (int s2 = 0; s2 < kIn / 16; ++s2) {
+                        if (16 * s2 >= K) break;
+                        asm volatile(
+                            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+                            " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(acc),
+                            "l"(ad), "l"(bd), "r"(idesc), "r"(s2));
+                        ad += 2 * kTcRows * 16 / 16;  // the next 16 columns of both operands
+                        bd += 2 * N * 16 / 16;
+                    }
+                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(mbar)
+                                 : "memory");
                 }
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(mbar)
-                             : "memory");
+                __syncwarp();
             }
             ok = wait(mbar, phase) && ok;
             phase ^= 1u;
@@ -869,14 +882,6 @@ __device__ __forceinline__ void bar_arrive(int id, int threads)
     asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
 }
 
-// True in one lane of a converged warp, always the same one.
-__device__ __forceinline__ bool elect_one()
-{
-    uint32_t one;
-    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
-    return one != 0;
-}
-
 __global__ void __launch_bounds__(kTfThreads + 32, 1)
 k_guide_train_fused(const unsigned char *img, const float *params, GuideParams gp, const float *pos, const float *dir,
                     const float *sdir, const float *weight, uint32_t n, const float *weight_parts, uint32_t nweight,
@@ -1024,8 +1029,8 @@ k_guide_train_fused(const unsigned char *img, const float *params, GuideParams g
         // Pair k of the encoded columns of chunk part + 4 j (8 columns) of a row.
         // A tile's rows are loaded a tile ahead and encoded while the products of
         // the tile before run (3,700 cycles a tile otherwise).
-        float p[3], d[3];
-        uint32_t in[3][4];
+        float p[3] = {}, d[3] = {};
+        uint32_t in[3][4] = {};
         auto encode = [&](int j, int k) {
             const int c = 8 * (part + 4 * j) + 2 * k, axis = c / 24;
             float v0 = 0.0f, v1 = 0.0f;
