@@ -166,13 +166,13 @@ __host__ __device__ inline GuideLobeTerm guide_lobe_term(const float *y, float p
 {
     GuideLobeTerm T;
     const float k = guide_exp(fminf(fmaxf(y[1], kGuideLogKMin), kGuideLogKMax));
-    const float n2 = y[2] * y[2] + y[3] * y[3] + y[4] * y[4];
+    const float n2 = fmaf(y[4], y[4], fmaf(y[2], y[2], y[3] * y[3]));  // contracted as guide_loss_grad's sum
     T.kappa = k;
     T.n = sqrtf(n2);
     const bool deg = n2 < 1e-24f;
     const float r = 1.0f / T.n;
     T.mx = deg ? 0.0f : y[2] * r, T.my = deg ? 0.0f : y[3] * r, T.mz = deg ? 1.0f : y[4] * r;
-    T.cosang = T.mx * wx + T.my * wy + T.mz * wz;
+    T.cosang = fmaf(T.mz, wz, fmaf(T.mx, wx, T.my * wy));
     // kappa >= e^-4: 1 - e^{-2 kappa} needs no series
     const float lognorm = logf(k) - 1.83787706641f - log1pf(-guide_exp(-2.0f * k));
     T.t = logf(pi) + lognorm + k * (T.cosang - 1.0f);
