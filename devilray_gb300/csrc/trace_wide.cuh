@@ -58,14 +58,14 @@ constexpr int kWideStack = 64;
 #ifndef DR_PACKED_SLAB
 #define DR_PACKED_SLAB 0
 #endif
-// Grid planes through FP16 in the closest-hit traversal of the persistent
-// kernels: one byte permute places bytes j and j + 2 of a plane word under
+// Grid planes through FP16 in the persistent kernels: one byte permute places bytes j and j + 2 of a plane word under
 // FP16 exponent bits (1024 + q, exact), two conversions (cvt.f32.f16) make
 // them FP32, so half of the extraction leaves the ALU pipe (the busiest: 69 %
 // of cycles) for the FMA pipe; the slab constants fold 1024 instead of 2^15
 // (slab_axis_h). Measured on the incoherent workload (2^20 triangles, 16.8 M
-// rays): closest hit 3.334 -> 3.269 ms; any hit 2.843 -> 2.915 ms, so any-hit
-// traversal keeps the byte permutes.
+// rays): closest hit 3.334 -> 3.269 ms; any hit, watertight test, 2.62 -> 2.40 ms
+// (4 M segments of 300,000 triangles 531 -> 490 us), reference test within 0.4 %
+// (2.28 ms; 1 M segments of 5,000 triangles 78 -> 74 us).
 #ifndef DR_HALF_CVT
 #define DR_HALF_CVT 1
 #endif
@@ -104,19 +104,10 @@ constexpr int kWideStack = 64;
 #ifndef DR_NO_OCT_ORDER
 #define DR_NO_OCT_ORDER 0
 #endif
-// The internal hit mask moved from slot to traversal order (bit s -> bit
-// s ^ oct) by one lookup in a 2 KB shared-memory table per block
-// instead of three conditional swaps, in the persistent kernels: 1 all of
-// them, 2 the any-hit ones. Measured on the incoherent workload: any hit
-// 2.842 -> 2.791 ms with the table; closest hit 3.192 -> 3.307 ms, and
-// 3.275 / 3.285 ms with 6 / 4 shared stack entries, which give back the L1
-// the table takes (with the table the closest-hit kernel spills 26 bytes at
-// its 72 registers). So only the any-hit kernels use it (many-light 1080p
-// render, 16 spp: 40.46-40.55 -> 40.40-40.43 ms).
-#ifndef DR_OCT_LUT
-#define DR_OCT_LUT 2
-#endif
-// (Measured and dropped, same workload: the children in slot order instead of
+// (Measured and dropped, same workload: the internal hit mask moved to traversal
+// order by a lookup in a 2 KB shared-memory table instead of three conditional
+// swaps, closest hit 3.19 -> 3.31 ms, any hit with FP16 planes 491 -> 503 us for
+// 4 M segments; the children in slot order instead of
 // the ray's octant order, 3.19 -> 3.71 ms; 128-byte nodes that store the
 // grid planes as FP16 words, so that no byte permute or near/far select is
 // left, 3.96 ms: the node loads cost more than the instructions saved.)
@@ -274,11 +265,10 @@ __device__ __forceinline__ float2 byte_pair_h(uint32_t w, uint32_t j)
 // Tests the 8 child boxes of `node` against [0, tmax]; returns the internal
 // hit mask in traversal order (bit k = slot k ^ oct) and the triangle mask.
 // HALF: grid planes through FP16 (DR_HALF_CVT).
-template <bool HALF = false, bool LUT = false>
+template <bool HALF = false>
 __host__ __device__ __forceinline__ void wide_node_test(const Bvh8Node *node, const DevRay &r, uint32_t oct, float tmax,
                                                         uint32_t &child_base, uint32_t &imask, uint32_t &hit_internal,
-                                                        uint32_t &tri_base, uint32_t &tri_mask, uint32_t &nboxes,
-                                                        const uint8_t *oct_lut = nullptr)
+                                                        uint32_t &tri_base, uint32_t &tri_mask, uint32_t &nboxes)
 {
     const uint4 w0 = DR_LD(&node->w[0]);
     const uint4 w1 = DR_LD(&node->w[1]);
@@ -489,13 +479,9 @@ __host__ __device__ __forceinline__ void wide_node_test(const Bvh8Node *node, co
 #endif
     // internal hits from slot order to traversal order: bit s -> bit s ^ oct
 #if !DR_NO_OCT_ORDER
-    if (LUT) {
-        m = oct_lut[(oct << 8) | m];
-    } else {
-        if (oct & 1u) m = ((m & 0x55u) << 1) | ((m >> 1) & 0x55u);
-        if (oct & 2u) m = ((m & 0x33u) << 2) | ((m >> 2) & 0x33u);
-        if (oct & 4u) m = ((m & 0x0fu) << 4) | ((m >> 4) & 0x0fu);
-    }
+    if (oct & 1u) m = ((m & 0x55u) << 1) | ((m >> 1) & 0x55u);
+    if (oct & 2u) m = ((m & 0x33u) << 2) | ((m >> 2) & 0x33u);
+    if (oct & 4u) m = ((m & 0x0fu) << 4) | ((m >> 4) & 0x0fu);
 #endif
     hit_internal = m;
 #endif
@@ -548,13 +534,13 @@ constexpr uint32_t kTriGroupFlag = 0x80000000u;
 
 // Node test of the persistent kernels: the node's internal hits become the
 // current group, its hit leaf triangles the pending triangle group.
-template <int MODE, bool HALF = false, bool LUT = false>
+template <int MODE, bool HALF = false>
 __device__ __forceinline__ void wide_visit(const Wide8Args &a, WideState &s, unsigned long long &nn,
-                                           unsigned long long &nb, const uint8_t *oct_lut = nullptr)
+                                           unsigned long long &nb)
 {
     uint32_t child_base, imask, hit_int, nbx, tri_base, tri_mask;
-    wide_node_test<HALF, LUT>(a.nodes + s.node, s.r, s.oct, s.best_t, child_base, imask, hit_int, tri_base, tri_mask,
-                              nbx, oct_lut);
+    wide_node_test<HALF>(a.nodes + s.node, s.r, s.oct, s.best_t, child_base, imask, hit_int, tri_base, tri_mask,
+                         nbx);
     ++nn;
     nb += nbx;
     s.group = make_uint2(child_base, (hit_int << 8) | imask);
