@@ -925,16 +925,16 @@ k_guide_train_fused(const unsigned char *img, const float *params, GuideParams g
     const uint32_t taddr = *reinterpret_cast<volatile uint32_t *>(smem + kTfBar + 8);
     const uint32_t d_base = smem_u32(smem + kTfD), w_img = smem_u32(smem + kTfW), x_base = smem_u32(smem);
     const uint32_t woff[kLayers] = {kTcW0, kTcW1, kTcW1 + 8192, kTcW1 + 16384, kTcW4};
-    if (!mbar_wait(cbar, 0)) {  // the weights have landed
-        *reinterpret_cast<volatile int *>(&s_failed) = 1;
-        atomicOr(error, ERR_TIMEOUT);
-    }
 
     if (!worker) {
         // The products of every step, by one lane of a warp of their own: in a
         // worker's warp their issue (up to 1,000 cycles a step, as the tensor
         // pipe takes them) would keep that warp's rows waiting.
         const bool leader = elect_one();
+        if (!mbar_wait(cbar, 0)) {  // the weights have landed
+            *reinterpret_cast<volatile int *>(&s_failed) = 1;
+            atomicOr(error, ERR_TIMEOUT);
+        }
         auto ready = [&] {
             bar_sync(kTfReadyBar, kTfThreads + 32);
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -996,11 +996,8 @@ k_guide_train_fused(const unsigned char *img, const float *params, GuideParams g
         allow_next();
     } else {
         const uint32_t lane_addr = taddr + ((uint32_t)(32 * (warp & 3)) << 16);
-        // mean sample weight: the same sum in every thread of every block
         float wsum = (uint32_t)lane < nweight ? weight_parts[lane] : 0.0f;
-        if ((uint32_t)lane + 32 < nweight) wsum += weight_parts[lane + 32];
-        for (int o = 16; o > 0; o >>= 1) wsum += __shfl_xor_sync(0xffffffffu, wsum, o);
-        const float wmean = wsum / (float)n;
+        const float wsum2 = (uint32_t)lane + 32 < nweight ? weight_parts[lane + 32] : 0.0f;
         float loss_sum = 0.0f;  // of the part 0 threads' rows
         uint32_t phase = 0;
         bool failed = false;  // warp-uniform
@@ -1050,6 +1047,10 @@ k_guide_train_fused(const unsigned char *img, const float *params, GuideParams g
 #pragma unroll
             for (int i = 0; i < 12; ++i) encode(i / 4, i % 4);
         }
+        // mean sample weight: the same sum in every thread of every block
+        wsum += wsum2;
+        for (int o = 16; o > 0; o >>= 1) wsum += __shfl_xor_sync(0xffffffffu, wsum, o);
+        const float wmean = wsum / (float)n;
         for (; (uint64_t)tile * kTcRows < n; tile += gridDim.x) {
             const uint32_t r = tile * kTcRows + row;
             const bool live = r < n;
@@ -1384,10 +1385,12 @@ __global__ void __launch_bounds__(16 * kAdamSplits) k_guide_adam(const float *pa
         if (i >= w_off(l) && i < b_off(l)) store_weight(a.wb, a.img, l, i - w_off(l), p);
 }
 
-__global__ void k_guide_export(const float *params, __nv_bfloat16 *wb, unsigned char *img)
+// The BF16 copies of the parameters; clears the Adam moments unless m is NULL.
+__global__ void k_guide_export(const float *params, __nv_bfloat16 *wb, unsigned char *img, float *m, float *v)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= kNumParams) return;
+    if (m) m[i] = v[i] = 0.0f;
     for (int l = 0; l < kLayers; ++l)
         if (i >= w_off(l) && i < b_off(l)) store_weight(wb, img, l, i - w_off(l), params[i]);
 }
@@ -1665,10 +1668,8 @@ dr_status dr_guide_set_params(dr_guide *g, const float *host, uint32_t n)
     DR_CHECK_ARG(g && host && n == (uint32_t)kNumParams, "dr_guide_set_params: bad argument");
     DR_CUDA(cudaSetDevice(g->ctx->device));
     DR_CUDA(cudaMemcpy(g->params, host, kNumParams * 4, cudaMemcpyHostToDevice));
-    DR_CUDA(cudaMemset(g->m, 0, kNumParams * 4));
-    DR_CUDA(cudaMemset(g->v, 0, kNumParams * 4));
     g->step = 0;
-    k_guide_export<<<(kNumParams + 255) / 256, 256>>>(g->params, g->wb, g->img);
+    k_guide_export<<<(kNumParams + 255) / 256, 256>>>(g->params, g->wb, g->img, g->m, g->v);
     DR_CUDA(cudaGetLastError());
     DR_CUDA(cudaDeviceSynchronize());
     return DR_OK;
@@ -1724,7 +1725,7 @@ dr_status dr_guide_set_state(dr_guide *g, const void *host, uint64_t bytes)
     DR_CUDA(cudaMemcpy(g->v, f + 2 * kNumParams, kNumParams * 4, cudaMemcpyHostToDevice));
     g->cfg = h.cfg;
     g->step = (int)h.step;
-    k_guide_export<<<(kNumParams + 255) / 256, 256>>>(g->params, g->wb, g->img);
+    k_guide_export<<<(kNumParams + 255) / 256, 256>>>(g->params, g->wb, g->img, nullptr, nullptr);
     DR_CUDA(cudaGetLastError());
     DR_CUDA(cudaDeviceSynchronize());
     return DR_OK;
