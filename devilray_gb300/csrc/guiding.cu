@@ -4,8 +4,10 @@
 // Network: 80 inputs (12-frequency encoding of the normalised position, a
 // direction, zero padding) -> 4 hidden layers of 64 (ReLU) -> 48 outputs (40
 // used: the 8-lobe vMF mixture of guide_math.cuh). Weights and layer inputs
-// are BF16, every product accumulates in FP32 (mma.sync m16n8k16 on the
-// tensor cores); master weights and Adam moments are FP32.
+// are BF16, every product accumulates in FP32; master weights and Adam moments
+// are FP32. Inference and training run on the 5th-generation tensor cores
+// (k_guide_infer_tc, k_guide_train_fused); the kernels with warp-level mma.sync
+// m16n8k16 are their alternatives and work as follows.
 //
 // A warp carries 16 rows through all layers in registers: the FP32
 // accumulator fragment of one layer is, pair by pair, the BF16 A fragment of

@@ -4,9 +4,12 @@
 // 22-102, include/tracing/PathGeneration.hpp:363-515): one thread per pixel
 // that builds a whole path, then shades it, becomes a wave of kernels over a
 // batch of path slots:
-//   camera -> for each bounce: closest hit -> shade (emission with MIS, a light
+//   camera -> for each bounce: closest hit, and any hit of the bounce before's
+//   shadow rays (+ next-event contribution) -> shade (emission with MIS, a light
 //   sample, the BSDF sample; compaction of surviving paths and of shadow rays by
-//   warp ballot) -> shadow any hit (+ next-event contribution) -> accumulate.
+//   warp ballot) -> accumulate.
+// Small waves, and the last paths of large ones, are carried to their ends by one
+// kernel (k_wave_paths).
 // The shading restates the reference's arithmetic in a forward order that adds
 // the same terms in the same sequence (emission of vertex k, then its light
 // sample, then vertex k+1), so each sample's colour is bit-identical to the
