@@ -67,14 +67,21 @@ constexpr int kShadeMinBlocks = DR_SHADE_MIN_BLOCKS;
 // time by bounces / in one kernel: 65,536 (box room) 696 / 464 us; 129,600
 // (2^17-triangle many-light) 853 / 490 us; 163,840 (box room) 950 / 872 us;
 // 262,144 (box room) 1,030 / 1,111 us. Larger waves hand over when at most
-// kTailPathsPerSm paths per SM (32,832) are left at bounce 2, 4, 8, 16 or 32: a
-// check that does not take over costs an empty launch (2 us). Limits of 16,384 /
+// kTailPathsPerSm paths per SM (32,832) are left (tail_check). Limits of 16,384 /
 // 32,768 / 65,536 paths: many-light 2^16 triangles 512x512, 4 spp 1,439 / 1,359 /
 // 1,367 us (1,716 without), eight uneven scenes 967 / 969 / 969 us (1,286); a
 // limit of 131,072 makes the 1080p many-light image slower (10.0 -> 12.7 ms), where
 // the longest walks of a 2^20-triangle scene want more rays in flight.
 constexpr uint32_t kWholePathsPerSm = 1024, kTailPathsPerSm = 216;
-constexpr bool tail_check(int b) { return b >= 2 && (b & (b - 1)) == 0; }
+// Looked at before bounces 2, 3, 4, 6, 8, 12, ..: a look that finds too many paths
+// costs 3 us, one that comes a bounce late some 60. Eight uneven scenes, 4 spp,
+// 885 us with powers of two only, 858 us; 860 us before every bounce, which costs
+// images that keep their paths up to 1 %.
+constexpr bool tail_check(int b)
+{
+    const int odd = b % 3 == 0 ? b / 3 : b;
+    return b >= 2 && (odd & (odd - 1)) == 0;
+}
 
 struct RenderParams {
     TraceArgs trace;
