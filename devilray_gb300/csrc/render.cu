@@ -64,8 +64,8 @@ constexpr int kShadeMinBlocks = DR_SHADE_MIN_BLOCKS;
 
 // Where k_wave_paths takes over. Waves of up to kWholePathsPerSm paths per SM
 // (155,648 on 152 SMs) run in it from the camera rays on; paths per wave and
-// time by bounces / in one kernel: 65,536 (box room) 696 / 464 us; 129,600
-// (2^17-triangle many-light) 853 / 490 us; 163,840 (box room) 950 / 872 us;
+// time by bounces / in one kernel: 65,536 (box room) 696 / 464 us (415 now); 129,600
+// (2^17-triangle many-light) 853 / 490 us (447 now); 163,840 (box room) 950 / 872 us;
 // 262,144 (box room) 1,030 / 1,111 us. Larger waves hand over when at most
 // kTailPathsPerSm paths per SM (32,832) are left (tail_check). Limits of 16,384 /
 // 32,768 / 65,536 paths: many-light 2^16 triangles 512x512, 4 spp 1,439 / 1,359 /
