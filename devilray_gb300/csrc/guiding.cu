@@ -1314,7 +1314,13 @@ __global__ void __launch_bounds__(256) k_guide_weight_sum(const float *w, uint32
     float v = 0.0f;
     wait_previous();  // the sums' last reader, and whatever wrote the weights
     allow_next();
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) v += w[i];
+    const uint32_t stride = gridDim.x * blockDim.x;
+    uint64_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    for (; i + 3 * stride < n; i += 4 * stride) {  // four loads in flight, added in order
+        const float a = w[i], b = w[i + stride], c = w[i + 2 * stride], d = w[i + 3 * stride];
+        v += a, v += b, v += c, v += d;
+    }
+    for (; i < n; i += stride) v += w[i];
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
     __syncthreads();
