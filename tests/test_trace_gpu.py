@@ -145,6 +145,30 @@ def test_grazing_rays_match_brute_force(native, ctx, oracle, layout, mode):
     assert np.array_equal(occ.astype(bool), pb >= 0)
 
 
+@pytest.mark.parametrize("layout,scale", [(2, 1.0), (8, 1.0), (8, 2.0 ** 28)])
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("n", [4000, 70000])
+def test_directions_whose_reciprocal_is_subnormal(native, ctx, oracle, mode, layout, scale, n):
+    """Direction components above 2^126 (finite, so the ray is valid) have a
+    subnormal reciprocal, which the box tests must keep: the hits are the
+    brute-force ones, near the origin and at coordinates of 2^32."""
+    half = scenes.density_half(1000)
+    soup, _, _ = scenes.incoherent_soup(1000, seed=31, half=half)
+    rays = scenes.incoherent_rays(n, seed=32, half=half)
+    soup = soup * np.float32(scale)
+    rays[:, 0:3] *= np.float32(scale)
+    rays[:, 4:7] *= np.float32(3e38)
+    assert (np.abs(rays[:, 4:7]) > 2.0 ** 126).any(1).mean() > 0.9
+    scene = native.Scene(ctx, soup, layout=layout)
+    tb, pb = oracle.trace_brute(soup, rays, tri_mode=mode)
+    assert (pb >= 0).sum() > 20
+    t, prim, _ = gpu_closest(native, scene, rays, mode)
+    bad = np.flatnonzero((_bits(t) != _bits(tb)) | (prim != pb))
+    assert bad.size == 0, f"{bad.size} of {int((pb >= 0).sum())} hits differ, e.g. {prim[bad[:5]]} for {pb[bad[:5]]}"
+    assert np.array_equal(gpu_any(native, scene, rays, mode).astype(bool), pb >= 0)
+    ctx.check()
+
+
 @pytest.mark.parametrize("layout", [2, 8])
 def test_edge_cases(native, ctx, oracle, layout):
     unit = np.array([[0, 0, 0, 1, 0, 0, 0, 1, 0]], np.float32)
