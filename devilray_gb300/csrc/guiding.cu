@@ -383,12 +383,11 @@ __device__ __forceinline__ void fetch_weight_image(uint32_t dst, const unsigned 
                  : "memory");
 }
 
-// BF16 pair (lo, hi) of max(x, 0), as the layers' inputs are rounded.
+// BF16 pair (lo, hi) of max(x, 0), as the layers' inputs are rounded; 0 for a NaN.
 __device__ __forceinline__ uint32_t relu_bf16(float lo, float hi)
 {
-    uint32_t d;
-    asm("cvt.rn.relu.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
-    return d;
+    const __nv_bfloat162 v = __hmax2(__floats2bfloat162_rn(lo, hi), __floats2bfloat162_rn(0.0f, 0.0f));
+    return *reinterpret_cast<const uint32_t *>(&v);
 }
 
 __device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %0, 128;\n" ::"r"(group + 1) : "memory"); }

@@ -128,3 +128,33 @@ def test_tcgen05_training_at_tile_edges(native, ctx, n):
     # the step uses the same sums: one Adam step from the same parameters agrees
     tc.train_step(pos, nrm, sdir, w, n)
     assert tc.last_loss() == l_tc
+
+
+@pytest.mark.parametrize("n", [5, 300])
+def test_rows_of_non_finite_directions_stay_finite(native, ctx, n):
+    """The ReLU takes a NaN to 0, in both kernels: a row whose direction is not
+    finite gives the outputs of a network whose hidden layers are 0 (here the
+    output biases, as the hidden ones are 0), and leaves its neighbours alone."""
+    rng = np.random.default_rng(n)
+    pos = torch.from_numpy(rng.uniform(-10, 10, (n, 3)).astype(np.float32)).cuda()
+    d = rng.normal(size=(n, 3))
+    d = (d / np.linalg.norm(d, axis=1, keepdims=True)).astype(np.float32)
+    bad = np.arange(0, n, 4)
+    odd = d.copy()
+    odd[bad, rng.integers(0, 3, len(bad))] = np.nan
+    out = {}
+    for kernel in (0, 1):
+        g = native.Guide(ctx, seed=9, half_extent=10.0, infer_kernel=kernel)
+        p = g.params()
+        bias = rng.normal(0, 0.3, 48).astype(np.float32) if kernel == 0 else bias
+        p[-48:] = bias
+        g.set_params(p)
+        for name, rows in (("good", d), ("odd", odd)):
+            y = torch.full((n, 40), float("nan"), dtype=torch.float32, device="cuda")
+            g.infer(pos, torch.from_numpy(rows).cuda(), n, y)
+            out[kernel, name] = y.cpu().numpy()
+    ctx.check()
+    keep = np.setdiff1d(np.arange(n), bad)
+    for kernel in (0, 1):
+        assert np.array_equal(out[kernel, "odd"][bad], np.broadcast_to(bias[:40], (len(bad), 40)))
+        assert np.array_equal(out[kernel, "odd"][keep], out[kernel, "good"][keep])
