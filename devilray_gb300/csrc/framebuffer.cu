@@ -244,7 +244,8 @@ dr_status dr_tonemap(const float *accum_dev, int32_t width, int32_t height, int3
     DR_CHECK_ARG(accum_dev && rgba_dev && width > 0 && height > 0, "dr_tonemap: bad argument");
     DR_CHECK_ARG(height <= 65535 && (uint64_t)width * (uint64_t)height < (1ull << 31), "dr_tonemap: image too large");
     DR_CHECK_ARG(((uintptr_t)accum_dev & 15) == 0, "dr_tonemap: accum_dev must be 16-byte aligned");
-    const dim3 grid((width + 128 * kPixels - 1) / (128 * kPixels), height);
+    // (unsigned: widths up to 2^31 - 1 are accepted)
+    const dim3 grid(((unsigned)width + 128 * kPixels - 1) / (128 * kPixels), height);
     const auto st = static_cast<cudaStream_t>(stream);
     const auto *accum = reinterpret_cast<const float4 *>(accum_dev);
     if (gamma_corrected) k_tonemap<true><<<grid, 128, 0, st>>>(accum, width, height, rgba_dev);

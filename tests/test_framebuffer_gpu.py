@@ -154,3 +154,22 @@ def test_tonemap_bytes_at_every_step(native, ctx, spp):
     got = out.cpu().numpy().view(np.uint32)
     bad = np.flatnonzero(got != want)
     assert bad.size == 0, f"{bad.size} of {len(r)} differ, e.g. {r[bad[:4]]}: {got[bad[:4]]} vs {want[bad[:4]]}"
+
+
+def test_tonemap_of_the_widest_image(native, ctx):
+    """One row of nearly 2^31 pixels: the launch covers every width that the
+    argument check lets through."""
+    w = 2 ** 31 - 200
+    if torch.cuda.mem_get_info()[0] < 60 << 30:
+        pytest.skip("needs 43 GB of device memory")
+    acc = torch.zeros((w, 4), dtype=torch.float32, device="cuda")
+    ends = torch.tensor([0, 1, 255, 256, w - 2, w - 1], device="cuda")
+    acc[ends] = 1.0
+    out = torch.zeros(w, dtype=torch.int32, device="cuda")
+    native.tonemap(acc, w, 1, out)
+    torch.cuda.synchronize()
+    assert bool((out[ends] == -1).all())
+    out[ends] = -(1 << 24)
+    assert int((out != -(1 << 24)).sum()) == 0
+    del acc, out
+    torch.cuda.empty_cache()
