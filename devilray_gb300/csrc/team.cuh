@@ -11,6 +11,7 @@
 // slab times are the same FMAs on the same values), so hits are identical.
 #pragma once
 
+#include "team_stack.cuh"
 #include "trace_kernels.cuh"
 #include "trace_wide.cuh"
 
@@ -212,38 +213,12 @@ __device__ __forceinline__ void team_wide(const Wide8Args &a, const Source &src,
                 }
             }
         }
-        // 3. the next node: the nearest child hit, else from the stack
-        __syncwarp();
-        if (active && !done) {
-            uint32_t base = child_base, im = imask;
-            if (hits == 0) {
-                if (sp == 0) {
-                    done = true;
-                } else {
-                    --sp;
-                    const uint2 e = sp < DEPTH ? stack[sp] : over[sp - DEPTH];
-                    base = e.x;
-                    im = e.y & 0xffu;
-                    hits = e.y >> 8;
-                }
-            }
-            if (!done) {
-                const uint32_t slot = (uint32_t)(__ffs(hits) - 1) ^ oct;
-                const uint32_t rest = hits & (hits - 1u);
-                node = base + (uint32_t)__popc(im & ((1u << slot) - 1u));
-                if (rest) {
-                    if ((uint32_t)sp >= a.stack_limit) {
-                        if (sub == 0) atomicOr(a.error, ERR_STACK_OVERFLOW);
-                        done = true;
-                    } else {
-                        const uint2 e = make_uint2(base, (rest << 8) | im);
-                        if (sp >= DEPTH) over[sp - DEPTH] = e;
-                        else if (sub == 0) stack[sp] = e;
-                        ++sp;
-                    }
-                }
-            }
-        }
+        // 3. the next node, in octant order
+        bool full = false;
+        const bool end = team_next_node<DEPTH>(active && !done, sub == 0, oct, child_base, imask, hits, stack, over, a.stack_limit, sp,
+                                               node, full, [] { __syncwarp(); });
+        done = done || end;
+        if (full && sub == 0) atomicOr(a.error, ERR_STACK_OVERFLOW);
         if (active && done) {
             if (sub == 0) {
                 if (any) src.any(idx, found);

@@ -10,6 +10,7 @@
 // smaller triangle index), so the result equals a brute-force scan.
 #pragma once
 
+#include "bits.cuh"
 #include "dr_internal.h"
 #include "tri_device.cuh"
 
@@ -182,24 +183,6 @@ __host__ __device__ __forceinline__ float bits_f(uint32_t u)
     float f;
     memcpy(&f, &u, 4);
     return f;
-}
-
-__host__ __device__ __forceinline__ int lowest_bit(uint32_t m)
-{
-#if defined(__CUDA_ARCH__)
-    return __ffs(m) - 1;
-#else
-    return __builtin_ctz(m);
-#endif
-}
-
-__host__ __device__ __forceinline__ int popcount(uint32_t m)
-{
-#if defined(__CUDA_ARCH__)
-    return __popc(m);
-#else
-    return __builtin_popcount(m);
-#endif
 }
 
 __host__ __device__ __forceinline__ uint32_t nonzero_bytes(uint32_t x)
