@@ -309,9 +309,21 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N)
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // Bounded wait on an mbarrier phase; false after the iteration limit.
-__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t phase)
+__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t phase, uint32_t polls = kMbarWaitPolls)
 {
-    return mbar_wait_bounded(mbar, phase, kMbarWaitPolls);
+    return mbar_wait_bounded(mbar, phase, polls);
+}
+
+__device__ __forceinline__ void mbar_init(uint32_t mbar, uint32_t arrivals)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(mbar), "r"(arrivals) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+}
+
+// Arrives on `mbar` once every product that this thread has issued is complete.
+__device__ __forceinline__ void commit_products(uint32_t mbar)
+{
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(mbar) : "memory");
 }
 
 // True in one lane of a converged warp, always the same one.
@@ -353,8 +365,8 @@ static_assert(kTcABytes == kTcRows * kGuideOut * 4, "the output rows fit the inp
 // of one group each, with their own copies of the weights, took 178 us.
 constexpr int kInferGroups = 6;
 constexpr uint32_t kTcBias = kTcA + kInferGroups * kTcABytes;
-constexpr uint32_t kTcBar = kTcBias + (4 * kHid + kOut) * 4;  // per group: MMA mbarrier; then copy mbarrier, TMEM address
-constexpr uint32_t kTcSmem = kTcBar + 8 * (kInferGroups + 2);
+constexpr uint32_t kTcBar = kTcBias + (4 * kHid + kOut) * 4;  // MMA mbarrier of each group, copy mbarrier, TMEM address, drain mbarrier
+constexpr uint32_t kTcSmem = kTcBar + 8 * (kInferGroups + 3);
 
 // The weights as the tcgen05 kernels hold them in shared memory, kept in
 // global memory beside the BF16 copy so a CTA fetches them with one bulk
@@ -375,8 +387,7 @@ __device__ __forceinline__ void store_weight(__nv_bfloat16 *wb, unsigned char *i
 // memory, completing on the mbarrier `cbar` (issued by one thread).
 __device__ __forceinline__ void fetch_weight_image(uint32_t dst, const unsigned char *img, uint32_t bytes, uint32_t cbar)
 {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(cbar) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    mbar_init(cbar, 1);
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(cbar), "r"(bytes) : "memory");
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst),
                  "l"(img), "r"(bytes), "r"(cbar)
@@ -395,7 +406,7 @@ __device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %
 template <bool DECODED>
 __global__ void __launch_bounds__(128 * kInferGroups, 1)
 k_guide_infer_tc(const unsigned char *img, const float *params, GuideParams gp, const float *pos, const float *dir,
-                 const uint32_t *list, const uint32_t *count, uint32_t n_fixed, float *y, uint32_t *error)
+                 const uint32_t *list, const uint32_t *count, uint32_t n_fixed, float *y, uint32_t polls, uint32_t *error)
 {
     constexpr int kCols = 16;  // accumulator columns an epilogue holds at once
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -408,15 +419,13 @@ k_guide_infer_tc(const unsigned char *img, const float *params, GuideParams gp, 
     // weights in the canonical layout (B operands: N = outputs, K = inputs):
     // the weight image, one bulk copy
     const uint32_t cbar = smem_u32(smem + kTcBar + 8 * kInferGroups);
-    const uint32_t tslot = cbar + 8, mbar = smem_u32(smem + kTcBar) + 8 * group;
+    const uint32_t tslot = cbar + 8, dbar = cbar + 16, mbar = smem_u32(smem + kTcBar) + 8 * group;
     if (tid == 0) {
         s_failed = 0;
+        mbar_init(dbar, kInferGroups);
         fetch_weight_image(smem_u32(smem + kTcW0), img, kImgBytes, cbar);
     }
-    if (row == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(mbar) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    }
+    if (row == 0) mbar_init(mbar, 1);
     float *bias = reinterpret_cast<float *>(smem + kTcBias);
     for (int i = tid; i < 4 * kHid + kOut; i += blockDim.x) bias[i] = params[b_off(i / kHid) + i % kHid];
     if (warp == 0) {
@@ -434,14 +443,14 @@ k_guide_infer_tc(const unsigned char *img, const float *params, GuideParams gp, 
     // Every wait is bounded. A thread whose wait gives up (or that sees the
     // block's flag) goes on through its group's barriers without working, so the
     // block ends together.
-    auto wait = [&](uint32_t bar, uint32_t ph) {
+    auto wait = [&](uint32_t bar, uint32_t ph, uint32_t limit) {
         if (*reinterpret_cast<volatile int *>(&s_failed)) return false;
-        if (mbar_wait(bar, ph)) return true;
+        if (mbar_wait(bar, ph, limit)) return true;
         *reinterpret_cast<volatile int *>(&s_failed) = 1;
         atomicOr(error, ERR_TIMEOUT);
         return false;
     };
-    bool ok = wait(cbar, 0);  // the weights have landed
+    bool ok = wait(cbar, 0, kMbarWaitPolls);  // the weights have landed
     // tiles go to the blocks first, then to the groups of each block
     for (uint32_t tile = blockIdx.x + gridDim.x * group; (uint64_t)tile * kTcRows < n; tile += gridDim.x * kInferGroups) {
         const uint32_t r = tile * kTcRows + row;
@@ -490,12 +499,11 @@ k_guide_infer_tc(const unsigned char *img, const float *params, GuideParams gp, 
                         ad += 2 * kTcRows * 16 / 16;  // the next 16 columns of both operands
                         bd += 2 * N * 16 / 16;
                     }
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(mbar)
-                                 : "memory");
+                    commit_products(mbar);
                 }
                 __syncwarp();
             }
-            ok = wait(mbar, phase) && ok;
+            ok = wait(mbar, phase, polls) && ok;
             phase ^= 1u;
             w_base += (uint32_t)(K * N * 2);
             __syncwarp();
@@ -603,13 +611,20 @@ float o[kGuideOut];
         }
         group_sync(group);  // the staged rows are read before the next tile's inputs replace them
     }
-    if (!ok) {
-        // MMAs or the weight copy still in flight: wait again (bounded) before freeing their memory
-        mbar_wait(mbar, phase ^ 1u);
-        mbar_wait(cbar, 0);
-    }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
+    // After a wait gave up, products or the weight copy may still be in flight:
+    // wait (bounded) before their memory is freed. The lane that issued a group's
+    // products commits them all to a barrier of its own: the parity of the
+    // group's last commit depends on where the wait gave up.
+    if (*reinterpret_cast<volatile int *>(&s_failed)) {
+        if ((warp & 3) == 0 && elect_one()) commit_products(dbar);
+        if (warp == 0) {
+            mbar_wait(dbar, 0);
+            mbar_wait(cbar, 0);
+        }
+        __syncthreads();
+    }
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;\n" ::"r"(taddr) : "memory");
 }
 
@@ -844,8 +859,8 @@ constexpr uint32_t kTfD = kTfX1 + 4 * 10 * 2048;               // two tiles [del
 constexpr uint32_t kTfW = kTfD + 2 * 16 * 2048;                // forward weights, as kTcW0..kTcW4
 constexpr uint32_t kTfBias = kTfW + kImgBytes;
 constexpr uint32_t kTfLse = kTfBias + (4 * kHid + kOut) * 4;   // [part][row] log densities of two lobes
-constexpr uint32_t kTfBar = kTfLse + 4 * kTcRows * 8;          // MMA mbarrier, TMEM address, copy mbarrier
-constexpr uint32_t kTfSmem = kTfBar + 24;
+constexpr uint32_t kTfBar = kTfLse + 4 * kTcRows * 8;          // MMA mbarrier, TMEM address, copy mbarrier, drain mbarrier
+constexpr uint32_t kTfSmem = kTfBar + 32;
 // tensor-memory columns: [0, 64) the forward / backward product, then dW_l
 __host__ __device__ constexpr uint32_t tf_dcol(int l) { return l == 0 ? 64u : 160u + 80u * (uint32_t)(l - 1); }
 // 16-column chunks of the dW_l (weights and the bias column), in order of their columns
@@ -875,8 +890,8 @@ __device__ __forceinline__ void split_bf16(float c0, float c1, uint32_t &hi, uin
 
 // Named barriers of k_guide_train_fused (0 is __syncthreads).
 constexpr int kTfRowBar = 1;    // + row group: the four threads of each of 32 rows
-constexpr int kTfReadyBar = 5;  // the operands of the next products are in shared memory
-constexpr int kTfWorkBar = 6;   // all workers
+constexpr int kTfReadyBar = 5;  // + step & 1: the operands of the step's products are in shared memory
+constexpr int kTfWorkBar = 7;   // all workers
 __device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory"); }
 __device__ __forceinline__ void bar_arrive(int id, int threads)
 {
@@ -886,7 +901,7 @@ __device__ __forceinline__ void bar_arrive(int id, int threads)
 __global__ void __launch_bounds__(kTfThreads + 32, 1)
 k_guide_train_fused(const unsigned char *img, const float *params, GuideParams gp, const float *pos, const float *dir,
                     const float *sdir, const float *weight, uint32_t n, const float *weight_parts, uint32_t nweight,
-                    float *parts, uint32_t *error)
+                    float *parts, uint32_t polls, uint32_t *error)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ float s_loss[4];
@@ -894,7 +909,7 @@ k_guide_train_fused(const unsigned char *img, const float *params, GuideParams g
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int row = 32 * (warp & 3) + lane, part = warp >> 2;
     const bool worker = warp < kTfThreads / 32;  // the last warp issues the products
-    const uint32_t cbar = smem_u32(smem + kTfBar + 16);
+    const uint32_t cbar = smem_u32(smem + kTfBar + 16), dbar = cbar + 8;
     float *bias = reinterpret_cast<float *>(smem + kTfBias);
     const uint32_t xoff[kLayers] = {kTfX0, kTfX1, kTfX1 + 20480, kTfX1 + 40960, kTfX1 + 61440};
     // the columns of ones (in .. in + 15) of every x_l
@@ -908,8 +923,8 @@ k_guide_train_fused(const unsigned char *img, const float *params, GuideParams g
     const uint32_t mbar = smem_u32(smem + kTfBar);
     const uint32_t tslot = smem_u32(smem + kTfBar + 8);
     if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(mbar) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        mbar_init(mbar, 1);
+        mbar_init(dbar, 1);
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;\n" ::"r"(tslot) : "memory");
@@ -926,6 +941,7 @@ k_guide_train_fused(const unsigned char *img, const float *params, GuideParams g
     const uint32_t taddr = *reinterpret_cast<volatile uint32_t *>(smem + kTfBar + 8);
     const uint32_t d_base = smem_u32(smem + kTfD), w_img = smem_u32(smem + kTfW), x_base = smem_u32(smem);
     const uint32_t woff[kLayers] = {kTcW0, kTcW1, kTcW1 + 8192, kTcW1 + 16384, kTcW4};
+    uint32_t step = 0;  // steps begun: products that the workers wait for
 
     if (!worker) {
         // The products of every step, by one lane of a warp of their own: in a
@@ -937,12 +953,8 @@ k_guide_train_fused(const unsigned char *img, const float *params, GuideParams g
             atomicOr(error, ERR_TIMEOUT);
         }
         auto ready = [&] {
-            bar_sync(kTfReadyBar, kTfThreads + 32);
+            bar_sync(kTfReadyBar + (int)(step++ & 1u), kTfThreads + 32);
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        };
-        auto commit = [&] {
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(mbar)
-                         : "memory");
         };
         // dW_l += [delta_hi | delta_lo]^T x_l over the tile's 128 rows (8 MMAs of
         // 16 rows; MN-major operands: 8-row groups 128 B apart, 8-column groups
@@ -963,7 +975,7 @@ k_guide_train_fused(const unsigned char *img, const float *params, GuideParams g
                     uint64_t a = smem_desc(x_base + xoff[l], kTcRows * 16, 128), b = smem_desc(w_img + woff[l], N * 16, 128);
 #pragma unroll
                     for (uint32_t s2 = 0; s2 < fan_in(l) / 16; ++s2, a += kTcRows * 2, b += N * 2) tc_mma(taddr, a, b, idesc, s2 > 0);
-                    commit();
+                    commit_products(mbar);
                 }
                 __syncwarp();
             }
@@ -981,7 +993,7 @@ k_guide_train_fused(const unsigned char *img, const float *params, GuideParams g
 #pragma unroll
                         for (uint32_t s2 = 0; s2 < O / 16; ++s2, a += kTcRows * 2, b += 16) tc_mma(taddr, a, b, idesc, half + s2 > 0);
                     }
-                    commit();
+                    commit_products(mbar);
                     wgrad(l, !first);
                 }
                 __syncwarp();
@@ -989,7 +1001,7 @@ k_guide_train_fused(const unsigned char *img, const float *params, GuideParams g
             ready();
             if (leader) {
                 wgrad(0, !first);
-                commit();
+                commit_products(mbar);
             }
             __syncwarp();
             first = false;
@@ -1000,27 +1012,29 @@ k_guide_train_fused(const unsigned char *img, const float *params, GuideParams g
         float wsum = (uint32_t)lane < nweight ? weight_parts[lane] : 0.0f;
         const float wsum2 = (uint32_t)lane + 32 < nweight ? weight_parts[lane + 32] : 0.0f;
         float loss_sum = 0.0f;  // of the part 0 threads' rows
-        uint32_t phase = 0;
         bool failed = false;  // warp-uniform
         // this thread's shared-memory stores (and tensor-memory loads) are done
         auto ready = [&] {
             asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-            if (failed) bar_sync(kTfReadyBar, kTfThreads + 32);
-            else bar_arrive(kTfReadyBar, kTfThreads + 32);
+            const int bar = kTfReadyBar + (int)(step++ & 1u);
+            if (failed) bar_sync(bar, kTfThreads + 32);
+            else bar_arrive(bar, kTfThreads + 32);
         };
-        // Waits for the last commit (which covers every product issued before it).
+        // Waits for the step's commit (which covers every product issued before it).
         // Every wait is bounded; once one gives up the block runs on without waiting
-        // (but in step, at the barrier), so that it ends together, and its sums are
-        // dropped.
+        // (but in step, at the barriers), so that it ends together, and its sums are
+        // dropped. A warp that gives up may come to the next step's barrier before
+        // the others have come to this one's, so two barriers take turns: on one
+        // alone it would arrive twice in a phase and leave a later phase short of an
+        // arrival.
         auto finish = [&] {
             bool bad = *reinterpret_cast<volatile int *>(&s_failed) != 0;
-            if (!bad && !mbar_wait(mbar, phase)) {
+            if (!bad && !mbar_wait(mbar, (step - 1u) & 1u, polls)) {
                 *reinterpret_cast<volatile int *>(&s_failed) = 1;
                 atomicOr(error, ERR_TIMEOUT);
                 bad = true;
             }
-            phase ^= 1u;
             failed = __any_sync(0xffffffffu, bad);
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         };
@@ -1222,16 +1236,23 @@ k_guide_train_fused(const unsigned char *img, const float *params, GuideParams g
             if (part == 0 && lane == 0) s_loss[warp] = loss_sum;
             bar_sync(kTfWorkBar, kTfThreads);
             if (tid == 0) out[kNumParams] = (s_loss[0] + s_loss[1]) + (s_loss[2] + s_loss[3]);
-        } else {
-            // MMAs or the weight copy still in flight: wait again (bounded) before
-            // freeing their memory; the sums of this CTA count as nothing
-            mbar_wait(mbar, phase);
-            mbar_wait(cbar, 0);
+        } else {  // the sums of this CTA count as nothing
             for (int i = tid; i < kPartStride; i += kTfThreads) out[i] = 0.0f;
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
+    // After a wait gave up, products or the weight copy may still be in flight,
+    // several commits deep: the issuing lane commits them all to a barrier of its
+    // own, and its warp waits (bounded) before their memory is freed.
+    if (*reinterpret_cast<volatile int *>(&s_failed)) {
+        if (!worker) {
+            if (elect_one()) commit_products(dbar);
+            mbar_wait(dbar, 0);
+            mbar_wait(cbar, 0);
+        }
+        __syncthreads();
+    }
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;\n" ::"r"(taddr) : "memory");
 }
 
@@ -1515,7 +1536,7 @@ dr_status run_gradients(dr_guide *g, const float *pos, const float *dir, const f
         const unsigned tiles = (n + kTcRows - 1) / kTcRows;
         const unsigned blocks = std::min<unsigned>(tiles, (unsigned)g->ctx->num_sms);
         DR_CUDA(launch_after(k_guide_train_fused, blocks, kTfThreads + 32, kTfSmem, st, g->img, g->params, gp, pos, dir, sdir, weight, n,
-                             sums, sum_blocks, g->parts, g->ctx->d_error));
+                             sums, sum_blocks, g->parts, g->ctx->product_polls, g->ctx->d_error));
         *parts = g->parts;
         *nparts = (int)blocks;
     } else {
@@ -1565,7 +1586,7 @@ cudaError_t launch_guide_infer(const dr_guide *g, const float *pos, const float 
         const unsigned blocks = std::min<unsigned>(tiles, (unsigned)g->ctx->num_sms);
         const auto kernel = decoded ? k_guide_infer_tc<true> : k_guide_infer_tc<false>;
         const cudaError_t e = launch_after(kernel, blocks, 128 * kInferGroups, kTcSmem, st, g->img, g->params, guide_params(g),
-                                           pos, dir, list, count, max_rows, y, g->ctx->d_error);
+                                           pos, dir, list, count, max_rows, y, g->ctx->product_polls, g->ctx->d_error);
         if (e != cudaSuccess) return e;
     } else {
         const unsigned tiles = (max_rows + 15) / 16;

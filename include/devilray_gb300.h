@@ -575,6 +575,13 @@ dr_status dr_debug_expire_wait(dr_context *ctx, uint32_t polls, void *stream);
  * DR_ERR_STACK_OVERFLOW); its hit is not valid. */
 dr_status dr_debug_stack_limit(dr_context *ctx, uint32_t entries);
 
+/* At most `polls` polls (0: none) in each wait of this context's tcgen05 guiding
+ * kernels for their matrix products, so that waits give up while products are in
+ * flight; 2^22 and above restore the normal limit. The kernels then set the
+ * timeout bit, wait (with the normal limit) for what is in flight and end; what
+ * they wrote is not valid. */
+dr_status dr_debug_product_polls(dr_context *ctx, uint32_t polls);
+
 /* Makes the `after`-th next device allocation of the library (after = 1:
  * the next one) fail as cudaMalloc does when the device is out of memory;
  * 0 turns it off. Process-wide. The failing call returns DR_ERR_OUT_OF_MEMORY

@@ -94,6 +94,49 @@ def test_stack_cap_reports_overflow(native, oracle):
     assert lib.dr_debug_stack_limit(c.handle, 65) == 1  # DR_ERR_INVALID_ARGUMENT
 
 
+@pytest.mark.parametrize("n", [100, 30000])
+def test_timed_out_products_are_drained(native, n):
+    """Waits of the tcgen05 guiding kernels that give up while matrix products
+    are in flight (on some or all of the steps): the block ends together, waits
+    for its products before it gives back their memory, and reports the timeout;
+    the calls after it are exact. One tile, and more tiles than SMs."""
+    lib = native.load()
+    c = native.Context(0)
+    rng = np.random.default_rng(n)
+    g = native.Guide(c, seed=3, half_extent=10.0, infer_kernel=0)
+
+    def unit():
+        d = rng.normal(size=(n, 3))
+        return torch.from_numpy((d / np.linalg.norm(d, axis=1, keepdims=True)).astype(np.float32)).cuda()
+
+    pos = torch.from_numpy(rng.uniform(-10, 10, (n, 3)).astype(np.float32)).cuda()
+    nrm, sdir, w = unit(), unit(), torch.ones(n, device="cuda")
+
+    def infer():
+        y = torch.zeros((n, 40), device="cuda")
+        g.infer(pos, nrm, n, y)
+        torch.cuda.synchronize()
+        return y.cpu().numpy()
+
+    want_y, (want_loss, want_grad) = infer(), g.gradients(pos, nrm, sdir, w, n)
+    assert _status_of(c.check) == 0
+    for polls in (0, 1, 2, 5, 0):
+        native.check(lib.dr_debug_product_polls(c.handle, polls))
+        y = infer()
+        status = _status_of(c.check)
+        assert status == 5 if polls == 0 else status in (0, 5)  # DR_ERR_TIMEOUT
+        assert status == 5 or np.array_equal(y, want_y)
+        loss, grad = g.gradients(pos, nrm, sdir, w, n)
+        status = _status_of(c.check)
+        assert status == 5 if polls == 0 else status in (0, 5)
+        assert status == 5 or (loss == want_loss and np.array_equal(grad, want_grad))
+        native.check(lib.dr_debug_product_polls(c.handle, 1 << 22))
+        assert np.array_equal(infer(), want_y)
+        loss, grad = g.gradients(pos, nrm, sdir, w, n)
+        assert loss == want_loss and np.array_equal(grad, want_grad)
+        assert _status_of(c.check) == 0
+
+
 def _workload(native, ctx, spec, cam):
     """Scene creation, a render, a framebuffer, a guiding network and a batch:
     every call that allocates device memory."""
