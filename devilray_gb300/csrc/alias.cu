@@ -23,6 +23,7 @@
 #include <cooperative_groups.h>
 
 #include <climits>
+#include <mutex>
 
 namespace dr {
 
@@ -585,8 +586,8 @@ __global__ void __launch_bounds__(kCoarse) k_sweep_assign(const float *__restric
 // meetings and of the scattered list stores. Build of 66,356 weights 42.5 ->
 // 29 us, of 1,000 33 -> 17 us, of 3 28 -> 13 us; 131,072 weights 57 -> 39 us (the
 // separate kernels, which take over above, 53 us at 131,073).
-constexpr int kListBlock = 1024, kListItems = 8, kListCluster = 16;
-constexpr uint32_t kListMax = (uint32_t)kListBlock * kListItems * kListCluster;  // 131,072 weights
+constexpr int kListBlock = 1024, kListItems = 8;
+constexpr unsigned kListCluster = 16;
 // Tables of up to this many weights get their entries from the same launch
 // (100 weights: 16.8 -> 14.0 us; at 1,000 one SM's FP64 units take longer than
 // another launch: 16.8 -> 25.0 us).
@@ -750,26 +751,57 @@ __global__ void __launch_bounds__(kListBlock) k_sweep_lists(const float *__restr
     }
 }
 
-static cudaError_t launch_sweep_lists(const float *w, uint32_t n, SweepScalars *sc, int32_t *lights, i128 *Dexcl, int32_t *heavies,
-                                      i128 *Sincl, dr_alias_entry *out, cudaStream_t st)
-{
-    // as few blocks as give every thread one item, up to the cluster's 16; then more items
-    unsigned blocks = 1;
-    while (blocks < kListCluster && (uint64_t)blocks * kListBlock < n) blocks *= 2;
-    const uint32_t per_thread = (n + blocks * kListBlock - 1) / (blocks * kListBlock);
-    cudaError_t e = cudaFuncSetAttribute(k_sweep_lists, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return e;
+// The launch of one cluster of `blocks` blocks.
+struct ClusterLaunch {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(kListBlock);
-    cfg.stream = st;
     cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = blocks;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, k_sweep_lists, w, n, per_thread, sc, lights, Dexcl, heavies, Sincl, out);
+    ClusterLaunch(unsigned blocks, cudaStream_t st)
+    {
+        cfg.gridDim = dim3(blocks);
+        cfg.blockDim = dim3(kListBlock);
+        cfg.stream = st;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = blocks;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+    }
+};
+
+// The largest cluster of k_sweep_lists that the current device can run: 16
+// blocks, more than the 8 that every device offers, need as many free SMs in one
+// of its SM clusters, which a partition of a GPU may not have. 0: none.
+static unsigned list_cluster_limit()
+{
+    constexpr int kMaxDevices = 64;
+    static std::mutex mu;
+    static int known[kMaxDevices];  // limit + 1
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kMaxDevices) return 0;
+    std::lock_guard<std::mutex> lock(mu);
+    if (known[device] == 0) {
+        unsigned limit = kListCluster;
+        if (cudaFuncSetAttribute(k_sweep_lists, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) limit = 8;
+        for (; limit > 0; limit /= 2) {
+            const ClusterLaunch l(limit, nullptr);
+            int clusters = 0;
+            if (cudaOccupancyMaxActiveClusters(&clusters, k_sweep_lists, &l.cfg) == cudaSuccess && clusters > 0) break;
+        }
+        cudaGetLastError();
+        known[device] = (int)limit + 1;
+    }
+    return (unsigned)known[device] - 1;
+}
+
+static cudaError_t launch_sweep_lists(const float *w, uint32_t n, unsigned max_blocks, SweepScalars *sc, int32_t *lights, i128 *Dexcl,
+                                      int32_t *heavies, i128 *Sincl, dr_alias_entry *out, cudaStream_t st)
+{
+    // as few blocks as give every thread one item, up to the largest cluster; then more items
+    unsigned blocks = 1;
+    while (blocks < max_blocks && (uint64_t)blocks * kListBlock < n) blocks *= 2;
+    const uint32_t per_thread = (n + blocks * kListBlock - 1) / (blocks * kListBlock);
+    const ClusterLaunch l(blocks, st);
+    const cudaError_t e = cudaLaunchKernelEx(&l.cfg, k_sweep_lists, w, n, per_thread, sc, lights, Dexcl, heavies, Sincl, out);
     if (e != cudaSuccess || n <= kListWhole) return e;
     return launch_after(k_sweep_assign, (n + kCoarse - 1) / kCoarse, kCoarse, 0, st, w, n, sc, lights, Dexcl, heavies, Sincl, out);
 }
@@ -918,7 +950,7 @@ size_t alias_scratch_bytes(uint32_t n, int mode)
 static inline char *align256(char *p) { return reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(p) + 255) & ~uintptr_t(255)); }
 
 cudaError_t launch_alias_build(const float *w, uint32_t n, dr_alias_entry *out, int mode, void *scratch,
-                               size_t scratch_bytes, int num_sms, cudaStream_t st)
+                               size_t scratch_bytes, int num_sms, cudaStream_t st, unsigned max_cluster)
 {
     if (n == 0) return cudaSuccess;
     if (scratch_bytes < alias_scratch_bytes(n, mode)) return cudaErrorInvalidValue;
@@ -943,7 +975,10 @@ cudaError_t launch_alias_build(const float *w, uint32_t n, dr_alias_entry *out, 
     i128 *Sincl = Dexcl + n;
     int32_t *lights = reinterpret_cast<int32_t *>(Sincl + n);
     int32_t *heavies = lights + n;
-    if (n <= kListMax) return launch_sweep_lists(w, n, sc, lights, Dexcl, heavies, Sincl, out, st);
+    // the one-launch lists up to 8 items per thread of a cluster: 131,072 weights with 16 blocks
+    const unsigned cluster = std::min(list_cluster_limit(), max_cluster);
+    if (n <= (uint64_t)cluster * kListBlock * kListItems)
+        return launch_sweep_lists(w, n, cluster, sc, lights, Dexcl, heavies, Sincl, out, st);
     const int grid = (int)std::min<uint32_t>((n + 255) / 256, (uint32_t)num_sms * 8);
     k_sweep_init<<<1, 32, 0, st>>>(sc, n);
     k_sweep_exponent<<<grid, 256, 0, st>>>(w, n, sc);

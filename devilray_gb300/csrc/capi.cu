@@ -622,7 +622,7 @@ dr_status dr_alias_build(dr_context *ctx, const float *w, uint32_t n, dr_alias_e
         const dr_status s = ensure_scratch(ctx, need);
         if (s != DR_OK) return s;
     }
-    DR_CUDA(launch_alias_build(w, n, table, mode, ctx->scratch, ctx->scratch_bytes, ctx->num_sms, st));
+    DR_CUDA(launch_alias_build(w, n, table, mode, ctx->scratch, ctx->scratch_bytes, ctx->num_sms, st, ctx->max_cluster));
     return DR_OK;
 }
 

@@ -3,10 +3,11 @@
 //    kernels (streaming reads of a buffer that fits in L2 give the L2 read
 //    bandwidth, a buffer larger than L2 the HBM read bandwidth);
 //  * the failure paths' test hooks: a bounded mbarrier wait made to give up,
-//    a lower cap on the traversal stack and on the guiding kernels' waits for
-//    their products, and failed device allocations. None of them faults, traps
-//    or hangs a GPU: each makes the library take the same error path that a real
-//    timeout, overflow or out-of-memory takes.
+//    a lower cap on the traversal stack, on the guiding kernels' waits for their
+//    products and on the clusters of an alias build, and failed device
+//    allocations. None of them faults, traps or hangs a GPU: each makes the
+//    library take the same path that a real timeout, overflow, smaller device or
+//    out-of-memory takes.
 
 #include "dr_internal.h"
 #include "mbarrier.cuh"
@@ -68,6 +69,14 @@ extern "C" dr_status dr_debug_stack_limit(dr_context *ctx, uint32_t entries)
     DR_CHECK_ARG(ctx, "dr_debug_stack_limit: NULL context");
     DR_CHECK_ARG(entries <= 64, "dr_debug_stack_limit: at most 64 entries");
     ctx->stack_limit = entries ? entries : 64;
+    return DR_OK;
+}
+
+extern "C" dr_status dr_debug_max_cluster(dr_context *ctx, uint32_t blocks)
+{
+    DR_CHECK_ARG(ctx, "dr_debug_max_cluster: NULL context");
+    DR_CHECK_ARG(blocks <= 16 && (blocks & (blocks - 1)) == 0, "dr_debug_max_cluster: 0 or a power of two up to 16");
+    ctx->max_cluster = blocks;
     return DR_OK;
 }
 

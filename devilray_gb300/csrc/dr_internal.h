@@ -184,6 +184,7 @@ struct dr_context {
     void *scratch = nullptr;                    // grows on demand (alias builds, staging)
     size_t scratch_bytes = 0;
     uint32_t stack_limit = 64;                  // 8-wide traversal stack entries (dr_debug_stack_limit)
+    uint32_t max_cluster = 16;                  // blocks of an alias build's cluster (dr_debug_max_cluster)
     uint32_t product_polls = 1u << 22;          // limit of the guiding kernels' waits for their products (dr_debug_product_polls)
 };
 

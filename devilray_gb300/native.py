@@ -217,6 +217,7 @@ SIGNATURES = {
     "dr_debug_expire_wait": (C.c_int, [C.c_void_p, C.c_uint32, C.c_void_p]),
     "dr_debug_stack_limit": (C.c_int, [C.c_void_p, C.c_uint32]),
     "dr_debug_product_polls": (C.c_int, [C.c_void_p, C.c_uint32]),
+    "dr_debug_max_cluster": (C.c_int, [C.c_void_p, C.c_uint32]),
     "dr_debug_fail_allocation": (C.c_int, [C.c_uint32]),
 }
 

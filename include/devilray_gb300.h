@@ -582,6 +582,11 @@ dr_status dr_debug_stack_limit(dr_context *ctx, uint32_t entries);
  * they wrote is not valid. */
 dr_status dr_debug_product_polls(dr_context *ctx, uint32_t polls);
 
+/* dr_alias_build of this context runs with clusters of at most `blocks` blocks (0: no
+ * clusters, or a power of two up to 16, the default), as on a device or a
+ * partition that has no larger ones. Tables are the same. */
+dr_status dr_debug_max_cluster(dr_context *ctx, uint32_t blocks);
+
 /* Makes the `after`-th next device allocation of the library (after = 1:
  * the next one) fail as cudaMalloc does when the device is out of memory;
  * 0 turns it off. Process-wide. The failing call returns DR_ERR_OUT_OF_MEMORY

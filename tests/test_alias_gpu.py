@@ -110,3 +110,18 @@ def test_sweep_mode_at_cluster_sizes(native, ctx, oracle, n, kind):
         w[n - 1] = 2.5
     tab = device_build(ctx, native, w, native.DR_ALIAS_SWEEP)
     assert tab.tobytes() == oracle.alias_build_sweep(w).tobytes()
+
+
+@pytest.mark.parametrize("blocks", [0, 1, 2, 8])
+def test_sweep_mode_with_smaller_clusters(native, oracle, blocks):
+    """Devices without clusters of 16 blocks: smaller clusters with more items
+    per thread, the separate kernels above their reach (8,192 weights per block);
+    the tables are the same."""
+    lib = native.load()
+    c = native.Context(0)
+    native.check(lib.dr_debug_max_cluster(c.handle, blocks))
+    for n in (1, 200, 1025, 8192, 8193, 16385, 65536, 65537, 131072):
+        w = np.random.default_rng(n).lognormal(0, 1.5, n).astype(np.float32)
+        tab = device_build(c, native, w, native.DR_ALIAS_SWEEP)
+        assert tab.tobytes() == oracle.alias_build_sweep(w).tobytes(), n
+    assert lib.dr_debug_max_cluster(c.handle, 3) == 1 and lib.dr_debug_max_cluster(c.handle, 32) == 1
