@@ -1473,7 +1473,9 @@ struct dr_guide {
     __nv_bfloat16 *wb = nullptr;
     unsigned char *img = nullptr;  // weight image of the tcgen05 kernels (kImgBytes)
     float *scalars = nullptr;  // [0] sum of the batch's sample weights (mma.sync path), [1] loss, [4..] weight sums per block
-    float *parts = nullptr;    // partial gradients and loss of the tcgen05 training kernel, one row per CTA
+    float *parts = nullptr;    // partial gradients and loss, one row per CTA of the training kernel
+    int part_rows = 0;
+    void *parts_mem = nullptr; // the rows of a batch of several tiles (ensure_parts)
     dr::TrainBuffers tb{};
     void *tb_mem = nullptr;
     uint32_t capacity = 0;
@@ -1496,6 +1498,7 @@ void free_guide(dr_guide *g)
 {
     if (!g) return;
     cudaFree(g->mem);
+    cudaFree(g->parts_mem);
     cudaFree(g->tb_mem);
     delete g;
 }
@@ -1523,6 +1526,24 @@ dr_status ensure_train_capacity(dr_guide *g, uint32_t n)
     return DR_OK;
 }
 
+// Rows for the partial sums of `blocks` CTAs: the network comes with one (a
+// network that only infers needs none, and mapping 12.6 MB takes 0.1 ms), the
+// first batch of several tiles allocates one per SM. That call may be under
+// stream capture, where an allocation, which is no stream operation, needs the
+// relaxed mode.
+dr_status ensure_parts(dr_guide *g, int blocks)
+{
+    if (blocks <= g->part_rows) return DR_OK;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    DR_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    const cudaError_t e = dev_malloc(&g->parts_mem, (size_t)g->ctx->num_sms * kPartStride * sizeof(float));
+    DR_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    DR_CUDA(e);
+    g->parts = static_cast<float *>(g->parts_mem);
+    g->part_rows = g->ctx->num_sms;
+    return DR_OK;
+}
+
 // Loss and gradients of one batch, as *nparts rows of partial sums at *parts.
 dr_status run_gradients(dr_guide *g, const float *pos, const float *dir, const float *sdir, const float *weight,
                         uint32_t n, cudaStream_t st, const float **parts, int *nparts)
@@ -1530,20 +1551,20 @@ dr_status run_gradients(dr_guide *g, const float *pos, const float *dir, const f
     const GuideParams gp = guide_params(g);
     const unsigned sum_blocks = std::min<unsigned>((n + 255) / 256, kWeightParts);
     float *sums = g->scalars + 4;
+    // the tcgen05 kernel: one CTA per SM (its shared memory and 512 tensor-memory
+    // columns); the per-layer delta and activation buffers serve the mma.sync path
+    // only (the tcgen05 kernel keeps them on chip), whose sums meet in one row
+    const bool tc = g->cfg.infer_kernel == DR_GUIDE_INFER_TCGEN05;
+    const unsigned blocks = std::min<unsigned>((n + kTcRows - 1) / kTcRows, (unsigned)g->ctx->num_sms);
+    const dr_status r = tc ? ensure_parts(g, (int)blocks) : ensure_train_capacity(g, n);
+    if (r != DR_OK) return r;
     DR_CUDA(launch_after(k_guide_weight_sum, sum_blocks, 256, 0, st, weight, n, sums));
-    if (g->cfg.infer_kernel == DR_GUIDE_INFER_TCGEN05) {
-        // one CTA per SM (its shared memory and 512 tensor-memory columns)
-        const unsigned tiles = (n + kTcRows - 1) / kTcRows;
-        const unsigned blocks = std::min<unsigned>(tiles, (unsigned)g->ctx->num_sms);
+    if (tc) {
         DR_CUDA(launch_after(k_guide_train_fused, blocks, kTfThreads + 32, kTfSmem, st, g->img, g->params, gp, pos, dir, sdir, weight, n,
                              sums, sum_blocks, g->parts, g->ctx->product_polls, g->ctx->d_error));
         *parts = g->parts;
         *nparts = (int)blocks;
     } else {
-        // the per-layer delta and activation buffers serve the mma.sync path only
-        // (the tcgen05 kernel keeps them on chip); its sums meet in one row
-        const dr_status r = ensure_train_capacity(g, n);
-        if (r != DR_OK) return r;
         DR_CUDA(cudaMemsetAsync(g->parts, 0, kPartStride * sizeof(float), st));
         k_guide_add_sums<<<1, 32, 0, st>>>(sums, sum_blocks, g->scalars);
         k_guide_train_fb<<<(n + 63) / 64, 128, kTrainSmem, st>>>(g->wb, g->params, gp, pos, dir, sdir, weight, n,
@@ -1650,7 +1671,7 @@ dr_status dr_guide_create(dr_context *ctx, const dr_guide_config *cfg, dr_guide 
     };
     const size_t at_params = place(kNumParams * 4), at_m = place(kNumParams * 4), at_v = place(kNumParams * 4),
                  at_grad = place(kNumParams * 4), at_wb = place(kNumWeights * 2), at_img = place(kImgBytes),
-                 at_scalars = place(kScalarBytes), at_parts = place((size_t)ctx->num_sms * kPartStride * 4);
+                 at_scalars = place(kScalarBytes), at_parts = place(kPartStride * 4);
     cudaError_t e = dev_malloc(&g->mem, bytes);
     if (e == cudaSuccess) e = cudaMemset(g->mem + at_scalars, 0, kScalarBytes);
     if (e != cudaSuccess) {
@@ -1665,6 +1686,7 @@ dr_status dr_guide_create(dr_context *ctx, const dr_guide_config *cfg, dr_guide 
     g->img = g->mem + at_img;
     g->scalars = reinterpret_cast<float *>(g->mem + at_scalars);
     g->parts = reinterpret_cast<float *>(g->mem + at_parts);
+    g->part_rows = 1;
     // He-uniform initialisation (ReLU), last layer scaled by 0.1, zero biases
     std::mt19937_64 rng(g->cfg.seed);
     std::vector<float> p(kNumParams, 0.0f);

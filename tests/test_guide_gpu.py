@@ -218,3 +218,42 @@ def test_state_checkpoint_resumes_training(native, ctx):
         g2.set_state(bad)
     for g in (g1, g2, g3):
         g.close()
+
+
+def test_networks_that_do_not_train_take_little_memory(native, ctx):
+    """The partial sums of a training step (one row per SM) are allocated by the
+    first batch that needs them, not with the network."""
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    guides = [native.Guide(ctx, seed=k) for k in range(8)]
+    torch.cuda.synchronize()
+    assert free0 - torch.cuda.mem_get_info()[0] <= 16 << 20
+    for g in guides:
+        g.close()
+
+
+@pytest.mark.parametrize("n", [100, 5000])
+def test_first_training_step_under_capture(native, ctx, n):
+    """A network's first training step may be a captured one: one replay gives
+    the parameters of an uncaptured step, bit for bit, whether the batch needs
+    more partial sums than the network came with (more than one tile) or not."""
+    rng = np.random.default_rng(n)
+
+    def unit():
+        d = rng.normal(size=(n, 3))
+        return torch.from_numpy((d / np.linalg.norm(d, axis=1, keepdims=True)).astype(np.float32)).cuda()
+
+    pos = torch.from_numpy(rng.uniform(-1, 1, (n, 3)).astype(np.float32)).cuda()
+    nrm, sdir, w = unit(), unit(), torch.ones(n, device="cuda")
+    plain, captured = native.Guide(ctx, seed=2), native.Guide(ctx, seed=2)
+    plain.train_step(pos, nrm, sdir, w, n)
+    want = plain.params()
+    stream = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        captured.train_step(pos, nrm, sdir, w, n, stream=stream)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert np.array_equal(captured.params(), want)
+    ctx.check()
