@@ -3,12 +3,19 @@
 // stack depth) by timing short probe renders on the device.
 //
 // The search is coordinate descent from the defaults (8-wide, 2^22 paths per
-// wave, 3 streams, adaptive fetch, 8 stack entries): each knob in turn is set
+// wave, 3 streams, the default fetch, 8 stack entries): each knob in turn is set
 // to the fastest of its candidates with the others fixed, where a candidate
 // must beat the incumbent by more than 2 %. Every candidate renders the same
 // samples, and the images do not depend on the schedule, so the probes differ
 // only in time. Timing: CUDA events on the probe stream, one warm-up render,
 // then the minimum over `reps` renders.
+//
+// A probe runs the kernels that the render itself will run: 8-wide waves of up to
+// kWholePathsPerSm paths per SM are one kernel, which has no fetch size and no
+// shared stack to choose, larger ones are kernels per bounce. So a probe of a
+// render that is larger than such a wave takes as many samples as make it larger
+// too (four times, where the render has them: past the bounces of the wave's
+// last paths, which the one kernel takes as well).
 
 #include "dr_internal.h"
 
@@ -63,7 +70,7 @@ dr_status time_probe(Probe &p, uint32_t reps, F &&run, float &ms)
 
 const uint32_t kWaveCandidates[] = {1u << 19, 1u << 20, 1u << 21, 1u << 22, 1u << 23, 1u << 24};
 const uint32_t kStreamCandidates[] = {1, 2, 3};
-const uint32_t kChunkCandidates[] = {0, 32, 64, 128};
+const uint32_t kChunkCandidates[] = {0, 64, 128};  // 0: the renderer's default, 32
 const uint32_t kStackCandidates[] = {8, 4, 16};
 
 // A candidate replaces the incumbent only when its probe is faster by more
@@ -79,18 +86,29 @@ uint32_t &knob_ref(Knobs &k, int knob)
     return knob == 0 ? k.wave_paths : knob == 1 ? k.streams : knob == 2 ? k.chunk : k.stack;
 }
 
-// Coordinate descent over wave size, streams, fetch size and stack depth for
-// a fixed layout.
+uint64_t whole_paths(const dr_context *ctx) { return (uint64_t)ctx->num_sms * kWholePathsPerSm; }
+
+// Samples per pixel of a probe of `paths` paths in all over `pixels` pixels, at least `least`.
+uint32_t probe_samples(const dr_context *ctx, uint64_t pixels, uint64_t paths, uint32_t least)
+{
+    const uint64_t whole = whole_paths(ctx);
+    if (paths <= whole) return least;
+    const uint64_t target = std::min(paths, 4 * whole);
+    return (uint32_t)std::max<uint64_t>(least, (target + pixels - 1) / pixels);
+}
+
+// Coordinate descent over wave size and streams and, with `traversal` (waves of
+// the persistent 8-wide kernels), fetch size and stack depth for a fixed layout.
 template <class Measure>
-dr_status descend(Knobs &best, float &best_ms, Measure &&measure)
+dr_status descend(Knobs &best, float &best_ms, bool traversal, Measure &&measure)
 {
     for (int knob = 0; knob < 4; ++knob) {
         const uint32_t *cand = knob == 0   ? kWaveCandidates
                                : knob == 1 ? kStreamCandidates
                                : knob == 2 ? kChunkCandidates
                                            : kStackCandidates;
-        const int n = knob == 0 ? 6 : knob == 1 ? 3 : knob == 2 ? 4 : 3;
-        if (knob >= 2 && best.layout != 8) break;  // fetch size and stack belong to the persistent 8-wide kernels
+        const int n = knob == 0 ? 6 : 3;
+        if (knob >= 2 && (best.layout != 8 || !traversal)) break;
         Knobs winner = best;
         for (int i = 0; i < n; ++i) {
             Knobs k = best;
@@ -124,7 +142,9 @@ dr_status dr_autotune(dr_context *ctx, const dr_scene_desc *desc, const dr_camer
     DR_CHECK_ARG(cam->width > 0 && cam->height > 0, "dr_autotune: empty image");
     DR_CUDA(cudaSetDevice(ctx->device));
     *out = dr_autotune_result{};
-    const uint32_t probe_spp = tc && tc->probe_spp ? tc->probe_spp : std::max<uint32_t>(1, std::min<uint32_t>(cfg->spp, 2));
+    const uint64_t npix = (uint64_t)cam->width * (uint64_t)cam->height;
+    const uint32_t spp = std::max<uint32_t>(1, cfg->spp);
+    const uint32_t probe_spp = tc && tc->probe_spp ? tc->probe_spp : probe_samples(ctx, npix, npix * spp, std::min<uint32_t>(spp, 2));
     const uint32_t reps = tc && tc->reps ? tc->reps : 2;
     std::vector<uint32_t> layouts = {8};
     if (!tc || tc->try_layouts) layouts.push_back(2);
@@ -133,7 +153,6 @@ dr_status dr_autotune(dr_context *ctx, const dr_scene_desc *desc, const dr_camer
     DR_CUDA(cudaStreamCreateWithFlags(&p.stream, cudaStreamNonBlocking));
     DR_CUDA(cudaEventCreate(&p.t0));
     DR_CUDA(cudaEventCreate(&p.t1));
-    const size_t npix = (size_t)cam->width * (size_t)cam->height;
     void *accum = nullptr;
     dr_status st = dr_device_allocate(ctx, npix * 16, &accum);
     if (st != DR_OK) return st;
@@ -170,7 +189,8 @@ dr_status dr_autotune(dr_context *ctx, const dr_scene_desc *desc, const dr_camer
     }
     if (st == DR_OK) {
         dr_scene *s = scenes[best.layout == 8 ? 0 : 1];
-        st = descend(best, best_ms, [&](const Knobs &k, float &ms) { return measure_on(s, k, ms); });
+        st = descend(best, best_ms, npix * probe_spp > whole_paths(ctx),
+                     [&](const Knobs &k, float &ms) { return measure_on(s, k, ms); });
     }
     for (dr_scene *s : scenes) dr_scene_destroy(s);
     dr_device_free(ctx, accum);
@@ -191,7 +211,13 @@ dr_status dr_autotune_batch(dr_context *ctx, const dr_job *jobs, uint32_t njobs,
     DR_CUDA(cudaSetDevice(ctx->device));
     *out = dr_autotune_result{};
     const uint32_t reps = tc && tc->reps ? tc->reps : 2;
-    const uint32_t probe_spp = tc && tc->probe_spp ? tc->probe_spp : 1;
+    uint64_t pixels = 0, paths = 0;
+    for (uint32_t j = 0; j < njobs; ++j) {
+        const uint64_t npix = (uint64_t)jobs[j].camera.width * (uint64_t)jobs[j].camera.height;
+        pixels += npix;
+        paths += npix * jobs[j].config.spp;
+    }
+    const uint32_t probe_spp = tc && tc->probe_spp ? tc->probe_spp : probe_samples(ctx, std::max<uint64_t>(pixels, 1), paths, 1);
     Probe p;
     DR_CUDA(cudaStreamCreateWithFlags(&p.stream, cudaStreamNonBlocking));
     DR_CUDA(cudaEventCreate(&p.t0));
@@ -220,7 +246,7 @@ dr_status dr_autotune_batch(dr_context *ctx, const dr_job *jobs, uint32_t njobs,
         return r;
     };
     if (st == DR_OK) st = measure(best, best_ms);
-    if (st == DR_OK) st = descend(best, best_ms, measure);
+    if (st == DR_OK) st = descend(best, best_ms, pixels * probe_spp > whole_paths(ctx), measure);
     for (void *q : scratch) dr_device_free(ctx, q);
     if (st != DR_OK) return st;
     out->layout = best.layout;

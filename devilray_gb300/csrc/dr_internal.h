@@ -198,6 +198,12 @@ namespace dr {
 dr_status ensure_scratch(dr_context *ctx, size_t bytes);
 }  // namespace dr
 
+namespace dr {
+// 8-wide waves of up to this many paths per SM run whole paths in one kernel
+// (render.cu says why), larger ones a kernel per step and bounce.
+constexpr uint32_t kWholePathsPerSm = 1024;
+}  // namespace dr
+
 struct dr_scene;
 namespace dr {
 // Uploads the shading records, objects, materials and light tables of a scene

@@ -72,7 +72,7 @@ constexpr int kShadeMinBlocks = DR_SHADE_MIN_BLOCKS;
 // 1,367 us (1,716 without), eight uneven scenes 967 / 969 / 969 us (1,286); a
 // limit of 131,072 makes the 1080p many-light image slower (10.0 -> 12.7 ms), where
 // the longest walks of a 2^20-triangle scene want more rays in flight.
-constexpr uint32_t kWholePathsPerSm = 1024, kTailPathsPerSm = 216;
+constexpr uint32_t kTailPathsPerSm = 216;
 // Looked at before bounces 2, 3, 4, 6, 8, 12, ..: a look that finds too many paths
 // costs 3 us, one that comes a bounce late some 60. Eight uneven scenes, 4 spp,
 // 885 us with powers of two only, 858 us; 860 us before every bounce, which costs

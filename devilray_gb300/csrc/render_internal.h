@@ -73,7 +73,7 @@ struct WaveConfig {
     // 1080p, 64 spp: 2^21 -> 188 ms, 2^22 -> 163 ms
     uint32_t wave_paths = 1u << 22;
     uint32_t streams = kMaxWaveStreams;
-    uint32_t chunk = 0;              // rays per warp fetch of the persistent traversal, 0 = adaptive
+    uint32_t chunk = 0;              // rays per warp fetch of the persistent traversal, 0 = 32
     uint32_t stack = 8;              // shared-memory stack entries per lane: 4, 8 or 16
 };
 

@@ -570,7 +570,7 @@ class Batch:
             pass
 
 
-def autotune_batch(ctx: "Context", jobs: list, probe_spp: int = 1, reps: int = 2) -> AutotuneResult:
+def autotune_batch(ctx: "Context", jobs: list, probe_spp: int = 0, reps: int = 2) -> AutotuneResult:
     arr = (Job * len(jobs))(*jobs)
     tc = AutotuneConfig(probe_spp, reps, 0, 0)
     out = AutotuneResult()

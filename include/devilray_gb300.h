@@ -274,7 +274,9 @@ typedef struct dr_render_config {
     int32_t debug;           /* dr_debug_view */
     uint32_t streams;        /* concurrent waves, 1..3, 0 = 3 */
     uint32_t chunk;          /* rays per warp fetch of the persistent traversal
-                                (32, 64, 96 or 128), 0 = adaptive */
+                                (32, 64, 96 or 128), 0 = the default, 32; waves of up
+                                to 1,024 paths per SM, which run whole paths in one
+                                kernel, use neither chunk nor stack */
     uint32_t stack;          /* traversal-stack entries per lane kept in shared memory
                                 by the 8-wide kernels (4, 8 or 16), 0 = 8 */
 } dr_render_config;
@@ -342,7 +344,7 @@ typedef struct dr_job {
 typedef struct dr_batch_config {
     uint32_t wave_paths;     /* path slots per wave, 0 = 2^22 (at least one sample of the largest image) */
     uint32_t streams;        /* concurrent waves, 1..3, 0 = 3 */
-    uint32_t chunk;          /* persistent traversal fetch (32..128, multiple of 32), 0 = adaptive */
+    uint32_t chunk;          /* persistent traversal fetch (32..128, multiple of 32), 0 = 32 */
     uint32_t use_graph;      /* 1: capture the schedule into a CUDA graph on the first render */
     uint32_t stack;          /* shared-memory traversal-stack entries per lane (4, 8 or 16), 0 = 8 */
 } dr_batch_config;
@@ -379,7 +381,8 @@ dr_status dr_render_batch(dr_context *ctx, const dr_job *jobs, uint32_t njobs, c
 /* ---- autotuning ------------------------------------------------------------------- */
 
 typedef struct dr_autotune_config {
-    uint32_t probe_spp;      /* samples per probe render; 0 = min(spp, 2) (dr_autotune), 1 (batch) */
+    uint32_t probe_spp;      /* samples per probe render; 0 = min(spp, 2) (dr_autotune), 1 (batch), and as
+                                many more as the probe needs to run the kernels of the whole render */
     uint32_t reps;           /* timed renders per candidate, minimum taken; 0 = 2 */
     uint32_t try_layouts;    /* dr_autotune: 1 = build the scene 8-wide and 2-wide and time both */
     uint32_t max_leaf_size;  /* build setting of the probe scenes, 0 = default */

@@ -179,3 +179,39 @@ def test_invalid_stack_depth_is_rejected(native, ctx):
     jobs, _ = _batch_buffers(native, scs, _job_specs()[:2])
     with pytest.raises(Exception, match="stack"):
         native.render_batch(ctx, jobs, stack=5)
+
+
+def _render_ms(scene, cam, spp):
+    acc = torch.zeros((cam["width"] * cam["height"], 4), dtype=torch.float32, device="cuda")
+    best = 1e30
+    for _ in range(4):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        scene.render(cam, acc, spp=spp, max_depth=8)
+        b.record()
+        torch.cuda.synchronize()
+        best = min(best, a.elapsed_time(b))
+    return best
+
+
+def test_autotune_probes_run_the_kernels_of_the_render(native, ctx):
+    """A render whose waves go through the per-bounce kernels is probed with
+    enough samples to go through them too (a probe of two samples of this image
+    would be one whole-path wave), with each fetch size once; one that fits a
+    whole-path wave has no fetch size or stack depth to choose."""
+    spec, cam, spp = scenes.box_room(sphere_level=2), scenes.camera(64, 48), 256
+    scene = native.Scene.from_spec(ctx, spec)
+    two = _render_ms(scene, cam, 2)
+    large = native.autotune(ctx, spec, cam, spp=spp, max_depth=8, reps=1)
+    assert large.best_ms > 2 * two
+    if large.layout == 8:
+        cands = large.as_dict()["candidates"]
+        assert {c["chunk"] for c in cands} == {0, 64, 128} and {c["stack"] for c in cands} == {4, 8, 16}
+    small = native.autotune(ctx, spec, cam, spp=4, max_depth=8, reps=1)
+    assert {c["chunk"] for c in small.as_dict()["candidates"]} == {0}
+    assert small.best_ms < large.best_ms
+    n = 64 * 48
+    acc = torch.zeros((n, 4), dtype=torch.float32, device="cuda")
+    res = native.autotune_batch(ctx, [native.make_job(scene, cam, acc, spp=spp, max_depth=8)], reps=1)
+    assert res.best_ms > 2 * two and not acc.any()
+    assert {c["chunk"] for c in res.as_dict()["candidates"]} == {0, 64, 128}
