@@ -451,17 +451,19 @@ __global__ void k_sweep_scatter(const float *__restrict__ w, uint32_t n, const S
 
 __device__ __forceinline__ float pdf_of(long long m, unsigned long long W) { return (float)((double)m / (double)W); }
 
-// (float)(x / Wd) for x >= 0, with inv = 1 / Wd: the product x inv is within two
-// units of the last place of the quotient, so both round to the same float
-// unless the product's 29 bits below a float's lie that close to half; there
+// (float)(x / Wd) for a whole x >= 0, with inv = 1 / Wd: the product x inv is
+// within two units of the last place of the quotient, so both round to the same
+// float unless the product's 29 bits below a float's lie that close to half; there
 // (once in 2^26) the division decides. FP64 runs at 1/64 of the FP32 rate, and a
 // division is some ten operations. Below 2^-126, where a float has fewer bits, the
-// division decides as well.
+// division decides as well, but not for 0, the weight of everything that does not
+// emit (66,356 weights, 2 % / 98 % of them 0: 28.8 -> 27.2 / 30.1 -> 29.2 us).
 __device__ __forceinline__ float ratio_f(double x, double Wd, double inv)
 {
     const double q = x * inv;
-    const uint32_t low = (uint32_t)__double2loint(q) & 0x1fffffffu;
-    if (low - 0x0ffffffcu <= 8u || q < 0x1p-126) return (float)(x / Wd);
+    const uint32_t low = (uint32_t)__double2loint(q) & 0x1fffffffu, high = (uint32_t)__double2hiint(q);
+    // high - 1 of a zero wraps round; 2^-126 has the high word (1023 - 126) << 20
+    if (low - 0x0ffffffcu <= 8u || high - 1u < ((1023u - 126u) << 20) - 1u) return (float)(x / Wd);
     return (float)q;
 }
 
@@ -470,7 +472,7 @@ __device__ __forceinline__ float ratio_f(double x, double Wd, double inv)
 // memory.
 constexpr int kCoarse = 256;
 template <bool GREATER>
-__device__ __forceinline__ int32_t list_search(const i128 *__restrict__ list, int32_t count, const i128 *coarse, int32_t step, i128 key)
+__device__ __forceinline__ int32_t list_search(const i128 *list, int32_t count, const i128 *coarse, int32_t step, i128 key)
 {
     // coarse[c] = list[min((c + 1) step, count) - 1]
     int32_t lo = 0, hi = kCoarse;
