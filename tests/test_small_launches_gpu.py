@@ -114,3 +114,90 @@ def test_captured_waves_equal_a_plain_render(native, ctx, streams):
         images.append((acc, casts))
     assert torch.equal(images[0][0].view(torch.int32), images[1][0].view(torch.int32))
     assert torch.equal(images[0][1], images[1][1])
+
+
+def test_grazing_rays_in_a_large_launch(native, ctx, oracle):
+    """Rays through vertices and edges, in a launch above the team limit: the
+    persistent closest-hit and any-hit kernels, both triangle tests."""
+    from test_trace_gpu import grazing_rays
+    half = scenes.density_half(6000)
+    soup, _, _ = scenes.incoherent_soup(6000, seed=41, half=half)
+    rays = grazing_rays(soup, _team_limit() + 1, seed=42)
+    scene = native.Scene(ctx, soup)
+    dev = torch.from_numpy(rays).cuda()
+    for mode in (0, 1):
+        hits = torch.empty((len(rays), 2), dtype=torch.int32, device="cuda")
+        occ = torch.empty(len(rays), dtype=torch.uint8, device="cuda")
+        scene.trace_closest(dev, len(rays), hits, mode)
+        scene.trace_any(dev, len(rays), occ, mode)
+        h = hits.cpu().numpy()
+        tb, pb = oracle.trace_brute(soup, rays, tri_mode=mode)
+        assert (pb >= 0).mean() > 0.5
+        assert np.array_equal(h[:, 0], tb.view(np.int32)) and np.array_equal(h[:, 1], pb)
+        assert np.array_equal(occ.cpu().numpy().astype(bool), pb >= 0)
+    ctx.check()
+
+
+def test_stack_cap_reports_overflow_in_large_launches(native):
+    """The overflow exits of the persistent kernels (the small launches take the
+    team kernels): closest hit, any hit and the renderer's per-bounce traversal
+    report it, and are exact again with the full stack."""
+    lib = native.load()
+    c = native.Context(0)
+    half = scenes.density_half(65536)
+    soup, _, _ = scenes.incoherent_soup(65536, seed=5, half=half)
+    n = _team_limit() + 1
+    dev = torch.from_numpy(scenes.incoherent_rays(n, seed=6, half=half)).cuda()
+    scene = native.Scene(c, soup)
+    rscene = native.Scene.from_spec(c, scenes.many_light(6 * 1280, 40, seed=3, half=6.0))
+    w, h = 512, -(-1024 * torch.cuda.get_device_properties(0).multi_processor_count // 512) + 1
+    cam = scenes.outside_camera(w, h, distance=20.0, half=6.0)
+
+    def closest():
+        out = torch.zeros((n, 2), dtype=torch.int32, device="cuda")
+        scene.trace_closest(dev, n, out)
+        return out
+
+    def occluded():
+        out = torch.zeros(n, dtype=torch.uint8, device="cuda")
+        scene.trace_any(dev, n, out)
+        return out
+
+    def image():
+        acc = torch.zeros((w * h, 4), dtype=torch.float32, device="cuda")
+        rscene.render(cam, acc, spp=1, max_depth=6)
+        return acc.view(torch.int32)
+
+    want = [f() for f in (closest, occluded, image)]
+    c.check()
+    for f in (closest, occluded, image):
+        native.check(lib.dr_debug_stack_limit(c.handle, 1))
+        f()
+        torch.cuda.synchronize()
+        assert lib.dr_context_check(c.handle) == 6  # DR_ERR_STACK_OVERFLOW
+        native.check(lib.dr_debug_stack_limit(c.handle, 0))
+    assert all(torch.equal(f(), w0) for f, w0 in zip((closest, occluded, image), want))
+    c.check()
+
+
+@pytest.mark.parametrize("streams,chunk,stack", [(1, 64, 4), (2, 128, 16), (3, 0, 4), (1, 0, 16), (2, 96, 8)])
+def test_large_batch_waves_of_several_scenes(native, ctx, streams, chunk, stack):
+    """Waves above the whole-path limit that mix the images of three scenes, with
+    every shared-stack depth and fetch size of the per-bounce traversal: each
+    image equals the one rendered alone."""
+    specs = [scenes.box_room(2), scenes.many_light(6 * 1280, 40, seed=3, half=6.0), scenes.box_room(1)]
+    scs = [native.Scene.from_spec(ctx, s) for s in specs]
+    jobs, outs, alone = [], [], []
+    for k, (si, w, h, spp, depth) in enumerate([(0, 300, 200, 3, 6), (1, 257, 190, 2, 9), (2, 320, 240, 2, 4), (1, 129, 65, 5, 12)]):
+        cam = scenes.outside_camera(w, h, distance=20.0, half=6.0) if si == 1 else scenes.camera(w, h)
+        acc, ref = (torch.zeros((w * h, 4), dtype=torch.float32, device="cuda") for _ in range(2))
+        casts, rcasts = (torch.zeros(w * h, dtype=torch.int32, device="cuda") for _ in range(2))
+        jobs.append(native.make_job(scs[si], cam, acc, casts, spp=spp, max_depth=depth, seed=k))
+        scs[si].render(cam, ref, rcasts, spp=spp, max_depth=depth, seed=k)
+        outs.append((acc, casts))
+        alone.append((ref, rcasts))
+    native.render_batch(ctx, jobs, wave_paths=200000, streams=streams, chunk=chunk, stack=stack)
+    torch.cuda.synchronize()
+    ctx.check()
+    for (a, c), (ra, rc) in zip(outs, alone):
+        assert torch.equal(a.view(torch.int32), ra.view(torch.int32)) and torch.equal(c, rc)
