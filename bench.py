@@ -6,14 +6,17 @@ log-uniform in [0.5,3]; rays with origins uniform in the cube and directions
 uniform on the sphere), FP32, reference triangle test (bit-exact t and hit
 index against the reference). Synthetic, seeded inputs.
 
-  python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
+  python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference|port]
 
 ``value``  : rays/s with rays resident in device memory (CUDA events on the
              launching stream, max over ranks), in Mrays/s.
 ``e2e``    : the same through dr_trace_closest_host with pinned host buffers:
              the ray upload and the hit download are inside the timed region.
-``--impl reference`` times the reference's CPU traversal (the oracle's port of
-getIntersectionImpl over the reference's median-split BBH) on the host cores.
+``--impl reference`` is the unmodified reference's own run; the reference is a
+CMake / Conan C++ project that does not install as a Python package, so this says
+that it is unavailable. ``--impl port`` times this repository's restatement of the
+reference's CPU traversal (the oracle's getIntersectionImpl over the
+reference's median-split BBH) on the host cores.
 """
 from __future__ import annotations
 
@@ -45,8 +48,8 @@ NCU_PROFILE = {8: "trace_closest_p8_incoherent_1M_tris_16M_rays.md",
 # per scheduler and cycle).
 NCU_WARP_INST_PER_RAY = {8: 3_146_615_735 / NUM_RAYS}
 METRIC = "Mrays/s closest-hit"
-# Seconds the reference arm's timed steps may take in all (it sizes its
-# per-step sample of the workload to fit).
+# Seconds the timed steps of --impl port may take in all (it sizes its per-step
+# sample of the workload to fit).
 REF_TIMED_BUDGET_S = 150
 WORKLOAD = "incoherent closest-hit: 2^20-triangle icosphere soup, 16,777,216 rays"
 L2_BYTES = 129 * 1024 * 1024
@@ -142,6 +145,17 @@ def cpu_baseline(soup, rays, sample: int, threads: int):
 
 
 def run_reference(args):
+    """The reference cannot be installed here: one line that says so, from rank 0."""
+    rank, local, world = _env_rank()
+    if rank == 0:
+        print(json.dumps({"impl": "reference", "unavailable":
+                          "pip finds neither setup.py nor pyproject.toml: the reference is a CMake/Conan C++ project "
+                          "without a Python package"}), flush=True)
+    return 0
+
+
+def run_port(args):
+    """The reference's CPU traversal as the oracle restates it, on the host cores."""
     rank, local, world = _env_rank()
     if rank != 0:
         return 0
@@ -174,7 +188,7 @@ def run_reference(args):
     total = sum(times)
     value = sample * args.steps / total / 1e6
     line = {
-        "impl": "reference", "metric": METRIC, "value": value, "unit": "Mrays/s", "n_gpus": args.gpus,
+        "impl": "port", "metric": METRIC, "value": value, "unit": "Mrays/s", "n_gpus": args.gpus,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": 1e3 * total / args.steps,
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
         "config": {"workload": WORKLOAD, "num_triangles": NUM_TRIS, "num_rays": NUM_RAYS,
@@ -924,10 +938,10 @@ def main():
     ap.add_argument("--gpus", type=int, default=1)
     ap.add_argument("--steps", type=int, default=200)
     ap.add_argument("--warmup", type=int, default=3)
-    ap.add_argument("--impl", choices=["ours", "reference"], default="ours")
+    ap.add_argument("--impl", choices=["ours", "reference", "port"], default="ours")
     ap.add_argument("--cpu-sample", type=int, default=1 << 20)
     ap.add_argument("--ref-sample", type=int, default=0,
-                    help="rays per timed step of --impl reference (0: the whole workload if the steps fit)")
+                    help="rays per timed step of --impl port (0: the whole workload if the steps fit)")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-render", action="store_true")
     ap.add_argument("--no-batch", action="store_true")
@@ -949,6 +963,8 @@ def main():
         args.warmup = 3
     if args.impl == "reference":
         return run_reference(args)
+    if args.impl == "port":
+        return run_port(args)
     return run_ours(args)
 
 

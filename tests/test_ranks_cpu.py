@@ -66,3 +66,17 @@ def test_reference_arm_runs_on_rank_zero_only(monkeypatch):
     # a non-zero rank exits 0 at once, before building any workload
     monkeypatch.setattr(bench, "build_workload", lambda rank: pytest.fail("rank 1 built a workload"))
     assert bench.run_reference(None) == 0
+
+
+def test_reference_arm_says_that_it_is_unavailable(capsys, monkeypatch):
+    """The reference arm runs nothing of this repository in the reference's
+    name: one line on rank 0 with the reason."""
+    import argparse
+    import json
+    import bench
+    for name in ("RANK", "LOCAL_RANK", "WORLD_SIZE"):
+        monkeypatch.delenv(name, raising=False)
+    args = argparse.Namespace(gpus=1, steps=1, warmup=3, ref_sample=1 << 16)
+    assert bench.run_reference(args) == 0
+    line = json.loads(capsys.readouterr().out)
+    assert line["impl"] == "reference" and line["unavailable"] and "value" not in line
