@@ -408,7 +408,6 @@ __global__ void __launch_bounds__(128 * kInferGroups, 1)
 k_guide_infer_tc(const unsigned char *img, const float *params, GuideParams gp, const float *pos, const float *dir,
                  const uint32_t *list, const uint32_t *count, uint32_t n_fixed, float *y, uint32_t polls, uint32_t *error)
 {
-    constexpr int kCols = 16;  // accumulator columns an epilogue holds at once
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ int s_failed;
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, group = warp >> 2, row = tid & 127;
@@ -511,25 +510,23 @@ k_guide_infer_tc(const unsigned char *img, const float *params, GuideParams gp, 
             const float4 *b = reinterpret_cast<const float4 *>(bias + l * kHid);
             if (l < kLayers - 1) {
 #pragma unroll
-                for (int h = 0; h < 64 / kCols; ++h) {
-                    float v[kCols];
-#pragma unroll
-                    for (int c = 0; c < kCols; c += 16) tmem_ld16(lane_addr + kCols * h + c, v + c);
+                for (int h = 0; h < 64; h += 16) {  // 16 columns at once: 32 are no faster
+                    float v[16];
+                    tmem_ld16(lane_addr + h, v);
                     asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
-                    for (int j = 0; j < kCols / 8; ++j) {
+                    for (int j = 0; j < 2; ++j) {
                         uint32_t q[4];
 #pragma unroll
                         for (int k = 0; k < 2; ++k) {
                             const int i = 8 * j + 4 * k;
-                            const float4 c = b[kCols / 4 * h + i / 4];
+                            const float4 c = b[(h + i) / 4];
                             const float2 x = __fadd2_rn(make_float2(v[i], v[i + 1]), make_float2(c.x, c.y));
                             const float2 z = __fadd2_rn(make_float2(v[i + 2], v[i + 3]), make_float2(c.z, c.w));
                             q[2 * k] = relu_bf16(x.x, x.y);
                             q[2 * k + 1] = relu_bf16(z.x, z.y);
                         }
-                        *reinterpret_cast<uint4 *>(A + canon_off(row, kCols * h + 8 * j, kTcRows)) =
-                            make_uint4(q[0], q[1], q[2], q[3]);
+                        *reinterpret_cast<uint4 *>(A + canon_off(row, h + 8 * j, kTcRows)) = make_uint4(q[0], q[1], q[2], q[3]);
                     }
                 }
             } else {
@@ -558,7 +555,7 @@ k_guide_infer_tc(const unsigned char *img, const float *params, GuideParams gp, 
 #pragma unroll
                     for (int j = 0; j < kQ; ++j) put(j, reinterpret_cast<const float4 *>(out)[j]);
                 } else {
-float o[kGuideOut];
+                    float o[kGuideOut];
                     {
                         float v[48];
 #pragma unroll

@@ -39,13 +39,8 @@ constexpr int kP8MinBlocks = DR_P8_MIN_BLOCKS;
 #ifndef DR_REFILL_MIN
 #define DR_REFILL_MIN 4
 #endif
-// A lane postpones its leaf triangles while fewer than this many lanes of its
-// warp have triangles to test (0: never). Measured on the incoherent workload
-// (2^20 triangles, 16.8 M rays): 0 -> 3.75, 4 -> 3.67, 8..16 -> 3.66 Grays/s,
-// so it stays off; results are identical either way.
-#ifndef DR_POSTPONE_MIN
-#define DR_POSTPONE_MIN 0
-#endif
+// (Measured and dropped: leaf triangles postponed while fewer than 4, or 8 to 16,
+// lanes of the warp have triangles to test, 3.75 -> 3.67 and 3.66 Grays/s.)
 // Which public traversals send their leaf triangles through the warp's staged
 // triangle batch (tri_batch.cuh) instead of each lane's own loop. Measured
 // (incoherent workload: 2^20 triangles, 16.8 M rays, 23 % hits): closest hit
@@ -110,9 +105,10 @@ constexpr int kP8MinBlocks = DR_P8_MIN_BLOCKS;
 
 
 
-// Indices a warp reserves at once: 128 when there is plenty of work, down to
-// one per lane when few rays are left, so a small launch still spreads over
-// many warps (warp-uniform). A nonzero `fixed` (a multiple of 32) overrides it.
+// Indices a warp reserves at once: kPersistentChunk when there is plenty of work
+// (64, the renderer 32), down to one per lane in a small launch, so that it still
+// spreads over many warps (warp-uniform). A nonzero `fixed` (a multiple of 32)
+// overrides it.
 __device__ __forceinline__ uint32_t persistent_chunk(uint64_t n, uint32_t fixed = 0)
 {
     if (fixed) return fixed;
@@ -293,20 +289,11 @@ __device__ __forceinline__ void persistent_wide(const Wide8Args &a, const Source
                     if (!fin && s.have_node) wide_visit<MODE, HALF>(a, s, cn, cb);
                 }
             }
-            // 2. leaf triangles: tested now when enough lanes of the warp have
-            //    some (or the lane has no node to go to); otherwise pushed as a
-            //    group and tested when popped (Ylitie, Karras and Laine 2017,
-            //    triangle postponing). Results do not depend on the order of
-            //    the tests.
-            const bool has_tri = active && s.tmask != 0;
-            const unsigned tri_lanes = __ballot_sync(FULL, has_tri);
-            if (has_tri) {
-                const bool postpone = DR_POSTPONE_MIN > 0 && __popc(tri_lanes) < DR_POSTPONE_MIN &&
-                                      (s.group.y >> 8) != 0 && s.sp < kWideStack - 8;
-                if (postpone) {
-                    stack.put(s.sp++, make_uint2(s.tbase, s.tmask | kTriGroupFlag));
-                    s.tmask = 0;
-                } else if (wide_triangles<MODE, Q>(a, s, ct)) {
+            // 2. leaf triangles (as one condition, or without the last of the
+            //    next step's, the compiler's order of the loop is 1 % slower: box
+            //    room 16 spp 1.687 -> 1.708 ms)
+            if (active && s.tmask != 0) {
+                if (wide_triangles<MODE, Q>(a, s, ct)) {
                     done = found = true;
                 }
             }

@@ -63,10 +63,13 @@ constexpr int kRenderBlock = 128;
 constexpr int kShadeMinBlocks = DR_SHADE_MIN_BLOCKS;
 
 // Where k_wave_paths takes over. Waves of up to kWholePathsPerSm paths per SM
-// (155,648 on 152 SMs) run in it from the camera rays on; paths per wave and
-// time by bounces / in one kernel: 65,536 (box room) 696 / 464 us (415 now); 129,600
-// (2^17-triangle many-light) 853 / 490 us (447 now); 163,840 (box room) 950 / 872 us;
-// 262,144 (box room) 1,030 / 1,111 us. Larger waves hand over when at most
+// (155,648 on 152 SMs) run in it from the camera rays on. Paths per wave and time
+// by bounces / in one kernel, when the line was drawn: 65,536 (box room) 696 / 464
+// us; 129,600 (2^17-triangle many-light) 853 / 490 us; 163,840 (box room) 950 / 872
+// us; 262,144 (box room) 1,030 / 1,111 us. Now, in one kernel: 433 and 447 us for the
+// first two; 2^20-triangle many-light, 16 bounces: 108,000 paths 804 us, 155,520 920
+// us, by bounces with the tail 168,000 950 us, 204,800 1,008 us: no step at the
+// line. Larger waves hand over when at most
 // kTailPathsPerSm paths per SM (32,832) are left (tail_check). Limits of 16,384 /
 // 32,768 / 65,536 paths: many-light 2^16 triangles 512x512, 4 spp 1,439 / 1,359 /
 // 1,367 us (1,716 without), eight uneven scenes 967 / 969 / 969 us (1,286); a
@@ -274,63 +277,18 @@ __device__ __forceinline__ uint32_t slot_root(const RenderParams &p, uint32_t sl
 #define DR_GUIDE_FULL_EMISSION 1
 #endif
 
-// Decoded mixture in the wave buffer (DR_GUIDE_DECODED): the inference
+// Decoded mixture in the wave buffer: the inference
 // kernel writes each guided vertex's mixture already decoded, as five arrays
 // of 8 (guide_store_decoded), and the shading kernel reads them from memory at
 // each use, lobe by lobe, instead of holding the mixture in registers across
 // next-event estimation, so it runs with more warps per SM. Measured on the
 // occluded-light scene (480x270, 64 spp, frozen network): guided shading
 // 7.1 -> 5.4 ms over its 16 launches.
-#ifndef DR_GUIDE_DECODED
-#define DR_GUIDE_DECODED 1
-#endif
 #ifndef DR_GUIDE_SHADE_BLOCKS
-#define DR_GUIDE_SHADE_BLOCKS (DR_GUIDE_DECODED ? 6 : 4)
+#define DR_GUIDE_SHADE_BLOCKS 6
 #endif
 
-#if !DR_GUIDE_DECODED
-// The mixture held in registers (GuideMix), decoded by the shading kernel.
-__device__ __forceinline__ float guide_mix_pdf(const GuideMix &M, F3 w)
-{
-    float p = 0.0f;
-#pragma unroll
-    for (int j = 0; j < kGuideLobes; ++j) {
-        const float c = M.mx[j] * w.x + M.my[j] * w.y + M.mz[j] * w.z;
-        p += M.c[j] * __expf(M.kappa[j] * (c - 1.0f));
-    }
-    return p;
-}
 
-// Lobe by u0 (cumulative weights, as guide_sample), then its vMF by (u1, u2).
-__device__ __forceinline__ F3 guide_mix_sample(const GuideMix &M, float u0, float u1, float u2)
-{
-    float k = M.kappa[0], ax = M.mx[0], ay = M.my[0], az = M.mz[0];
-    float acc = M.pi[0];
-#pragma unroll
-    for (int j = 1; j < kGuideLobes; ++j) {
-        if (u0 >= acc) k = M.kappa[j], ax = M.mx[j], ay = M.my[j], az = M.mz[j];
-        acc += M.pi[j];
-    }
-    float wx, wy, wz;
-    vmf_sample(k, ax, ay, az, u1, u2, wx, wy, wz);
-    return f3(wx, wy, wz);
-}
-
-// Density of the guided part at w, for a surface of normal n.
-__device__ __forceinline__ float guide_pdf_above(const GuideMix &M, F3 w, F3 n)
-{
-#if DR_GUIDE_REFLECT
-    const float c = dot(w, n);
-    if (!(c > 0.0f)) return 0.0f;
-    const F3 r = sub(w, mul(n, 2.0f * c));
-    return guide_mix_pdf(M, w) + guide_mix_pdf(M, r);
-#else
-    return guide_mix_pdf(M, w);
-#endif
-}
-#endif
-
-#if DR_GUIDE_DECODED
 // Density of the guided part at w above a surface of normal n, from the
 // decoded mixture (the mirrored direction in the same pass over the lobes).
 __device__ __forceinline__ float guide_dec_pdf_above(const float *y, F3 w, F3 n)
@@ -370,22 +328,13 @@ __device__ __forceinline__ F3 guide_dec_sample(const float *y, float u0, float u
     vmf_sample(y[8 + sel], y[16 + sel], y[24 + sel], y[32 + sel], u1, u2, wx, wy, wz);
     return f3(wx, wy, wz);
 }
-#endif
 
 // The guided density and sampler the shading kernel uses.
-#if DR_GUIDE_DECODED
 __device__ __forceinline__ float guide_density(const float *y, F3 w, F3 n) { return guide_dec_pdf_above(y, w, n); }
 __device__ __forceinline__ F3 guide_draw(const float *y, float u0, float u1, float u2)
 {
     return guide_dec_sample(y, u0, u1, u2);
 }
-#else
-__device__ __forceinline__ float guide_density(const GuideMix &M, F3 w, F3 n) { return guide_pdf_above(M, w, n); }
-__device__ __forceinline__ F3 guide_draw(const GuideMix &M, float u0, float u1, float u2)
-{
-    return guide_mix_sample(M, u0, u1, u2);
-}
-#endif
 
 __global__ void __launch_bounds__(kRenderBlock) k_camera(RenderParams p)
 {
@@ -668,12 +617,7 @@ __device__ __forceinline__ void shade_vertex(const RenderParams &p, int b, uint3
             }
             if (emits) p.color[slot] = col;
             const float alpha = GUIDED && b < p.guide_bounces ? p.guide_alpha : 0.0f;
-#if DR_GUIDE_DECODED
             const float *lobes = GUIDED ? p.guide_y + (size_t)slot * kGuideOut : nullptr;
-#else
-            GuideMix lobes;
-            if (GUIDED && alpha > 0.0f) lobes = guide_mix(p.guide_y + (size_t)slot * kGuideOut);
-#endif
             // next-event estimation: samplePointOnLights (:234-272) and
             // evaluateDirectLighting (:336-361); visibility is the shadow ray
             if (J.lights) {
@@ -1450,7 +1394,7 @@ dr_status WaveRunner::enqueue(const SceneArrays &sc, const WavePlan &plan, const
                 if (b < (int)gr->bounces) {
                     DR_CUDA(launch_next(early, k_guide_prepare, shade_grid, kRenderBlock, 0, ws, q, b));
                     DR_CUDA(launch_guide_infer(gr->guide, q.guide_pos, q.guide_nrm, q.guide_list, q.guide_counts + b,
-                                               W, q.guide_y, ws, DR_GUIDE_DECODED != 0));
+                                               W, q.guide_y, ws, true));
                 }
                 DR_CUDA(launch_next(early, k_shade<true>, shade_grid, kRenderBlock, 0, ws, q, b, 0u));
             } else {

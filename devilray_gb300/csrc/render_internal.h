@@ -86,7 +86,6 @@ struct GuideRun {
     uint32_t batch = 16384;
     uint32_t steps = 4;
     uint32_t budget = 0;  // total Adam steps of the network after which training stops, 0 = none
-    uint32_t streams = 1; // concurrent waves; training of the waves runs one after another
     uint32_t target = 0;  // training target: 0 radiance, 1 log(1 + radiance)
     uint32_t bounces = 64;  // bounces b < bounces are guided
     uint32_t alpha_ramp = 0;  // alpha rises linearly over the network's first alpha_ramp steps, 0 = none
@@ -108,7 +107,6 @@ struct WaveRunner {
     size_t jobs_capacity = 0;
     WaveSegment *d_segs = nullptr;
     size_t segs_capacity = 0;
-    bool guided = false;              // slot buffers carry the guiding state
     void *d_train = nullptr;          // training ring (guided renders)
     uint32_t train_cap = 0;
     unsigned long long *d_totals = nullptr;  // rays of the last schedule: path, shadow

@@ -20,15 +20,16 @@ namespace dr {
 // Lanes per ray. Public launches: 8 lanes have the shorter chain per node (2^10
 // rays, 300,000 triangles, closest hit: 25 us against 27 us with 4 lanes and 41 us
 // with one lane per ray; 2^14 rays 34 / 40 / 54 us); 4 lanes keep more rays in
-// flight, which the path kernel wants (box room 256x256, 1 spp: 464 us against
-// 593 us with 8).
+// flight, which the path kernel wants (box room 256x256, 1 spp, before its paths
+// were dealt in runs: 464 us against 593 us with 8; now 433 us).
 constexpr int kTeamTrace = 8, kTeamPaths = 4;
 
 // Public launches of up to this many rays per SM run with teams (65,664 rays
 // on 152 SMs). Teams / one lane per ray, us, closest hit and any hit:
 // 300,000 triangles 2^8 rays 19 / 30, 15 / 29; 2^12 27 / 55, 26 / 54; 2^16
 // 63 / 74, 52 / 61; 2^17 96 / 83, 79 / 67; 5,000 triangles 2^16 32 / 35,
-// 29 / 35; 2^17 45 / 49, 41 / 38.
+// 29 / 35; 2^17 45 / 49, 41 / 38. 2^20 triangles (against the kernels of one lane per
+// ray before them): 2^12 35 / 61, 34 / 59; 65,600 74 / 87, 67 / 80.
 constexpr uint32_t kTeamRaysPerSm = 432;
 
 // The traversal stacks of a block of kTraceBlock threads in shared memory: 32
@@ -117,7 +118,7 @@ __device__ __forceinline__ void team_wide(const Wide8Args &a, const Source &src,
                     any = src.is_any(idx);
                     if (src.load(idx, r, root) && root != kNoRoot) {
                         if (MODE == 1) w = wt_setup(r.v);
-                        oct = DR_NO_OCT_ORDER ? 0u : ray_octant(r);
+                        oct = ray_octant(r);
                         best_t = r.tmax;
                         best_prim = INT_MAX;
                         node = root;

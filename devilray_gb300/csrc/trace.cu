@@ -1,19 +1,19 @@
 // trace.cu -- public closest-hit and any-hit kernels on sm_103a.
 //
 // Replaces the reference's per-object stackless descent with parent pointers
-// (DevilRay include/tracing/IntersectionTestsImpl.hpp:141-251) by the stack
-// traversal of trace_device.cuh over a binned-SAH two-box BVH. One thread per
-// ray; the result equals a brute-force scan of the reference triangle test
-// over the whole soup (smallest t, ties to the smaller triangle index).
+// (DevilRay include/tracing/IntersectionTestsImpl.hpp:141-251). The 8-wide
+// hierarchy is traversed by persistent warps (persistent.cuh), launches of few
+// rays by teams of lanes (team.cuh); the binary one by one thread per ray
+// (trace_device.cuh). The result equals a brute-force scan of the reference
+// triangle test over the whole soup (smallest t, ties to the smaller triangle
+// index).
 
-// The public 8-wide kernels run the slab FMAs of slots j and j + 4 as packed
-// FP32 pairs and are compiled for 7 resident blocks per SM (73 registers).
-// Measured on the incoherent workload (2^20 triangles, 16.8 M rays, closest
-// hit): scalar at 8 blocks 3.383 ms, packed at 7 blocks 3.336-3.339 ms,
-// packed at 6 blocks 3.534 ms, scalar at 7 blocks 3.409 ms; hits identical.
-#ifndef DR_PACKED_SLAB
-#define DR_PACKED_SLAB 1
-#endif
+// The public 8-wide kernels run the slab FMAs of two slots as packed FP32 pairs
+// and are compiled for 7 resident blocks per SM (72 registers), the closest hit
+// 3.14 ms on the incoherent workload (2^20 triangles, 16.8 M rays). Measured there
+// before the FP16 planes: scalar at 8 blocks 3.383 ms, packed at 7 blocks
+// 3.336-3.339 ms, packed at 6 blocks 3.534 ms, scalar at 7 blocks 3.409 ms; hits
+// identical.
 #ifndef DR_P8_MIN_BLOCKS
 #define DR_P8_MIN_BLOCKS 7
 #endif
