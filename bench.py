@@ -39,14 +39,14 @@ NUM_TRIS = 1 << 20
 NUM_RAYS = 1 << 24
 # DRAM bytes of one full 16.8 M-ray launch of the dominant kernel, from one
 # `ncu --set full` capture of this workload (the profiles named beside them).
-NCU_TRAFFIC = {8: 928_030_720 + 130_330_112, 2: 1_652_000_000 + 152_000_000}
+NCU_TRAFFIC = {8: 928_169_728 + 129_861_376, 2: 1_652_000_000 + 152_000_000}
 NCU_PROFILE = {8: "trace_closest_p8_incoherent_1M_tris_16M_rays.md",
                2: "trace_closest_bvh2_incoherent_1M_tris_16M_rays.md"}
 # Warp instructions per ray of the dominant kernel (smsp__inst_executed.sum of
 # the same capture / 16,777,216 rays): with the launch time and the sampled SM
 # clock it gives the issue-slot fraction (4 schedulers per SM, one instruction
 # per scheduler and cycle).
-NCU_WARP_INST_PER_RAY = {8: 3_146_615_735 / NUM_RAYS}
+NCU_WARP_INST_PER_RAY = {8: 3_093_323_880 / NUM_RAYS}
 METRIC = "Mrays/s closest-hit"
 # Seconds the timed steps of --impl port may take in all (it sizes its per-step
 # sample of the workload to fit).

@@ -279,7 +279,8 @@ __global__ void __launch_bounds__(128) k_guide_infer(const __nv_bfloat16 *wb, co
 // inputs and run epilogues. Same arithmetic as k_guide_infer (BF16 products,
 // FP32 sums). Bound by the shared / tensor memory data path (0.6 of it by loads
 // and stores, the operands of the MMAs beside them) and by that chain's latency;
-// 0.58 of the issue slots, 0.3 of HBM for 2^20 rows in 95 us. The sines and cosines
+// 0.58 of the issue slots, 0.3 of HBM for 2^20 rows in 95 us (98 since the ReLU takes
+// a NaN to 0, an instruction more per pair). The sines and cosines
 // of the inputs are some 19 us of it; outputs of whole tiles leave as one bulk copy
 // (117 against 108 us when every tile's rows went through loads and stores).
 
@@ -360,8 +361,8 @@ constexpr uint32_t kTcW4 = kTcW1 + 3 * 64 * 64 * 2;  // 48 x 64
 constexpr uint32_t kTcA = kTcW4 + 48 * 64 * 2;       // per group: 128 x 80 input / 128 x 64 hidden / 128 x 40 output
 constexpr uint32_t kTcABytes = kTcRows * kIn * 2;
 static_assert(kTcABytes == kTcRows * kGuideOut * 4, "the output rows fit the input tile");
-// Groups per CTA: 6 run at 80 registers (2^20 rows: 95 us; 200,000 rows 23.8),
-// 5 at 96 (101; 27.0), 7 and 8 spill at 72 and 64 (94; 24.7 and 25.7). Three CTAs
+// Groups per CTA, at that time: 6 run at 80 registers (2^20 rows: 95 us; 200,000
+// rows 23.8), 5 at 96 (101; 27.0), 7 and 8 spill at 72 and 64 (94; 24.7 and 25.7). Three CTAs
 // of one group each, with their own copies of the weights, took 178 us.
 constexpr int kInferGroups = 6;
 constexpr uint32_t kTcBias = kTcA + kInferGroups * kTcABytes;
@@ -1603,6 +1604,9 @@ cudaError_t launch_guide_infer(const dr_guide *g, const float *pos, const float 
         const unsigned tiles = (max_rows + kTcRows - 1) / kTcRows;
         const unsigned blocks = std::min<unsigned>(tiles, (unsigned)g->ctx->num_sms);
         const auto kernel = decoded ? k_guide_infer_tc<true> : k_guide_infer_tc<false>;
+        // early also beside the waves of other streams, where the renderer's own
+        // kernels are not: guided renders of 2 to 32 waves on 2 and 3 streams take
+        // the same time either way, and 2 to 3 % less with early training kernels
         const cudaError_t e = launch_after(kernel, blocks, 128 * kInferGroups, kTcSmem, st, g->img, g->params, guide_params(g),
                                            pos, dir, list, count, max_rows, y, g->ctx->product_polls, g->ctx->d_error);
         if (e != cudaSuccess) return e;

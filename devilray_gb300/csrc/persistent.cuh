@@ -40,7 +40,8 @@ constexpr int kP8MinBlocks = DR_P8_MIN_BLOCKS;
 #define DR_REFILL_MIN 4
 #endif
 // (Measured and dropped: leaf triangles postponed while fewer than 4, or 8 to 16,
-// lanes of the warp have triangles to test, 3.75 -> 3.67 and 3.66 Grays/s.)
+// lanes of the warp have triangles to test, 3.75 -> 3.67 and 3.66 Grays/s. The flag
+// by which a pop told such groups apart cost 3.178 -> 3.116 ms while it was there.)
 // Which public traversals send their leaf triangles through the warp's staged
 // triangle batch (tri_batch.cuh) instead of each lane's own loop. Measured
 // (incoherent workload: 2^20 triangles, 16.8 M rays, 23 % hits): closest hit

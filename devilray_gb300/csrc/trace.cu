@@ -10,7 +10,7 @@
 
 // The public 8-wide kernels run the slab FMAs of two slots as packed FP32 pairs
 // and are compiled for 7 resident blocks per SM (72 registers), the closest hit
-// 3.14 ms on the incoherent workload (2^20 triangles, 16.8 M rays). Measured there
+// 3.09 ms on the incoherent workload (2^20 triangles, 16.8 M rays). Measured there
 // before the FP16 planes: scalar at 8 blocks 3.383 ms, packed at 7 blocks
 // 3.336-3.339 ms, packed at 6 blocks 3.534 ms, scalar at 7 blocks 3.409 ms; hits
 // identical.

@@ -185,3 +185,32 @@ def test_failed_allocations_return_out_of_memory(native, ctx):
     torch.cuda.synchronize()
     free1 = torch.cuda.mem_get_info()[0]
     assert free0 - free1 < 16 << 20, f"{(free0 - free1) >> 20} MiB of device memory not returned"
+
+
+@pytest.mark.parametrize("kernel", [0, 1])
+def test_failed_allocation_of_a_training_step(native, ctx, kernel):
+    """A network's first training step allocates its buffers; when that fails the
+    step returns out-of-memory, takes no step, and the next one is exact."""
+    lib = native.load()
+    n = 3000
+    rng = np.random.default_rng(4)
+
+    def unit():
+        d = rng.normal(size=(n, 3))
+        return torch.from_numpy((d / np.linalg.norm(d, axis=1, keepdims=True)).astype(np.float32)).cuda()
+
+    pos = torch.from_numpy(rng.uniform(-1, 1, (n, 3)).astype(np.float32)).cuda()
+    args = (pos, unit(), unit(), torch.ones(n, device="cuda"), n)
+    g, plain = (native.Guide(ctx, seed=6, infer_kernel=kernel) for _ in range(2))
+    before = g.params()
+    native.check(lib.dr_debug_fail_allocation(1))
+    assert _status_of(lambda: g.train_step(*args)) == 3  # DR_ERR_OUT_OF_MEMORY
+    native.check(lib.dr_debug_fail_allocation(0))
+    torch.cuda.synchronize()
+    assert np.array_equal(g.params(), before) and g.get_state()[12:16].view(np.uint32)[0] == 0
+    g.train_step(*args)
+    plain.train_step(*args)
+    if kernel == 0:  # the mma.sync kernels add with atomics
+        assert np.array_equal(g.params(), plain.params())
+    assert not np.array_equal(g.params(), before)
+    assert _status_of(ctx.check) == 0
