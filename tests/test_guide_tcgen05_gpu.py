@@ -158,3 +158,32 @@ def test_rows_of_non_finite_directions_stay_finite(native, ctx, n):
     for kernel in (0, 1):
         assert np.array_equal(out[kernel, "odd"][bad], np.broadcast_to(bias[:40], (len(bad), 40)))
         assert np.array_equal(out[kernel, "odd"][keep], out[kernel, "good"][keep])
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), float("-inf")])
+def test_non_finite_rows_over_many_tiles(native, ctx, value):
+    """Tiles that hold a row of a non-finite direction are carried through twice,
+    in any group and pass of a block: both kernels give finite outputs for such
+    rows and agree; every other row has the bits it has without them."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n = 6 * 128 * sms + 7 * 128 + 50
+    rng = np.random.default_rng(12)
+    pos = torch.from_numpy(rng.uniform(-10, 10, (n, 3)).astype(np.float32)).cuda()
+    d = rng.normal(size=(n, 3))
+    d = torch.from_numpy((d / np.linalg.norm(d, axis=1, keepdims=True)).astype(np.float32)).cuda()
+    bad = torch.from_numpy(np.unique(rng.integers(0, n, 200))).cuda()
+    odd = d.clone()
+    odd[bad, 1] = value
+    out = []
+    for kernel in (0, 1):
+        g = native.Guide(ctx, seed=10, half_extent=10.0, infer_kernel=kernel)
+        y, z = (torch.full((n, 40), float("nan"), dtype=torch.float32, device="cuda") for _ in range(2))
+        g.infer(pos, d, n, y)
+        g.infer(pos, odd, n, z)
+        keep = torch.ones(n, dtype=torch.bool, device="cuda")
+        keep[bad] = False
+        assert bool(torch.isfinite(z).all()) and torch.equal(y[keep], z[keep])
+        out.append(z[bad])
+    ctx.check()
+    scale = float(out[1].abs().max()) + 1e-6
+    assert float((out[0] - out[1]).abs().max()) <= 2e-2 * scale
